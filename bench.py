@@ -441,7 +441,7 @@ def run_ours(args):
         names = ["rpy", "chol", "rd", "forces1", "move1", "frames", "forces2", "move2+frames", "total"]
         line = {"metric": METRIC, "value": value, "unit": "steps/s", "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
-                "vs_baseline": None, "dtype": "f64" if prec == PREC_FP64 else "bf16x3+f64",
+                "vs_baseline": None, "dtype": "f64" if prec == PREC_FP64 else "fp16x2+f64",
                 "data": "synthetic (seeded fiber generator, reference file formats)",
                 "config": {"workload": spec.name, "n_D": fib.n_D, "3N": m, "precision": args.precision,
                            "frequency_RP": args.frequency_rp, "noise": args.noise,
@@ -662,7 +662,7 @@ def run_batch(args):
     if rank == 0:
         line = {"metric": METRIC, "value": value, "unit": "replica-steps/s", "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
-                "vs_baseline": None, "dtype": "f64" if prec == PREC_FP64 else "bf16x3+f64",
+                "vs_baseline": None, "dtype": "f64" if prec == PREC_FP64 else "fp16x2+f64",
                 "data": "synthetic (seeded fiber generator, reference file formats)",
                 "config": {"workload": "cfg2_replicas", "replicas": len(fibers), "3N_min": min(sizes),
                            "3N_max": max(sizes), "3N_sum": sum(sizes), "precision": args.precision,

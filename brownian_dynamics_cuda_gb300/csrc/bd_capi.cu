@@ -170,7 +170,7 @@ static int step_phases(bd_ctx* c, const double* d_rr, const double* d_p, double*
       c->kev_pairs = 0;
       L += bdk::potrf_mixed(c->m, c->A, c->lda, c->PS, c->negpiv, c->d_err, st, kt ? c->kev.data() : nullptr,
                             kt ? &c->kev_pairs : nullptr, kt ? &c->kflop : nullptr,
-                            kt ? &c->kbytes : nullptr, c->mixed_passes);
+                            kt ? &c->kbytes : nullptr, c->mixed_passes, c->fscale);
     }
     else L += bdk::potrf_fp64(c->m, c->A, c->lda, nullptr, nullptr, 0.0, c->negpiv, st);
   }
@@ -346,6 +346,7 @@ extern "C" int bd_create(const bd_model* m, const bd_state* s, const bd_options*
   for (int i = 0; i < n; i++) rad_all[i] = m->rad[i];
   for (int i = 0; i < nt; i++) rad_all[n + i] = m->t_rad[i];
   for (int i = 0; i < nL; i++) rad_all[n + nt + i] = m->lh_rad[i];
+  c->fscale = bdk::mixed_scale(M.a1, rad_all.data(), M.n_D);
   // sizes.  Every buffer that depends on the linker-histone binding is sized
   // for every core bound (capacity), so that bd_set_lh_flags resizes the
   // context in place; the logical sizes (M.n_LH, M.n_D, c->m) follow the flags.
@@ -708,7 +709,7 @@ static int factor_now(bd_ctx* c) {
   CK(cudaMemsetAsync(c->negpiv, 0, sizeof(int), c->stream));
   if (c->precision == BD_PREC_MIXED) {
     bdk::potrf_mixed(c->m, c->A, c->lda, c->PS, c->negpiv, c->d_err, c->stream, nullptr, nullptr, nullptr, nullptr,
-                     c->mixed_passes);
+                     c->mixed_passes, c->fscale);
     int derr = 0;
     CK(cudaMemcpyAsync(&derr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -918,12 +919,13 @@ static int batch_prepare(bd_batch* b) {
     std::vector<double*> A(nr);
     std::vector<unsigned char*> PS(nr);
     std::vector<int*> np(nr), er(nr);
+    std::vector<float> sc(nr);
     for (size_t i = 0; i < nr; i++) {
       bd_ctx* c = b->ctx[i];
-      m[i] = c->m, lda[i] = c->lda, A[i] = c->A, PS[i] = c->PS, np[i] = c->negpiv, er[i] = c->d_err;
+      m[i] = c->m, lda[i] = c->lda, A[i] = c->A, PS[i] = c->PS, np[i] = c->negpiv, er[i] = c->d_err, sc[i] = c->fscale;
     }
     b->chol = bdk::mixed_batch_create((int)nr, m.data(), A.data(), lda.data(), PS.data(), np.data(), er.data(),
-                                      b->ctx[0]->mixed_passes);
+                                      sc.data(), b->ctx[0]->mixed_passes);
     if (!b->chol) return set_error(BD_ERR_NOMEM, "bd_batch: batched factorisation plan");
     if (b->lane.empty()) {  // kept when the plan is rebuilt (bd_batch_set_mixed_passes)
       const int nl = (int)std::min<size_t>(nr, kBatchLanes);
@@ -1325,6 +1327,12 @@ extern "C" int bd_set_lh_flags(bd_ctx* c, const int* nc_lh_flag, const double* r
       (rc = up(const_cast<double*>(M.rad_all) + n + nt, rad.data(), nLH, st)) ||
       (rc = up(c->X.r_lh, r_lh, 3 * nLH, st)))
     return rc;
+  {
+    std::vector<double> all(mc.rad.begin(), mc.rad.end());
+    all.insert(all.end(), mc.t_rad.begin(), mc.t_rad.end());
+    all.insert(all.end(), rad.begin(), rad.end());
+    c->fscale = bdk::mixed_scale(M.a1, all.data(), (int)all.size());
+  }
   // logical sizes and the offsets that depend on them
   M.n_LH = nLH;
   M.n_D = n + nt + nLH;

@@ -157,8 +157,11 @@ int set_mixed_attributes();
 // max_pass: at most this many panels (1..3) per bulk trailing pass.
 int potrf_mixed(int m, double* A, int lda, unsigned char* PS, int* negpiv, int* err, cudaStream_t st,
                 cudaEvent_t* kev = nullptr, int* kev_pairs = nullptr, double* kflop = nullptr,
-                double* kbytes = nullptr, int max_pass = 3);
+                double* kbytes = nullptr, int max_pass = 3, float scale = 1.f);
 int mixed_tiles(int m);
+// The power of two that a factor's FP16 panel slices are scaled by: nrad
+// radii, D_ii = a1 / rad_i
+float mixed_scale(double a1, const double* rad, int nrad);
 // k_krylov.cu: rd = s2dt D^{1/2} p by Lanczos on the lower-stored tensor
 size_t krylov_scratch_doubles(int m, int kmax);
 // tc_gemm.cu: C = alpha A op(B) on tcgen05 (row-major FP32, three BF16
@@ -200,7 +203,7 @@ int mixed_max_launches(int m);  // k_chol_step launches of one factorisation, at
 // scatter for all.  The plan holds the matrices' addresses.
 struct MixedBatch;
 MixedBatch* mixed_batch_create(int nrep, const int* m, double* const* A, const int* lda, unsigned char* const* PS,
-                               int* const* negpiv, int* const* err, int max_pass = 3);
+                               int* const* negpiv, int* const* err, const float* scale, int max_pass = 3);
 int mixed_batch_run(const MixedBatch* b, cudaStream_t st);  // returns the launches issued
 void mixed_batch_free(MixedBatch* b);
 
@@ -232,6 +235,7 @@ struct bd_ctx {
   int precision = BD_PREC_FP64;
   int freq_rp = 1;
   int use_graph = 0;
+  float fscale = 1.f;    // mixed path: the panel slices hold fscale * L (mixed_scale)
   int mixed_passes = 3;  // panels per bulk trailing pass of the mixed factorisation (bd_set_mixed_passes)
   // noise displacement: 0 = L p (the reference's), 1 = D^{1/2} p by Lanczos (bd_set_noise_mode)
   int noise_mode = 0;
@@ -249,7 +253,7 @@ struct bd_ctx {
   DevScratch S{};
   void* arena_base = nullptr;
   double* A = nullptr;   // m x lda, column-major; holds D then L (FP64 path)
-  unsigned char* PS = nullptr;  // mixed path: BF16 panel slices
+  unsigned char* PS = nullptr;  // mixed path: FP16 panel slices
   int* d_err = nullptr;         // device error code of the tensor-core kernels
   int m = 0, lda = 0;  // 3 n_D now, and the leading dimension of A (for m_cap)
   int m_cap = 0;       // largest m the buffers hold: every core with a linker histone

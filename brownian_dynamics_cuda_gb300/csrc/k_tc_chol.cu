@@ -11,28 +11,34 @@
 //                CTA 0 keeps it in a side buffer (copied into A after the
 //                last panel) and the others solve one 128-row tile each,
 //                L_ik = A_ik L_kk^-T, by forward substitution, write it back
-//                and split it into three BF16 slices (hi + mid + lo = the
-//                FP32 value exactly), stored pre-swizzled in the
-//                128-byte-swizzle K-major layout the MMA reads; a negative
-//                pivot is replaced by its absolute value and counted
+//                and split it into two FP16 slices (scaled by one power of
+//                two: hi + lo = the FP32 value to 2^-24), stored pre-swizzled
+//                in the 128-byte-swizzle K-major layout the MMA reads; a
+//                negative pivot is replaced by its absolute value and counted
 //                (func.cpp:827-833).
 //   update CTAs  trailing update A_IJ -= L_I L_J^T of one or two earlier
 //                panels, a run of tiles per CTA, warp-specialised:
-//                bulk-async operand copies, six BF16 products (hi.hi,
-//                hi.mid, mid.hi, hi.lo, mid.mid, lo.hi) per panel into one of
-//                two FP32 tensor-memory accumulators (tcgen05.mma,
-//                M = N = 128, K = 16 per instruction), tcgen05.ld epilogue
-//                subtracting into the double-float tile.  The dropped
-//                products are below 2^-24 of the kept ones: FP32-class
-//                products.
+//                bulk-async operand copies, three FP16 products (lo.hi,
+//                hi.lo, hi.hi) per panel into one of two FP32 tensor-memory
+//                accumulators (tcgen05.mma, M = N = 128, K = 16 per
+//                instruction), tcgen05.ld epilogue subtracting into the
+//                double-float tile.  The dropped product lo.lo is below
+//                2^-24 of the kept ones: FP32-class products.
+// Two FP16 slices and three products instead of three BF16 slices and six
+// (which hold the FP32 value exactly): half the tensor work, two thirds of
+// the operand bytes.  3N = 11,700: 7.0 -> 6.1 ms; 3N = 46,200: 202 -> 157 ms.
+// Error of L p against FP64 (2-norm, 13 fibers of 3N 912 .. 11,700):
+// 2.6e-7 .. 5.4e-7 before, 2.6e-7 .. 5.1e-7 now - the sums inside the tensor
+// core set it, not the split.
 // The launches run on one stream, one at a time (the schedule is at
 // potrf_mixed).  Every mbarrier wait is bounded; on a timeout the kernel
 // records an error code, frees its tensor memory and returns.
 #include <algorithm>
+#include <cmath>
 #include <utility>
 #include <vector>
 
-#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include "bd_internal.h"
@@ -44,10 +50,10 @@ namespace {
 
 
 constexpr int kT = 128;                 // tile / panel width
-constexpr int kSliceBytes = kT * kT * 2;  // one BF16 slice of a 128 x 128 tile (two 64-column halves)
+constexpr int kSliceBytes = kT * kT * 2;  // one FP16 slice of a 128 x 128 tile (two 64-column halves)
 constexpr int kHalfBytes = kSliceBytes / 2;
-constexpr int kTileSlices = 3;
-constexpr int kTileBytes = kTileSlices * kSliceBytes;  // 96 KB per 128-row panel tile
+constexpr int kTileSlices = 2;
+constexpr int kTileBytes = kTileSlices * kSliceBytes;  // 64 KB per 128-row panel tile
 constexpr uint32_t kWaitLimit = 1u << 24;
 
 inline int cdiv(int a, int b) { return (a + b - 1) / b; }
@@ -57,6 +63,20 @@ __device__ __forceinline__ int cdiv_d(int a, int b) { return (a + b - 1) / b; }
 __device__ __forceinline__ uint32_t swz_off(int r, int k) {
   int half = k >> 6, kk = k & 63;
   return half * kHalfBytes + (r >> 3) * 1024 + (r & 7) * 128 + ((((kk >> 3) ^ (r & 7)) & 7) << 4) + (kk & 7) * 2;
+}
+
+// Two scaled FP32 values as FP16 pairs: x = hi + lo to 2^-24 |x| (two
+// roundings to 11 bits each), low half first.  A finite value past FP16's
+// range (see the scale at StepArgs) is clamped; Inf and NaN stay.
+__device__ __forceinline__ void split_f16x2(float x0, float x1, uint32_t& hi, uint32_t& lo) {
+  const float lim = 65504.f;
+  if (fabsf(x0) > lim && !isinf(x0)) x0 = copysignf(lim, x0);
+  if (fabsf(x1) > lim && !isinf(x1)) x1 = copysignf(lim, x1);
+  const __half2 h = __floats2half2_rn(x0, x1);
+  const float2 hf = __half22float2(h);
+  const __half2 l = __floats2half2_rn(x0 - hf.x, x1 - hf.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
 // (hi, lo) - v in double-float arithmetic: exact two-sums (Knuth), so the
@@ -256,10 +276,9 @@ __device__ __forceinline__ void warp_chol32(float (&a)[32], int w, int lane, flo
 // Row r of the CTA's rows of L_ik (row rs of the 128-row tile), columns
 // c0 .. c0 + 31 (x[j] = 0 past column w): (L, 0) pairs into A (`g` = A at
 // column c0 of the CTA's first row) for rows inside the matrix, and the
-// 16-byte chunks of the three BF16 slices (x = hi + mid + lo exactly,
-// 8 + 8 + 8 significant bits) for every row of the tile.
+// 16-byte chunks of the two FP16 slices of scale * x for every row of the tile.
 __device__ __forceinline__ void dp_emit(const float (&x)[32], int r, int rs, int nrows, int c0, int w, float2* g,
-                                        int lda, unsigned char* ps) {
+                                        int lda, unsigned char* ps, float scale) {
   if (r < nrows) {  // read again only by the noise product after the factorisation (BD_DP_EVICT_FIRST)
     const uint64_t pol = sm100::policy_evict_first();
 #pragma unroll
@@ -271,28 +290,12 @@ __device__ __forceinline__ void dp_emit(const float (&x)[32], int r, int rs, int
   }
 #pragma unroll
   for (int q8 = 0; q8 < 4; q8++) {
-    uint32_t hw[4], mw[4], lw[4];
+    uint32_t hw[4], lw[4];
 #pragma unroll
-    for (int j2 = 0; j2 < 4; j2++) {
-      uint32_t h2 = 0u, m2 = 0u, l2 = 0u;
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const float v = x[8 * q8 + 2 * j2 + e];
-        const __nv_bfloat16 h = __float2bfloat16_rn(v);
-        const float r1 = v - __bfloat162float(h);
-        const __nv_bfloat16 md = __float2bfloat16_rn(r1);
-        const float r2 = r1 - __bfloat162float(md);
-        const __nv_bfloat16 lo = __float2bfloat16_rn(r2);
-        h2 |= (uint32_t)__bfloat16_as_ushort(h) << (16 * e);
-        m2 |= (uint32_t)__bfloat16_as_ushort(md) << (16 * e);
-        l2 |= (uint32_t)__bfloat16_as_ushort(lo) << (16 * e);
-      }
-      hw[j2] = h2, mw[j2] = m2, lw[j2] = l2;
-    }
+    for (int j2 = 0; j2 < 4; j2++) split_f16x2(x[8 * q8 + 2 * j2] * scale, x[8 * q8 + 2 * j2 + 1] * scale, hw[j2], lw[j2]);
     const uint32_t off = swz_off(rs, c0 + 8 * q8);
     *reinterpret_cast<uint4*>(ps + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-    *reinterpret_cast<uint4*>(ps + kSliceBytes + off) = make_uint4(mw[0], mw[1], mw[2], mw[3]);
-    *reinterpret_cast<uint4*>(ps + 2 * kSliceBytes + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+    *reinterpret_cast<uint4*>(ps + kSliceBytes + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
   }
 }
 
@@ -302,7 +305,7 @@ __device__ __forceinline__ void dp_emit(const float (&x)[32], int r, int rs, int
 // The previous panel's update of this panel's column, applied in the panel
 // CTA itself (so no separate launch precedes the panel): with panel p's
 // slices PSpre, D0 = L_kp L_kp^T for the diagonal tile and (tile CTAs)
-// D1 = L_ip L_kp^T for the CTA's tile, six BF16 products per K step on
+// D1 = L_ip L_kp^T for the CTA's tile, three FP16 products per K step on
 // tcgen05 into two 128-column TMEM accumulators.  The operands are streamed
 // in two K-halves into the memory the panel later uses for S, so the
 // products are complete before S is loaded; they are subtracted from S
@@ -311,11 +314,13 @@ struct PreBars {
   uint64_t full[2], done;
   uint32_t slot;
 };
-constexpr int kPreStage = 2 * kTileSlices * kHalfBytes;  // one K-half of the A and B slices (96 KB)
+constexpr int kPreStage = 2 * kTileSlices * kHalfBytes;  // one K-half of the A and B slices (64 KB)
+constexpr int kPreBarOff = 137 * 1024;                   // the barriers lie past the stages and the panel
+static_assert(kPreBarOff >= 2 * kPreStage && kPreBarOff >= (int)kDpSmem, "barriers past both uses of the memory");
 
 __device__ __forceinline__ void dpanel_body(float4* sm4, float2* A, float* Ldg, int lda, int m, int k0, int kb, int tile0,
                                             int b, unsigned char* PS, int* negpiv, const unsigned char* PSpre,
-                                            int* err, int rpc) {
+                                            int* err, int rpc, float scale, float iscale2) {
   float (*S)[kLd] = reinterpret_cast<float (*)[kLd]>(sm4);  // rows 0..127 diagonal block, 128..255 tile
   float* T = reinterpret_cast<float*>(sm4) + 2 * kT * kLd;  // the current 32 x 32 factor, transposed
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -328,7 +333,7 @@ __device__ __forceinline__ void dpanel_body(float4* sm4, float2* A, float* Ldg, 
   const int nrows = is_diag ? 0 : max(0, min(rpc, m - row0));
   DP_MARK(0);
   unsigned char* smA = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(sm4) + 1023) & ~uintptr_t(1023));
-  PreBars* pbar = reinterpret_cast<PreBars*>(smA + 2 * kPreStage);
+  PreBars* pbar = reinterpret_cast<PreBars*>(smA + kPreBarOff);
   uint32_t tmem = 0;
   bool pre_ok = true;
   if (PSpre) {
@@ -346,7 +351,7 @@ __device__ __forceinline__ void dpanel_body(float4* sm4, float2* A, float* Ldg, 
     if (tid == 0) {
       const unsigned char* gB = PSpre + (size_t)(tile0 - 1) * kTileBytes;  // this panel's tile row
       const unsigned char* gA = PSpre + (size_t)tile * kTileBytes;
-      for (int h = 0; h < 2; h++) {  // stage h: [A: three 16 KB slice halves][B: three]
+      for (int h = 0; h < 2; h++) {  // stage h: [A: two 16 KB slice halves][B: two]
         unsigned char* st = smA + h * kPreStage;
         sm100::mbar_arrive_expect_tx(&pbar->full[h], (is_diag ? 1 : 2) * kTileSlices * kHalfBytes);
         for (int s2 = 0; s2 < kTileSlices; s2++)
@@ -356,9 +361,9 @@ __device__ __forceinline__ void dpanel_body(float4* sm4, float2* A, float* Ldg, 
           for (int s2 = 0; s2 < kTileSlices; s2++)
             sm100::bulk_g2s(st + s2 * kHalfBytes, gA + s2 * kSliceBytes + h * kHalfBytes, kHalfBytes, &pbar->full[h]);
       }
-      const uint32_t idesc = sm100::idesc_bf16_f32(128, 128);
-      const int pa[6] = {2, 1, 0, 1, 0, 0};  // (A slice, B slice) products, smallest first
-      const int pb[6] = {0, 1, 2, 0, 1, 0};
+      const uint32_t idesc = sm100::idesc_f16_f32(128, 128);
+      const int pa[3] = {1, 0, 0};  // (A slice, B slice) products, smallest first
+      const int pb[3] = {0, 1, 0};
       bool ok = true;
       for (int h = 0; h < 2 && ok; h++) {
         ok = sm100::mbar_wait(&pbar->full[h], 0, kWaitLimit);
@@ -367,16 +372,16 @@ __device__ __forceinline__ void dpanel_body(float4* sm4, float2* A, float* Ldg, 
         const unsigned char* sa = smA + h * kPreStage;
         const unsigned char* sb = sa + kTileSlices * kHalfBytes;
 #pragma unroll
-        for (int p = 0; p < 6; p++) {
+        for (int p = 0; p < 3; p++) {
           const uint32_t b0 = sm100::smem_u32(sb + pa[p] * kHalfBytes), b1 = sm100::smem_u32(sb + pb[p] * kHalfBytes);
           const uint32_t a0 = sm100::smem_u32(sa + pa[p] * kHalfBytes);
 #pragma unroll
           for (int kk = 0; kk < 4; kk++) {
             const uint32_t acc = (h | p | kk) != 0;
-            sm100::mma_bf16(tmem, sm100::desc_kmajor_sw128(b0 + kk * 32), sm100::desc_kmajor_sw128(b1 + kk * 32), idesc,
+            sm100::mma_f16(tmem, sm100::desc_kmajor_sw128(b0 + kk * 32), sm100::desc_kmajor_sw128(b1 + kk * 32), idesc,
                             acc);
             if (!is_diag)
-              sm100::mma_bf16(tmem + kT, sm100::desc_kmajor_sw128(a0 + kk * 32), sm100::desc_kmajor_sw128(b1 + kk * 32),
+              sm100::mma_f16(tmem + kT, sm100::desc_kmajor_sw128(a0 + kk * 32), sm100::desc_kmajor_sw128(b1 + kk * 32),
                               idesc, acc);
           }
         }
@@ -440,7 +445,8 @@ __device__ __forceinline__ void dpanel_body(float4* sm4, float2* A, float* Ldg, 
       for (int k4 = 0; k4 < 8; k4++) {
         float4* p4 = reinterpret_cast<float4*>(row + cc + 4 * k4);
         float4 x = *p4;
-        x.x -= v[4 * k4], x.y -= v[4 * k4 + 1], x.z -= v[4 * k4 + 2], x.w -= v[4 * k4 + 3];
+        x.x -= v[4 * k4] * iscale2, x.y -= v[4 * k4 + 1] * iscale2;
+        x.z -= v[4 * k4 + 2] * iscale2, x.w -= v[4 * k4 + 3] * iscale2;
         *p4 = x;
       }
     }
@@ -499,14 +505,14 @@ __device__ __forceinline__ void dpanel_body(float4* sm4, float2* A, float* Ldg, 
     DP_MARK(2 + 3 * jb);
     // B: the rows below the block, the rest of the diagonal block, then the
     // 128 tile rows; a tile row's 32 new entries of L_ik go out at once:
-    // back into A as (L, 0) pairs and as three BF16 slices, pre-swizzled
+    // back into A as (L, 0) pairs and as two FP16 slices, pre-swizzled
     // (consecutive lanes take consecutive rows, so the pair stores are
     // coalesced)
     if (tid < nd + nrt) {
       float x[32];
       dp_row_solve(&S[tid < nd ? c1 + tid : kT + tid - nd][c0], T, x);
       if (tid >= nd) dp_emit(x, tid - nd, part * rpc + tid - nd, nrows, c0, w, A + (size_t)(k0 + c0) * lda + row0, lda,
-                             PS + (size_t)tile * kTileBytes);
+                             PS + (size_t)tile * kTileBytes, scale);
     }
     __syncthreads();
     DP_MARK(3 + 3 * jb);
@@ -532,10 +538,10 @@ __device__ __forceinline__ void dpanel_body(float4* sm4, float2* A, float* Ldg, 
 // A_IJ -= L_I L_J^T for a run of up to `group` consecutive tiles per CTA
 // (row-major order over the tile triangle, so consecutive tiles share I and
 // the A operand stays in shared memory).  Warp-specialised, pipelined:
-//   warp 0 (one lane)  bulk-async copies: the three A slices when I changes,
-//                      the three B slices per tile in two K-halves (two
-//                      48 KB stages), and an L2 prefetch of the FP64 tile;
-//   warp 1 (one lane)  six BF16 products per K-half into one of two TMEM
+//   warp 0 (one lane)  bulk-async copies: the two A slices when I changes,
+//                      the two B slices per tile in two K-halves (two
+//                      32 KB stages), and an L2 prefetch of the FP64 tile;
+//   warp 1 (one lane)  three FP16 products per K-half into one of two TMEM
 //                      accumulators (128 columns each), tcgen05.commit to
 //                      release stages, the accumulator and the A operand;
 //   warps 2-9          epilogue: tcgen05.ld of the accumulator (warp w reads
@@ -570,8 +576,9 @@ __device__ __forceinline__ void dpanel_body(float4* sm4, float2* A, float* Ldg, 
 #define BD_REST_GMAX 8
 #endif
 constexpr int kRestThreads = 320;
-constexpr int kStageBytes = kTileSlices * kHalfBytes;  // one K-half of the three B slices
-constexpr size_t kRestSmem = (size_t)kTileBytes + 2 * kStageBytes + 1024 + 256;
+constexpr int kStageBytes = kTileSlices * kHalfBytes;  // one K-half of the two B slices
+constexpr size_t kRestSmem = kPreBarOff + 2 * 1024;
+static_assert(kRestSmem >= (size_t)kTileBytes + 2 * kStageBytes + 1024 + 256, "the update CTAs' operands");
 constexpr int kAccCols = 128;
 
 struct RestBars {
@@ -599,15 +606,15 @@ __device__ __forceinline__ void rest_tile(int t, int jlo, int mode, int nt, int&
 // NPAN = 1: one panel's update, the A operand resident per row of tiles.
 // NPAN = 2, 3: two or three consecutive panels' updates (PS, PS2, PS3) in one
 // read-modify-write of the tile (K = 256, 384): both operands streamed in
-// 2 NPAN chunks of 96 KB per tile (panel, K-half) through the two stages.
+// 2 NPAN chunks of 64 KB per tile (panel, K-half) through the two stages.
 template <int NPAN>
 __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int lda, int m, int jlo, int mode,
                                           int tlo, int thi, int group, int cta, const unsigned char* __restrict__ PS,
                                           const unsigned char* __restrict__ PS2, const unsigned char* __restrict__ PS3,
-                                          int* err) {
+                                          int* err, float iscale2) {
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smraw) + 1023) & ~uintptr_t(1023));
-  unsigned char* sA = sm;                 // 3 slices x 32 KB
-  unsigned char* sB = sm + kTileBytes;    // 2 stages x (3 slices x 16 KB)
+  unsigned char* sA = sm;                 // 2 slices x 32 KB
+  unsigned char* sB = sm + kTileBytes;    // 2 stages x (2 slices x 16 KB)
   RestBars* bars = reinterpret_cast<RestBars*>(sm + kTileBytes + 2 * kStageBytes);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tslot + 1);
@@ -730,9 +737,9 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
     if (lane == 0) {
       // ---------------- MMA issuer
       if constexpr (NPAN == 1) {
-      const uint32_t idesc = sm100::idesc_bf16_f32(128, 128);
-      const int pa[6] = {2, 1, 0, 1, 0, 0};  // (A slice, B slice) products, smallest first
-      const int pb[6] = {0, 1, 2, 0, 1, 0};
+      const uint32_t idesc = sm100::idesc_f16_f32(128, 128);
+      const int pa[3] = {1, 0, 0};  // (A slice, B slice) products, smallest first
+      const int pb[3] = {0, 1, 0};
       int curI = -1;
       uint32_t nA = 0;
       bool ok = true;
@@ -759,13 +766,13 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
           if (!ok) break;
           sm100::tc_fence_after();
 #pragma unroll
-          for (int p = 0; p < 6; p++) {
+          for (int p = 0; p < 3; p++) {
             const uint32_t aaddr = sm100::smem_u32(sA + pa[p] * kSliceBytes + h * kHalfBytes);
             const uint32_t baddr = (I == J) ? sm100::smem_u32(sA + pb[p] * kSliceBytes + h * kHalfBytes)
                                             : sm100::smem_u32(sB + h * kStageBytes + pb[p] * kHalfBytes);
 #pragma unroll
             for (int kk = 0; kk < 4; kk++)
-              sm100::mma_bf16(d, sm100::desc_kmajor_sw128(aaddr + kk * 32), sm100::desc_kmajor_sw128(baddr + kk * 32),
+              sm100::mma_f16(d, sm100::desc_kmajor_sw128(aaddr + kk * 32), sm100::desc_kmajor_sw128(baddr + kk * 32),
                               idesc, (h | p | kk) != 0);
           }
           sm100::mma_commit(&bars->emptyB[h]);
@@ -781,9 +788,9 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
         *abort_flag = 1;
       }
       } else {
-        const uint32_t idesc = sm100::idesc_bf16_f32(128, 128);
-        const int pa[6] = {2, 1, 0, 1, 0, 0};
-        const int pb[6] = {0, 1, 2, 0, 1, 0};
+        const uint32_t idesc = sm100::idesc_f16_f32(128, 128);
+        const int pa[3] = {1, 0, 0};
+        const int pb[3] = {0, 1, 0};
         uint32_t nuse[2] = {0, 0};
         int ctot = 0;
         bool ok = true;
@@ -808,12 +815,12 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
             const unsigned char* sa = sm + st * (2 * kStageBytes);
             const unsigned char* sb = dg ? sa : sa + kStageBytes;
 #pragma unroll
-            for (int p = 0; p < 6; p++) {
+            for (int p = 0; p < 3; p++) {
               const uint32_t aaddr = sm100::smem_u32(sa + pa[p] * kHalfBytes);
               const uint32_t baddr = sm100::smem_u32(sb + pb[p] * kHalfBytes);
 #pragma unroll
               for (int kk = 0; kk < 4; kk++)
-                sm100::mma_bf16(d, sm100::desc_kmajor_sw128(aaddr + kk * 32),
+                sm100::mma_f16(d, sm100::desc_kmajor_sw128(aaddr + kk * 32),
                                 sm100::desc_kmajor_sw128(baddr + kk * 32), idesc, (q | p | kk) != 0);
             }
             sm100::mma_commit(&bars->emptyB[st]);
@@ -913,7 +920,7 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
         const float* v = vt + kEpC * (c % kEpR);
 #pragma unroll
         for (int j = 0; j < kEpC; j++)
-          if (kEpC * c + j < jcnt) st_tile(colp + (size_t)(kEpC * c + j) * lda, df_sub(old[s2][j], v[j]));
+          if (kEpC * c + j < jcnt) st_tile(colp + (size_t)(kEpC * c + j) * lda, df_sub(old[s2][j], v[j] * iscale2));
         if (c + kEpS < kEpN) load_chunk(old[s2], colp, jcnt, c + kEpS);
         else if (more) load_chunk(old[s2], ncolp, njcnt, c + kEpS - kEpN);
       }
@@ -942,6 +949,7 @@ struct StepArgs {
   int* negpiv;
   int* err;
   int lda, m, ndp, pk0, pkb;
+  float scale, iscale2;  // the slices hold scale * L; iscale2 = scale^-2 (powers of two)
   int prows;  // tile rows per panel CTA (128, or 64 when the panel is split over twice the CTAs)
   UpdJob job[2];
 };
@@ -953,7 +961,7 @@ struct StepArgs {
 __device__ __forceinline__ void chol_step_body(const StepArgs& a, int b, float4* smem4) {
   if (b < a.ndp) {
     dpanel_body(smem4, a.A, a.Ldg, a.lda, a.m, a.pk0, a.pkb, a.pk0 / kT + 1, b, a.PSp, a.negpiv, a.PSpre, a.err,
-                a.prows);
+                a.prows, a.scale, a.iscale2);
     return;
   }
   b -= a.ndp;
@@ -962,13 +970,13 @@ __device__ __forceinline__ void chol_step_body(const StepArgs& a, int b, float4*
   const UpdJob& j = a.job[jn];
   if (j.ps3)
     rest_body<3>(reinterpret_cast<unsigned char*>(smem4), a.A, a.lda, a.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b,
-                 j.ps, j.ps2, j.ps3, a.err);
+                 j.ps, j.ps2, j.ps3, a.err, a.iscale2);
   else if (j.ps2)
     rest_body<2>(reinterpret_cast<unsigned char*>(smem4), a.A, a.lda, a.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b,
-                 j.ps, j.ps2, nullptr, a.err);
+                 j.ps, j.ps2, nullptr, a.err, a.iscale2);
   else
     rest_body<1>(reinterpret_cast<unsigned char*>(smem4), a.A, a.lda, a.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b,
-                 j.ps, nullptr, nullptr, a.err);
+                 j.ps, nullptr, nullptr, a.err, a.iscale2);
 }
 
 __global__ void __launch_bounds__(kRestThreads, 1) k_chol_step(const __grid_constant__ StepArgs a) {
@@ -1029,6 +1037,20 @@ size_t mixed_panel_bytes(int m) {  // the slice buffers, then the diagonal facto
 }
 int mixed_max_launches(int m) { return 2 * cdiv(m, kT) + 2; }
 int mixed_tiles(int m) { return cdiv(m, kT); }
+
+// |L_ij| <= sqrt(max D_ii): the slices' largest value is put into [2^8, 2^9),
+// so values down to 2^-34 of it stay in the pair (FP16's smallest subnormal
+// is 2^-24) and a factor with replaced negative pivots has 2^7 of room
+// before the clamp.  Radii that give no finite positive diagonal: 1.
+float mixed_scale(double a1, const double* rad, int nrad) {
+  double dmax = 0.0;
+  for (int i = 0; i < nrad; i++) dmax = std::max(dmax, std::fabs(a1 / rad[i]));
+  if (!(dmax > 0.0) || !std::isfinite(dmax)) return 1.f;
+  int e = 0;
+  std::frexp(std::sqrt(dmax), &e);  // sqrt(dmax) in [2^(e-1), 2^e)
+  e = 9 - e;
+  return std::ldexp(1.f, e > 60 ? 60 : (e < -60 ? -60 : e));
+}
 
 static bool g_attr_done = false;
 
@@ -1104,7 +1126,7 @@ struct Job {
 // most accurate.
 static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int* negpiv, int* err, cudaStream_t st,
                             cudaEvent_t* kev, int* kev_pairs, double* kflop, double* kbytes,
-                            std::vector<std::pair<StepArgs, int>>* plan, int max_pass) {
+                            std::vector<std::pair<StepArgs, int>>* plan, int max_pass, float scale) {
   float2* A = reinterpret_cast<float2*>(A64);  // double-float storage, 8 bytes per element
   const int nt = cdiv(m, kT);
   const size_t buf = (size_t)nt * kTileBytes;
@@ -1140,6 +1162,7 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
   auto launch = [&](int pn, const Job& j0, const Job& j1, bool pre) {
     StepArgs a{};
     a.A = A, a.negpiv = negpiv, a.err = err, a.lda = lda, a.m = m;
+    a.scale = scale, a.iscale2 = 1.f / (scale * scale);
     a.Ldg = Ld, a.PSp = PS, a.PSpre = nullptr, a.prows = kT;
     if (pn >= 0) {
       // the panel over twice the CTAs (64 tile rows each) when they fit on
@@ -1175,12 +1198,12 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
     L++;
     if (kbytes || kflop) {
       double by = pn >= 0 ? 16.0 * (double)(m - pn * kT) * kb_of(pn) : 0.0;  // panel read and written back
-      double fl = a.PSpre ? 6.0 * 2.0 * kT * kT * kT * (2 * a.ndp - 1) : 0.0;  // the panel CTAs' own products
+      double fl = a.PSpre ? 3.0 * 2.0 * kT * kT * kT * (2 * a.ndp - 1) : 0.0;  // the panel CTAs' own products
       for (int q = 0; q < 2; q++) {
         const Job& j = *js[q];
         if (j.tiles <= 0) continue;
         by += 16.0 * elems(j.jlo, j.mode == kCol ? j.jlo + 1 : nt);  // double-float tile read + write
-        fl += 6.0 * 2.0 * kT * kT * kT * j.tiles * (j.ps3 ? 3 : (j.ps2 ? 2 : 1));  // BF16 tensor work issued
+        fl += 3.0 * 2.0 * kT * kT * kT * j.tiles * (j.ps3 ? 3 : (j.ps2 ? 2 : 1));  // FP16 tensor work issued
       }
       if (kbytes) *kbytes += by;
       if (kflop) *kflop += fl;
@@ -1212,8 +1235,8 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
 }
 
 int potrf_mixed(int m, double* A64, int lda, unsigned char* PS, int* negpiv, int* err, cudaStream_t st,
-                cudaEvent_t* kev, int* kev_pairs, double* kflop, double* kbytes, int max_pass) {
-  return potrf_mixed_impl(m, A64, lda, PS, negpiv, err, st, kev, kev_pairs, kflop, kbytes, nullptr, max_pass);
+                cudaEvent_t* kev, int* kev_pairs, double* kflop, double* kbytes, int max_pass, float scale) {
+  return potrf_mixed_impl(m, A64, lda, PS, negpiv, err, st, kev, kev_pairs, kflop, kbytes, nullptr, max_pass, scale);
 }
 
 // Factorisations of a batch advanced together: launch i of the batch runs
@@ -1233,7 +1256,7 @@ struct MixedBatch {
 };
 
 MixedBatch* mixed_batch_create(int nrep, const int* m, double* const* A, const int* lda, unsigned char* const* PS,
-                               int* const* negpiv, int* const* err, int max_pass) {
+                               int* const* negpiv, int* const* err, const float* scale, int max_pass) {
   std::vector<std::vector<std::pair<StepArgs, int>>> plans(nrep);
   size_t steps = 0;
   MixedBatch* b = new MixedBatch();
@@ -1241,7 +1264,7 @@ MixedBatch* mixed_batch_create(int nrep, const int* m, double* const* A, const i
   std::vector<ScatterArgs> sc(nrep);
   for (int r = 0; r < nrep; r++) {
     potrf_mixed_impl(m[r], A[r], lda[r], PS[r], negpiv[r], err[r], nullptr, nullptr, nullptr, nullptr, nullptr,
-                     &plans[r], max_pass);
+                     &plans[r], max_pass, scale[r]);
     steps = std::max(steps, plans[r].size());
     const int nt = cdiv(m[r], kT);
     b->max_nt = std::max(b->max_nt, nt);

@@ -46,7 +46,7 @@ const char* bd_version(void);
 enum {
   BD_PREC_FP64 = 0,   /* plain FP64 step: parity path against the FP64 oracle */
   BD_PREC_MIXED = 1   /* FP32-class: RPY tensor in FP32 into double-float storage, Cholesky with
-                         FP32 panels and BF16x3 tensor-core (tcgen05) trailing updates, FP32
+                         FP32 panels and FP16-pair tensor-core (tcgen05) trailing updates, FP32
                          pair forces with compensated sums; no refinement.  Displacement
                          4e-7 to 8e-7 from the FP64 path on the benchmark fibers; up to
                          1.3e-6 on 3 of 256 uneven batch replicas (bd_set_mixed_passes) */
@@ -373,7 +373,7 @@ int bd_batch_run_device(bd_batch* b, int nsteps, unsigned long seed_base, double
 int bd_phase_times(bd_ctx* ctx, float* out9);
 /* Mixed path: total device time (CUDA events on the context's stream) of
  * the tensor-core trailing-update launches of the last step run with
- * timing enabled (see bd_phase_times), their number, and the BF16 tensor
+ * timing enabled (see bd_phase_times), their number, and the FP16 tensor
  * work they issued (flop). */
 int bd_kernel_time(bd_ctx* ctx, float* total_ms, int* launches, double* tensor_flop);
 /* The same launches one by one: out_ms[i] for i < min(max, launches), in
