@@ -5,16 +5,14 @@
 // element, ~48 significant bits), so the trailing updates accumulate without
 // an FP32 rounding per panel and without FP64 arithmetic (GB300's FP64 rate
 // is ~2 operations per clock per SM); the arithmetic is FP32-class.  One
-// kernel, k_chol_step, runs two kinds of CTA side by side:
-//   panel CTAs   factor the next panel: every one factors the 128 x 128
-//                diagonal block in shared memory (FP32, 32-column blocks),
-//                CTA 0 keeps it in a side buffer (copied into A after the
-//                last panel) and the others solve one 128-row tile each,
-//                L_ik = A_ik L_kk^-T, by forward substitution, write it back
-//                and split it into two FP16 slices (scaled by one power of
+// kernel, k_chol_step, runs these kinds of CTA side by side:
+//   panel CTAs   solve panel k's tiles, L_ik = A_ik L_kk^-T, write them back
+//                and split them into two FP16 slices (scaled by one power of
 //                two: hi + lo = the FP32 value to 2^-24), stored pre-swizzled
-//                in the 128-byte-swizzle K-major layout the MMA reads; a
-//                negative pivot is replaced by its absolute value and counted
+//                in the 128-byte-swizzle K-major layout the MMA reads; one of
+//                them, the chain CTA, then factors diagonal block k + 1 and
+//                inverts the factor for the next launch.  A negative pivot is
+//                replaced by its absolute value and counted
 //                (func.cpp:827-833).
 //   update CTAs  trailing update A_IJ -= L_I L_J^T of one or two earlier
 //                panels, a run of tiles per CTA, warp-specialised:
@@ -35,6 +33,7 @@
 // records an error code, frees its tensor memory and returns.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -66,17 +65,17 @@ __device__ __forceinline__ uint32_t swz_off(int r, int k) {
 }
 
 // Two scaled FP32 values as FP16 pairs: x = hi + lo to 2^-24 |x| (two
-// roundings to 11 bits each), low half first.  A finite value past FP16's
-// range (see the scale at StepArgs) is clamped; Inf and NaN stay.
+// roundings to 11 bits each), low half first.  Values past FP16's range (a
+// factor with replaced negative pivots, see mixed_scale) saturate; NaN stays.
+__device__ __forceinline__ uint32_t cvt_f16x2(float x0, float x1) {
+  uint32_t r;
+  asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(x1), "f"(x0));
+  return r;
+}
 __device__ __forceinline__ void split_f16x2(float x0, float x1, uint32_t& hi, uint32_t& lo) {
-  const float lim = 65504.f;
-  if (fabsf(x0) > lim && !isinf(x0)) x0 = copysignf(lim, x0);
-  if (fabsf(x1) > lim && !isinf(x1)) x1 = copysignf(lim, x1);
-  const __half2 h = __floats2half2_rn(x0, x1);
-  const float2 hf = __half22float2(h);
-  const __half2 l = __floats2half2_rn(x0 - hf.x, x1 - hf.y);
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  lo = *reinterpret_cast<const uint32_t*>(&l);
+  hi = cvt_f16x2(x0, x1);
+  const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+  lo = cvt_f16x2(x0 - hf.x, x1 - hf.y);
 }
 
 // (hi, lo) - v in double-float arithmetic: exact two-sums (Knuth), so the
@@ -93,445 +92,625 @@ __device__ __forceinline__ float2 df_sub(float2 a, float v) {
   return make_float2(h, l);
 }
 
-// ------------------------------------------------------------ diagonal block + panel
-// Panel k runs in CTAs of the step launch: every panel CTA loads the
-// 128 x 128 diagonal block and factors it in shared memory (the factor is
-// recomputed by each CTA instead of being passed between CTAs); CTA 0 keeps
-// L_kk, CTA b >= 1 also solves the 128-row tile k + b:  X L_kk^T = A_ik.
-//
-// The diagonal block and the tile are one tall 256-row panel in shared memory
-// (rows 0..127 the diagonal block, 128..255 the tile), factored in 32-column
-// blocks, left-looking across blocks: block column j first takes
-//   S[r][c] -= sum_{q < 32 j} S[r][q] L[c][q]
-// as one FP32 dot product per element (register-tiled, 7 rows x 4 columns per
-// thread), then the 32 x 32 diagonal block is factored by one warp in
-// registers and every row below it (diagonal-block rows and tile rows alike)
-// is solved by forward substitution, one row per thread.  A negative pivot is
-// replaced by its absolute value and counted (func.cpp:827-833), by CTA 0 only.
-constexpr int kLd = 132;             // shared row stride (floats): 16-byte rows, conflict-free 4-wide loads
-constexpr int kLt = 36;              // row stride of the transposed 32 x 32 factor
-constexpr int kDpThreads = 256;
-constexpr size_t kDpSmem = (2 * (size_t)kT * kLd + 32 * kLt) * sizeof(float);
+// ------------------------------------------------------------ one panel
+// Launch k of the factorisation solves panel k's tiles and factors diagonal
+// block k + 1:
+//   tile CTAs   L_ik = A_ik W_k^T with W_k = L_kk^-1 from the launch before:
+//               a product on the tensor cores in place of a substitution.
+//               The tile first takes panel k - 1's update (D = L_i,k-1
+//               L_k,k-1^T), also there.
+//   chain CTA   the same for the tile below the diagonal, then diagonal block
+//               k + 1 with the updates of panels k - 1 and k, its Cholesky
+//               factor (written into A) and that factor's inverse W_k+1.
+// So the serial chain of a factorisation is one CTA's work per panel, and no
+// CTA repeats another's.  Bound by that chain: 26 us (copies and the panel
+// k - 1 product 3, the tile and its products 5, the 128 columns 15, the last
+// of W 1) beside 9 us of the other tiles, and ~3 us between launches.  Before,
+// every panel CTA factored the diagonal block itself and solved its rows by
+// substitution, 41 us.  A step of 3N = 1,944: 1.13 -> 0.94 ms, 3N = 3,888:
+// 1.86 -> 1.43, 3N = 11,700: 7.6 -> 5.8 (with the FP16 slices); 24 replicas,
+// where the repeated work also filled the GPU: 28.7 -> 19.0.
+// The explicit inverse is as accurate as the substitution here (condition
+// numbers of L_kk below 10): error of L p against FP64, 2-norm over 13 fibers
+// of 3N 912 .. 11,700: 2.6e-7 .. 5.4e-7 before, 2.5e-7 .. 5.1e-7 now.
+constexpr int kLd = 132;  // row stride (floats) of the diagonal block in shared memory: conflict-free 16-byte rows
+constexpr int kChainS = kTileBytes;                  // shared-memory offset of the FP32 diagonal block
+constexpr int kChainW = 130 * 1024;                  // ... and of the inverse's slices
+constexpr int kPanelMisc = kChainW + kTileBytes;     // ... and of the barriers
+static_assert(kChainS + kT * kLd * 4 <= kChainW, "the diagonal block lies before the inverse's slices");
 
-#ifndef BD_DP_EVICT_FIRST
-#define BD_DP_EVICT_FIRST 1  // L2 evict-first hint on the panel's tile loads and (L, 0) stores
-#endif
-#ifndef DP_MARK
-#define DP_MARK(i)  // phase boundary of the panel CTAs (a timestamp hook for profiling builds)
-#endif
+struct PanelBars {
+  uint64_t fullPre, fullW, preDone, sReady, xDone, lReady, qDone, r0Free, trDone[3], trRest[2], helped[2], step[16];
+  uint32_t slot;
+  float rowf[2][kT];                 // undoes the scales of a row's rank-32 product (panel P in buffer P & 1)
+  alignas(16) float xsc[kT];         // X = D * xsc, by column
+  alignas(16) float dg[16][8][8];    // the 8 x 8 diagonal blocks, then L's
+};
+constexpr size_t kPanelSmem = kPanelMisc + sizeof(PanelBars) + 1024;
 
-// Row v of the block-column update: v < nd are diagonal-block rows c0 + v,
-// the rest tile rows kT + (v - nd); -1 past the end.
-__device__ __forceinline__ int dp_row(int v, int c0, int nd, int nv) {
-  return v < nd ? c0 + v : (v < nv ? kT + v - nd : -1);
+// The next 1024-byte boundary of shared memory, by an offset from smraw: a
+// pointer rounded as an integer is no longer known to be shared, and every
+// access through it becomes a generic one (the 128-column factorisation took
+// four times as long).
+__device__ __forceinline__ unsigned char* align1024(unsigned char* smraw) {
+  return smraw + ((0u - sm100::smem_u32(smraw)) & 1023u);
 }
 
-// S[r][c] -= sum_{qlo <= q < qhi} S[r][q] * S[c][q] for the nv rows of block
-// column c0 (c in [c0, c0 + w)), lower part only inside the diagonal block;
-// t in [0, 256) is the thread's index among the 256 taking part.  NI row
-// groups of 32 (nv <= 32 NI); the operands of step q + 4 are loaded while
-// step q's products are formed, and the products are issued component by
-// component so that consecutive FMAs are independent.
-template <int NI>
-__device__ __forceinline__ void dp_block_update_n(float (*S)[kLd], int t, int c0, int w, int nd, int nv, int qlo,
-                                                  int qhi) {
-  const int g = t & 7, rg = t >> 3;  // 8 column groups x 32 row groups
-  int rows[NI];
-  const float* xr[NI];
-  const float* lr[4];
-  float acc[NI][4];
+// 128 consecutive K of one product: D (+)= A B^T from slice operands at sa, sb
+// (two slices each), smallest products first.
+__device__ __forceinline__ void mma_tile(uint32_t d, const unsigned char* sa, const unsigned char* sb, bool acc) {
+  const uint32_t idesc = sm100::idesc_f16_f32(128, 128);
+  const int pa[3] = {1, 0, 0};  // (A slice, B slice)
+  const int pb[3] = {0, 1, 0};
 #pragma unroll
-  for (int i = 0; i < NI; i++) {
-    rows[i] = dp_row(rg + 32 * i, c0, nd, nv);
-    xr[i] = S[rows[i] < 0 ? 0 : rows[i]];  // rows past the end read row 0; their sums are dropped
+  for (int h = 0; h < 2; h++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+    for (int p = 0; p < 3; p++) {
+      const uint32_t aaddr = sm100::smem_u32(sa + pa[p] * kSliceBytes + h * kHalfBytes);
+      const uint32_t baddr = sm100::smem_u32(sb + pb[p] * kSliceBytes + h * kHalfBytes);
+#pragma unroll
+      for (int kk = 0; kk < 4; kk++)
+        sm100::mma_f16(d, sm100::desc_kmajor_sw128(aaddr + kk * 32), sm100::desc_kmajor_sw128(baddr + kk * 32), idesc,
+                       acc || (h | p | kk) != 0);
+    }
+}
+
+// 8 consecutive columns (from column c, c % 8 == 0) of row r of a slice pair at `base`
+__device__ __forceinline__ void put_slices8(unsigned char* base, int r, int c, const float (&x)[8]) {
+  uint32_t h[4], l[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) split_f16x2(x[2 * j], x[2 * j + 1], h[j], l[j]);
+  const uint32_t off = swz_off(r, c);
+  *reinterpret_cast<uint4*>(base + off) = make_uint4(h[0], h[1], h[2], h[3]);
+  *reinterpret_cast<uint4*>(base + kSliceBytes + off) = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+// The 8 x 8 diagonal block `dg` (lower part read) factored into d; x, a row of
+// the panel, solved against it.  Returns the number of negative pivots, each
+// replaced by its absolute value (func.cpp:827-833).
+__device__ __forceinline__ int factor8(const float (*dg)[8], float (&d)[8][8], float* x) {
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+#pragma unroll
+    for (int h = 0; h <= (i >> 2); h++) {
+      const float4 v = *reinterpret_cast<const float4*>(&dg[i][4 * h]);
+      d[i][4 * h] = v.x, d[i][4 * h + 1] = v.y, d[i][4 * h + 2] = v.z, d[i][4 * h + 3] = v.w;
+    }
+  int neg = 0;
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const float ad = fabsf(d[j][j]);
+    if (d[j][j] < 0.f) neg++;
+    const float rp = rsqrtf(ad);
+    d[j][j] = ad * rp;
+    x[j] *= rp;
+#pragma unroll
+    for (int i = j + 1; i < 8; i++) {
+      d[i][j] *= rp;
+      x[i] = fmaf(-x[j], d[i][j], x[i]);
+    }
+#pragma unroll
+    for (int i = j + 1; i < 8; i++)
+#pragma unroll
+      for (int l = j + 1; l <= i; l++) d[i][l] = fmaf(-d[i][j], d[l][j], d[i][l]);
   }
+  return neg;
+}
+
+constexpr int kTrSlice = 16 * 1024;  // one slice of a 128 x 32 operand, in 128-byte rows
+
+// Cholesky factor and inverse of the 128 x 128 block in S (row stride kLd; its
+// first 32 columns in x).  Four warps, a thread a row (r, its tensor-memory
+// lane too), in four panels of 32 columns that the thread keeps in registers:
+//   - 16 steps of eight columns: the 8 x 8 diagonal block goes through shared
+//     memory, every thread factors it (all the same) and solves its own row
+//     against it; the rows' values go to S, and every thread takes them off
+//     the rest of its panel, one column after the other.
+//   - the columns right of a panel take its rank-32 update on the tensor cores
+//     (FP16 pairs as the tiles' slices), this thread's next panel at once, the
+//     later columns by four helper warps (chol_help) beside the next panel.
+// A row above a step's block has been eliminated and carries the inverse
+// instead: row r of X = L^-T, started as the unit row in its own step, takes
+// the same solves and updates (in the rank-32 product with a scale of its
+// own: X's rows differ in size).  At the end S holds L below the 8 x 8
+// diagonal blocks, X on and above them; L's 8 x 8 blocks are in dg.  step[q]
+// is arrived at when step q's columns are final.
+// Bound by the chain of a step (two barriers, three shared-memory round trips,
+// eight reciprocal roots) and by the 16-byte loads of L's values, four cycles
+// of shared memory each however few of the bytes differ: eight columns a step
+// and rows in registers need the fewest of them (a register-tiled block with
+// four columns a step: 1.5 times longer).  neg += negative pivots.
+__device__ __forceinline__ void chol_inv128(float (*S)[kLd], PanelBars* bars, unsigned char* T, uint32_t tmem,
+                                            float (&x)[32], int r, int lane, float scale, int& neg, bool& ok) {
+  const float iscale = 1.f / scale;
+  const uint32_t trow = tmem + ((uint32_t)(r & ~31) << 16);
+  // x[j0 .. j1) of the panel P less the step s's columns; mk: 0 for a row that
+  // the step eliminated (it starts as a row of X), else 1 (a product: as a
+  // select it became a branch, 3 us a panel)
+  auto upd = [&](int P, auto sc, auto j0c, auto j1c, float mk) {
+    constexpr int s = decltype(sc)::value, j0 = decltype(j0c)::value, j1 = decltype(j1c)::value;
 #pragma unroll
-  for (int j = 0; j < 4; j++) lr[j] = S[c0 + g + 8 * j];
-  float4 lv[4], xv[NI];
+    for (int j = j0; j < j1; j++) {
+      const float4 l0 = *reinterpret_cast<const float4*>(&S[32 * P + j][32 * P + 8 * s]);
+      const float4 l1 = *reinterpret_cast<const float4*>(&S[32 * P + j][32 * P + 8 * s + 4]);
+      const float l[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+      x[j] *= mk;
 #pragma unroll
-  for (int j = 0; j < 4; j++) lv[j] = *reinterpret_cast<const float4*>(lr[j] + qlo);
+      for (int e = 0; e < 8; e++) x[j] = fmaf(-x[8 * s + e], l[e], x[j]);
+    }
+  };
+#pragma unroll 1
+  for (int P = 0; P < 4; P++) {
+    const bool mine = (r >> 5) == P;  // the panel's diagonal rows
+    float rho = scale, f = iscale * iscale;
+    auto step = [&](auto sc) {
+      constexpr int s = decltype(sc)::value;
+      const int q = 4 * P + s, c = 8 * q;  // (x[8 s ..] are columns c ..)
+      const bool blk = mine && (lane >> 3) == s;
+      float (*dg)[8] = bars->dg[q];
+      if (blk) {
+        *reinterpret_cast<float4*>(&dg[lane & 7][0]) = make_float4(x[8 * s], x[8 * s + 1], x[8 * s + 2], x[8 * s + 3]);
+        *reinterpret_cast<float4*>(&dg[lane & 7][4]) = make_float4(x[8 * s + 4], x[8 * s + 5], x[8 * s + 6], x[8 * s + 7]);
+      }
+      asm volatile("bar.sync 2, 128;" ::: "memory");
+      // the step before's update of the columns past this step's, beside this chain
+      if constexpr (s > 0)
+        upd(P, std::integral_constant<int, s - 1>{}, std::integral_constant<int, 8 * s + 8>{},
+            std::integral_constant<int, 32>{}, mine && (lane >> 3) == s - 1 ? 0.f : 1.f);
+      if (blk) {  // the block's own rows: unit rows from here on
 #pragma unroll
-  for (int i = 0; i < NI; i++) xv[i] = *reinterpret_cast<const float4*>(xr[i] + qlo);
-#pragma unroll 2
-  for (int q = qlo; q < qhi; q += 4) {
-    const int qn = (q + 4 < qhi) ? q + 4 : q;
-    float4 ln[4], xn[NI];
+        for (int j = 0; j < 8; j++) x[8 * s + j] = (lane & 7) == j ? 1.f : 0.f;
+      }
+      float d[8][8];
+      neg += factor8(dg, d, &x[8 * s]);
+      *reinterpret_cast<float4*>(&S[r][c]) = make_float4(x[8 * s], x[8 * s + 1], x[8 * s + 2], x[8 * s + 3]);
+      *reinterpret_cast<float4*>(&S[r][c + 4]) = make_float4(x[8 * s + 4], x[8 * s + 5], x[8 * s + 6], x[8 * s + 7]);
+      if constexpr (s == 3) {  // the scale of this row in the rank-32 product
+        if (mine) {  // a row eliminated in this panel takes part as a row of X alone
 #pragma unroll
-    for (int j = 0; j < 4; j++) ln[j] = *reinterpret_cast<const float4*>(lr[j] + qn);
+          for (int j = 0; j < 24; j++)
+            if (j < (lane & 24)) x[j] = 0.f;
+        }
+        if ((r >> 5) <= P) {
+          float m[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int i = 0; i < NI; i++) xn[i] = *reinterpret_cast<const float4*>(xr[i] + qn);
+          for (int j = 0; j < 32; j++) m[j & 3] = fmaxf(m[j & 3], fabsf(x[j]));
+          m[0] = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+          int e = 13 + 127 - (int)(__float_as_uint(m[0]) >> 23);
+          if (!(m[0] > 0.f) || isinf(m[0]) || e > 100 || e < -100) e = 0;
+          rho = __uint_as_float((uint32_t)(127 + e) << 23);
+          f = __uint_as_float((uint32_t)(127 - e) << 23) * iscale;
+        }
+        bars->rowf[P & 1][r] = f;  // (the buffer's last readers are done: helped[P - 2])
+      }
+      asm volatile("bar.sync 2, 128;" ::: "memory");
+      if (lane == 0 && (r >> 5) == 0) {
+        sm100::mbar_arrive(&bars->step[q]);
+        // L's block in place of the diagonal block, which every thread has
+        // read before the second barrier
 #pragma unroll
-    for (int i = 0; i < NI; i++)
+        for (int i = 0; i < 8; i++)
 #pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] = fmaf(xv[i].x, lv[j].x, acc[i][j]);
+          for (int h = 0; h < 2; h++)
+            *reinterpret_cast<float4*>(&dg[i][4 * h]) =
+                make_float4(i >= 4 * h ? d[i][4 * h] : 0.f, i > 4 * h ? d[i][4 * h + 1] : 0.f,
+                            i > 4 * h + 1 ? d[i][4 * h + 2] : 0.f, i > 4 * h + 2 ? d[i][4 * h + 3] : 0.f);
+      }
+      if constexpr (s < 3)  // the next step's columns
+        upd(P, sc, std::integral_constant<int, 8 * s + 8>{}, std::integral_constant<int, 8 * s + 16>{}, blk ? 0.f : 1.f);
+    };
+    step(std::integral_constant<int, 0>{});
+    step(std::integral_constant<int, 1>{});
+    step(std::integral_constant<int, 2>{});
+    step(std::integral_constant<int, 3>{});
+    if (P == 3) break;
+    // the rank-32 product: D[r][n] = row r of the panel . row 32 (P + 1) + n
+    // T is free: the tile's slices have been copied, the panel before's products
+    // formed and taken from tensor memory (its later columns, into S, by chol_help)
+    ok = sm100::mbar_wait(P == 0 ? &bars->r0Free : &bars->helped[P - 1], 0, kWaitLimit) && ok;
 #pragma unroll
-    for (int i = 0; i < NI; i++)
+    for (int j8 = 0; j8 < 4; j8++) {
+      uint32_t h[4], l[4];
 #pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] = fmaf(xv[i].y, lv[j].y, acc[i][j]);
+      for (int j = 0; j < 4; j++) split_f16x2(x[8 * j8 + 2 * j] * rho, x[8 * j8 + 2 * j + 1] * rho, h[j], l[j]);
+      const uint32_t off = swz_off(r, 8 * j8);
+      *reinterpret_cast<uint4*>(T + off) = make_uint4(h[0], h[1], h[2], h[3]);
+      *reinterpret_cast<uint4*>(T + kTrSlice + off) = make_uint4(l[0], l[1], l[2], l[3]);
+    }
+    sm100::fence_proxy_async();
+    sm100::tc_fence_before();
+    asm volatile("bar.sync 2, 128;" ::: "memory");
+    if (lane == 0 && (r >> 5) == 0) {
+      sm100::tc_fence_after();
+      // the next panel's columns, then the later ones
+      const uint32_t ta = sm100::smem_u32(T), tb = ta + 4096u * (P + 1);
 #pragma unroll
-    for (int i = 0; i < NI; i++)
+      for (int n = 0; n < 2; n++) {
+        if (n == 1 && P == 2) break;
+        const uint32_t idesc = sm100::idesc_f16_f32(128, n == 0 ? 32 : 64 - 32 * P);
 #pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] = fmaf(xv[i].z, lv[j].z, acc[i][j]);
+        for (int p = 0; p < 3; p++)
 #pragma unroll
-    for (int i = 0; i < NI; i++)
+          for (int kk = 0; kk < 2; kk++)
+            sm100::mma_f16(tmem + 32 * n, sm100::desc_kmajor_sw128(ta + (p == 0 ? kTrSlice : 0) + kk * 32),
+                           sm100::desc_kmajor_sw128(tb + 4096u * n + (p == 1 ? kTrSlice : 0) + kk * 32), idesc,
+                           (p | kk) != 0);
+        sm100::mma_commit(n == 0 ? &bars->trDone[P] : &bars->trRest[P]);
+      }
+    }
+    __syncwarp();
+    ok = sm100::mbar_wait(&bars->trDone[P], 0, kWaitLimit) && ok;
+    sm100::tc_fence_after();
+    float v[32];
+    sm100::tmem_ld32(trow, v);
 #pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] = fmaf(xv[i].w, lv[j].w, acc[i][j]);
-#pragma unroll
-    for (int j = 0; j < 4; j++) lv[j] = ln[j];
-#pragma unroll
-    for (int i = 0; i < NI; i++) xv[i] = xn[i];
+    for (int j = 0; j < 8; j++) {
+      const float4 o = *reinterpret_cast<const float4*>(&S[r][32 * (P + 1) + 4 * j]);
+      x[4 * j] = fmaf(-v[4 * j], f, mine ? 0.f : o.x), x[4 * j + 1] = fmaf(-v[4 * j + 1], f, mine ? 0.f : o.y);
+      x[4 * j + 2] = fmaf(-v[4 * j + 2], f, mine ? 0.f : o.z), x[4 * j + 3] = fmaf(-v[4 * j + 3], f, mine ? 0.f : o.w);
+    }
+    sm100::tc_fence_before();
   }
-#pragma unroll
-  for (int i = 0; i < NI; i++) {
-    const int r = rows[i];
+}
+
+// The rank-32 product of panel P: the columns past the next panel, into S (beside chol_inv128).
+__device__ __forceinline__ void chol_help(float (*S)[kLd], PanelBars* bars, uint32_t tmem, int P, int r, int lane,
+                                          bool& ok) {
+  const uint32_t trow = tmem + ((uint32_t)(r & ~31) << 16);
+  ok = sm100::mbar_wait(&bars->step[4 * P + 3], 0, kWaitLimit) && ok;  // (rowf)
+  ok = sm100::mbar_wait(&bars->trRest[P], 0, kWaitLimit) && ok;
+  sm100::tc_fence_after();
+  const float f = bars->rowf[P & 1][r];
+  const bool mine = (r >> 5) == P;
+#pragma unroll 1
+  for (int c = 0; c < 64 - 32 * P; c += 16) {
+    float v[16];
+    sm100::tmem_ld16(trow + 32 + c, v);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      const int c = c0 + g + 8 * j;
-      if (r >= 0 && c < c0 + w && (r >= kT || r >= c)) S[r][c] -= acc[i][j];
+      float4* o = reinterpret_cast<float4*>(&S[r][32 * (P + 2) + c + 4 * j]);
+      const float4 a = mine ? make_float4(0.f, 0.f, 0.f, 0.f) : *o;
+      *o = make_float4(fmaf(-v[4 * j], f, a.x), fmaf(-v[4 * j + 1], f, a.y), fmaf(-v[4 * j + 2], f, a.z),
+                       fmaf(-v[4 * j + 3], f, a.w));
     }
   }
-}
-
-// up to 96 diagonal-block rows + 128 tile rows: at most 7 row groups
-__device__ __forceinline__ void dp_block_update(float (*S)[kLd], int t, int c0, int w, int nd, int nv, int qlo,
-                                                int qhi) {
-  switch ((nv + 31) >> 5) {
-    case 1: dp_block_update_n<1>(S, t, c0, w, nd, nv, qlo, qhi); break;
-    case 2: dp_block_update_n<2>(S, t, c0, w, nd, nv, qlo, qhi); break;
-    case 3: dp_block_update_n<3>(S, t, c0, w, nd, nv, qlo, qhi); break;
-    case 4: dp_block_update_n<4>(S, t, c0, w, nd, nv, qlo, qhi); break;
-    case 5: dp_block_update_n<5>(S, t, c0, w, nd, nv, qlo, qhi); break;
-    case 6: dp_block_update_n<6>(S, t, c0, w, nd, nv, qlo, qhi); break;
-    default: dp_block_update_n<7>(S, t, c0, w, nd, nv, qlo, qhi); break;
-  }
-}
-
-// Forward substitution of one row (32 entries at `row`, 16-byte aligned)
-// against the factored 32 x 32 block, right-looking in registers:
-//   x[c] = (b[c] - sum_{q < c} x[q] L[c][q]) / L[c][c].
-// T is the block transposed, T[c][j] = L[j][c] (row stride kLt), with
-// 1 / L[c][c] on its diagonal, so column c of L is one contiguous row.
-__device__ __forceinline__ void dp_row_solve(float* row, const float* T, float (&x)[32]) {
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const float4 v = reinterpret_cast<const float4*>(row)[k];
-    x[4 * k] = v.x, x[4 * k + 1] = v.y, x[4 * k + 2] = v.z, x[4 * k + 3] = v.w;
-  }
-#pragma unroll
-  for (int c = 0; c < 32; c++) {
-    float t[32];
-#pragma unroll
-    for (int k = c >> 2; k < 8; k++) {
-      const float4 v = reinterpret_cast<const float4*>(T + c * kLt)[k];
-      t[4 * k] = v.x, t[4 * k + 1] = v.y, t[4 * k + 2] = v.z, t[4 * k + 3] = v.w;
-    }
-    x[c] *= t[c];
-#pragma unroll
-    for (int j = c + 1; j < 32; j++) x[j] = fmaf(-x[c], t[j], x[j]);
-  }
-#pragma unroll
-  for (int k = 0; k < 8; k++)
-    reinterpret_cast<float4*>(row)[k] = make_float4(x[4 * k], x[4 * k + 1], x[4 * k + 2], x[4 * k + 3]);
-}
-
-// Cholesky of a 32 x 32 block held by one warp, lane i holding row i (a[j],
-// j <= i), right-looking in registers.  Column c: 1/sqrt of the pivot once
-// (rsqrt), the column scaled, then written as row c of T (T[c][j] = L[j][c],
-// 1 / L[c][c] on the diagonal, zero above), from which every lane reads the
-// column back with 16-byte broadcast loads for its rank-1 update.  The next
-// pivot, A[c+1][c+1] - L[c+1][c]^2, is formed by lane c + 1 from its own
-// entries and shuffled to all lanes at once, so only one shuffle per column
-// is on the pivot chain.  FULL (w == 32) is branch-free; otherwise the rows
-// of T past w are zeroed.  A negative pivot is replaced by its absolute
-// value and flagged in `neg` (func.cpp:827-833).
-template <bool FULL>
-__device__ __forceinline__ void warp_chol32(float (&a)[32], int w, int lane, float* T, int& neg) {
-  float d = __shfl_sync(0xffffffffu, a[0], 0);
-#pragma unroll
-  for (int c = 0; c < 32; c++) {
-    if (!FULL && c >= w) break;
-    const float ad = fabsf(d);
-    const float inv = rsqrtf(ad);
-    if (lane == c) neg |= d < 0.f;
-    a[c] = (lane == c) ? ad * inv : ((lane > c) ? a[c] * inv : a[c]);
-    if (c + 1 < 32) d = __shfl_sync(0xffffffffu, fmaf(-a[c], a[c], a[c + 1]), c + 1);
-    T[c * kLt + lane] = (lane > c) ? a[c] : (lane == c ? inv : 0.f);
-    __syncwarp();
-#pragma unroll
-    for (int k = (c + 1) >> 2; k < 8; k++) {
-      const float4 tv = reinterpret_cast<const float4*>(T + c * kLt)[k];
-      const float t4[4] = {tv.x, tv.y, tv.z, tv.w};
-#pragma unroll
-      for (int e = 0; e < 4; e++)
-        if (4 * k + e > c) a[4 * k + e] = fmaf(-a[c], t4[e], a[4 * k + e]);
-    }
-  }
-  if (!FULL)
-    for (int c = w; c < 32; c++) T[c * kLt + lane] = 0.f;
+  sm100::tc_fence_before();
   __syncwarp();
+  if (lane == 0) sm100::mbar_arrive(&bars->helped[P]);
 }
 
-// Row r of the CTA's rows of L_ik (row rs of the 128-row tile), columns
-// c0 .. c0 + 31 (x[j] = 0 past column w): (L, 0) pairs into A (`g` = A at
-// column c0 of the CTA's first row) for rows inside the matrix, and the
-// 16-byte chunks of the two FP16 slices of scale * x for every row of the tile.
-__device__ __forceinline__ void dp_emit(const float (&x)[32], int r, int rs, int nrows, int c0, int w, float2* g,
-                                        int lda, unsigned char* ps, float scale) {
-  if (r < nrows) {  // read again only by the noise product after the factorisation (BD_DP_EVICT_FIRST)
-    const uint64_t pol = sm100::policy_evict_first();
+// Beside chol_inv128, step by step:
+// L's columns below the 8 x 8 diagonal blocks into A (G = A at the block), as
+// (L, 0) pairs ...
+__device__ __forceinline__ void chain_store_l(const float (*S)[kLd], PanelBars* bars, int lane, int kb, float2* G,
+                                              int lda, bool& ok) {
+#pragma unroll 1
+  for (int q = 0; q < 16; q++) {
+    ok = ok && sm100::mbar_wait(&bars->step[q], 0, kWaitLimit);
+#pragma unroll 1
+    for (int r = ((8 * q + 8) & ~31) + lane; r < kb; r += 32) {
+      if (r < 8 * q + 8) continue;
+      const float4 v0 = *reinterpret_cast<const float4*>(&S[r][8 * q]);
+      const float4 v1 = *reinterpret_cast<const float4*>(&S[r][8 * q + 4]);
+      const float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
 #pragma unroll
-    for (int j = 0; j < 32; j++)
-      if (j < w) {
-        if (BD_DP_EVICT_FIRST) sm100::st_f2_hint(g + (size_t)j * lda + r, make_float2(x[j], 0.f), pol);
-        else g[(size_t)j * lda + r] = make_float2(x[j], 0.f);
-      }
-  }
-#pragma unroll
-  for (int q8 = 0; q8 < 4; q8++) {
-    uint32_t hw[4], lw[4];
-#pragma unroll
-    for (int j2 = 0; j2 < 4; j2++) split_f16x2(x[8 * q8 + 2 * j2] * scale, x[8 * q8 + 2 * j2 + 1] * scale, hw[j2], lw[j2]);
-    const uint32_t off = swz_off(rs, c0 + 8 * q8);
-    *reinterpret_cast<uint4*>(ps + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-    *reinterpret_cast<uint4*>(ps + kSliceBytes + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-  }
-}
-
-// Runs in a CTA of kRestThreads (320) threads: 256 load, update and solve;
-// while warp 0 factors a diagonal block, warps 2..9 update the next block
-// column.  `b` is the CTA's index among the panel CTAs.
-// The previous panel's update of this panel's column, applied in the panel
-// CTA itself (so no separate launch precedes the panel): with panel p's
-// slices PSpre, D0 = L_kp L_kp^T for the diagonal tile and (tile CTAs)
-// D1 = L_ip L_kp^T for the CTA's tile, three FP16 products per K step on
-// tcgen05 into two 128-column TMEM accumulators.  The operands are streamed
-// in two K-halves into the memory the panel later uses for S, so the
-// products are complete before S is loaded; they are subtracted from S
-// after the load.  Every wait is bounded; a timeout records an error code.
-struct PreBars {
-  uint64_t full[2], done;
-  uint32_t slot;
-};
-constexpr int kPreStage = 2 * kTileSlices * kHalfBytes;  // one K-half of the A and B slices (64 KB)
-constexpr int kPreBarOff = 137 * 1024;                   // the barriers lie past the stages and the panel
-static_assert(kPreBarOff >= 2 * kPreStage && kPreBarOff >= (int)kDpSmem, "barriers past both uses of the memory");
-
-__device__ __forceinline__ void dpanel_body(float4* sm4, float2* A, float* Ldg, int lda, int m, int k0, int kb, int tile0,
-                                            int b, unsigned char* PS, int* negpiv, const unsigned char* PSpre,
-                                            int* err, int rpc, float scale, float iscale2) {
-  float (*S)[kLd] = reinterpret_cast<float (*)[kLd]>(sm4);  // rows 0..127 diagonal block, 128..255 tile
-  float* T = reinterpret_cast<float*>(sm4) + 2 * kT * kLd;  // the current 32 x 32 factor, transposed
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool work = tid < kDpThreads;
-  const bool is_diag = b == 0;
-  // tile CTAs take rpc (128 or 64) rows of a tile: b - 1 = (tile - tile0) (128 / rpc) + part
-  const int parts = kT / rpc, part = is_diag ? 0 : (b - 1) % parts;
-  const int tile = tile0 + (is_diag ? 0 : (b - 1) / parts);
-  const int row0 = tile * kT + part * rpc;
-  const int nrows = is_diag ? 0 : max(0, min(rpc, m - row0));
-  DP_MARK(0);
-  unsigned char* smA = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(sm4) + 1023) & ~uintptr_t(1023));
-  PreBars* pbar = reinterpret_cast<PreBars*>(smA + kPreBarOff);
-  uint32_t tmem = 0;
-  bool pre_ok = true;
-  if (PSpre) {
-    if (tid == 0) {
-      sm100::mbar_init(&pbar->full[0], 1);
-      sm100::mbar_init(&pbar->full[1], 1);
-      sm100::mbar_init(&pbar->done, 1);
-      sm100::fence_mbar_init();
+      for (int j = 0; j < 8; j++) G[(size_t)(8 * q + j) * lda + r] = make_float2(v[j], 0.f);
     }
-    if (warp == 1) sm100::tmem_alloc(&pbar->slot, 2 * kT);
-    sm100::tc_fence_before();
-    __syncthreads();
-    sm100::tc_fence_after();
-    tmem = pbar->slot;
-    if (tid == 0) {
-      const unsigned char* gB = PSpre + (size_t)(tile0 - 1) * kTileBytes;  // this panel's tile row
-      const unsigned char* gA = PSpre + (size_t)tile * kTileBytes;
-      for (int h = 0; h < 2; h++) {  // stage h: [A: two 16 KB slice halves][B: two]
-        unsigned char* st = smA + h * kPreStage;
-        sm100::mbar_arrive_expect_tx(&pbar->full[h], (is_diag ? 1 : 2) * kTileSlices * kHalfBytes);
-        for (int s2 = 0; s2 < kTileSlices; s2++)
-          sm100::bulk_g2s(st + kTileSlices * kHalfBytes + s2 * kHalfBytes, gB + s2 * kSliceBytes + h * kHalfBytes,
-                          kHalfBytes, &pbar->full[h]);
-        if (!is_diag)
-          for (int s2 = 0; s2 < kTileSlices; s2++)
-            sm100::bulk_g2s(st + s2 * kHalfBytes, gA + s2 * kSliceBytes + h * kHalfBytes, kHalfBytes, &pbar->full[h]);
+  }
+}
+// ... and rows 8 q .. 8 q + 7 of W = L^-1 (W[l][j] = X[j][l]) as slices in Wo
+// and on to Wn, every row scaled by a power of two that puts its largest entry
+// into [2^13, 2^14); wscn[l] undoes that scale and the tile's, cs.  The copies
+// are in the lanes' bulk groups.
+__device__ __forceinline__ void chain_store_w(const float (*S)[kLd], PanelBars* bars, int lane, int q, float cs,
+                                              unsigned char* Wo, unsigned char* Wn, float* wscn, bool& ok) {
+  ok = sm100::mbar_wait(&bars->step[q], 0, kWaitLimit) && ok;
+  // lane (i, jc): row 8 q + i, columns 8 (jc + 4 t) .. + 7 for t = 0 .. 3
+  const int i = lane & 7, jc = lane >> 3, row = 8 * q + i;
+  float x[4][8];
+  float m = 0.f;
+#pragma unroll
+  for (int t = 0; t < 4; t++) {
+    const int j0 = 8 * (jc + 4 * t);
+    const bool in = jc + 4 * t <= q;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      x[t][j] = in ? S[j0 + j][row] : 0.f;
+      m = fmaxf(m, fabsf(x[t][j]));
+    }
+  }
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+  int e = 13 + 127 - (int)(__float_as_uint(m) >> 23);
+  if (!(m > 0.f) || isinf(m) || e > 100 || e < -100) e = 0;
+  const float sc = __uint_as_float((uint32_t)(127 + e) << 23);
+  if (jc == 0) wscn[row] = 1.f / (cs * sc);
+#pragma unroll
+  for (int t = 0; t < 4; t++) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) x[t][j] *= sc;
+    put_slices8(Wo, row, 8 * (jc + 4 * t), x[t]);
+  }
+  sm100::fence_proxy_async();
+  __syncwarp();
+  if (lane < 2 * kTileSlices) {  // the rows' 1 KB in each half of a slice
+    const int off = lane * kHalfBytes + q * 1024;
+    sm100::bulk_s2g(Wn + off, Wo + off, 1024);
+  }
+}
+
+// What a panel CTA works on.  tile < 0: no tile (the first launch, which only
+// factors diagonal block 0).  PSpre: panel k - 1's slices, or null (k = 0).
+struct PanelArgs {
+  float2* A;
+  int lda, m, k, tile;            // panel k, tile row
+  unsigned char* PSp;             // panel k's slices
+  const unsigned char* PSpre;
+  const unsigned char* Wk;        // W_k's slices
+  const float* wsc;               // [128] X = D * wsc, by column
+  unsigned char* Wn;              // W_k+1's slices and factors (chain)
+  float* wscn;
+  int* negpiv;
+  int* err;
+  float scale, iscale2;
+};
+
+// Shared memory: R0 L_i,k-1 then L_ik's slices; R1 L_k,k-1 then the tile's
+// slices (the diagonal block from kChainS on reuses R1 and the start of R2);
+// R2 W_k.  Tensor memory: P at column 0, X at 128; chain: the updates of the
+// diagonal block by panel k at 256 and by panel k - 1 at 384 (apart: the tensor
+// core truncates its sums, so their error grows with the length).
+// Warp 0 copies, warp 1 issues the products, warps 2 .. 9 hold the tile: a
+// thread one row (TMEM lane) and 64 columns.
+template <bool CHAIN>
+__device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs& p) {
+  unsigned char* sm = align1024(smraw);
+  unsigned char *R0 = sm, *R1 = sm + kTileBytes, *R2 = sm + 2 * kTileBytes;
+  PanelBars* bars = reinterpret_cast<PanelBars*>(sm + kPanelMisc);
+  float (*S)[kLd] = reinterpret_cast<float (*)[kLd]>(sm + kChainS);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool has_tile = p.tile >= 0, pre = has_tile && p.PSpre != nullptr;
+  constexpr uint32_t kCols = CHAIN ? 512 : 256;
+  if (tid == 0) {
+    sm100::mbar_init(&bars->fullPre, 1);
+    sm100::mbar_init(&bars->fullW, 2);
+    sm100::mbar_init(&bars->preDone, 1);
+    sm100::mbar_init(&bars->sReady, 8);
+    sm100::mbar_init(&bars->xDone, 1);
+    sm100::mbar_init(&bars->lReady, 8);
+    sm100::mbar_init(&bars->qDone, 1);
+    if (CHAIN) {
+      sm100::mbar_init(&bars->r0Free, 1);
+      for (int q = 0; q < 3; q++) sm100::mbar_init(&bars->trDone[q], 1);
+      for (int q = 0; q < 2; q++) {
+        sm100::mbar_init(&bars->trRest[q], 1);
+        sm100::mbar_init(&bars->helped[q], 4);
       }
-      const uint32_t idesc = sm100::idesc_f16_f32(128, 128);
-      const int pa[3] = {1, 0, 0};  // (A slice, B slice) products, smallest first
-      const int pb[3] = {0, 1, 0};
-      bool ok = true;
-      for (int h = 0; h < 2 && ok; h++) {
-        ok = sm100::mbar_wait(&pbar->full[h], 0, kWaitLimit);
-        if (!ok) break;
+      for (int q = 0; q < 16; q++) sm100::mbar_init(&bars->step[q], 1);
+    }
+    sm100::fence_mbar_init();
+  }
+  if (warp == 1) sm100::tmem_alloc(&bars->slot, kCols);
+  sm100::tc_fence_before();
+  __syncthreads();
+  sm100::tc_fence_after();
+  const uint32_t tmem = bars->slot;
+  bool ok = true;
+
+  if (warp == 0) {
+    if (lane == 0 && has_tile) {
+      if (pre) {
+        sm100::mbar_arrive_expect_tx(&bars->fullPre, 2 * kTileBytes);
+        sm100::bulk_g2s(R0, p.PSpre + (size_t)p.tile * kTileBytes, kTileBytes, &bars->fullPre);
+        sm100::bulk_g2s(R1, p.PSpre + (size_t)p.k * kTileBytes, kTileBytes, &bars->fullPre);
+      }
+      sm100::mbar_arrive_expect_tx(&bars->fullW, kTileBytes);
+      sm100::bulk_g2s(R2, p.Wk, kTileBytes, &bars->fullW);
+    }
+    if (has_tile) {
+      *reinterpret_cast<float4*>(&bars->xsc[4 * lane]) = reinterpret_cast<const float4*>(p.wsc)[lane];
+      __syncwarp();
+      if (lane == 0) {
+        sm100::mbar_arrive(&bars->fullW);
+        ok = sm100::mbar_wait(&bars->lReady, 0, kWaitLimit);
+        if (ok) {
+          sm100::bulk_s2g(p.PSp + (size_t)p.tile * kTileBytes, R0, kTileBytes);
+          sm100::bulk_store_wait();
+        } else {  // copies in flight land before the CTA exits
+          if (pre) (void)sm100::mbar_wait(&bars->fullPre, 0, kWaitLimit);
+          (void)sm100::mbar_wait(&bars->fullW, 0, kWaitLimit);
+        }
+      }
+      __syncwarp();
+    }
+    if (CHAIN) {
+      const int nd = p.k + 1;
+      if (lane == 0) sm100::mbar_arrive(&bars->r0Free);
+      chain_store_l(S, bars, lane, min(kT, p.m - nd * kT), p.A + (size_t)(nd * kT) * p.lda + nd * kT, p.lda, ok);
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && has_tile) {
+      if (pre) {
+        ok = sm100::mbar_wait(&bars->fullPre, 0, kWaitLimit);
         sm100::tc_fence_after();
-        const unsigned char* sa = smA + h * kPreStage;
-        const unsigned char* sb = sa + kTileSlices * kHalfBytes;
+        if (ok) mma_tile(tmem, R0, R1, false);
+        sm100::mma_commit(&bars->preDone);
+        if (CHAIN && ok) mma_tile(tmem + 384, R0, R0, false);
+      }
+      ok = ok && sm100::mbar_wait(&bars->fullW, 0, kWaitLimit);
+      ok = ok && sm100::mbar_wait(&bars->sReady, 0, kWaitLimit);
+      sm100::tc_fence_after();
+      if (ok) mma_tile(tmem + 128, R1, R2, false);
+      sm100::mma_commit(&bars->xDone);
+      if (CHAIN) {
+        ok = ok && sm100::mbar_wait(&bars->lReady, 0, kWaitLimit);
+        sm100::tc_fence_after();
+        if (ok) mma_tile(tmem + 256, R0, R0, false);
+        sm100::mma_commit(&bars->qDone);
+      }
+      if (!ok) (void)sm100::mbar_wait(&bars->xDone, 0, kWaitLimit);
+    }
+  } else {
+    const int q = warp & 3, ch = (warp - 2) >> 2, r = 32 * q + lane;
+    const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(64 * ch);
+    const uint64_t pol = sm100::policy_evict_first();  // the tile's columns are read again only by the noise product
+    const int nd = p.k + 1;  // the diagonal block of the chain CTA (tile row of its tile too)
+    // 64 columns of the thread's row of L_ik, from tensor memory into A
+    auto store_l = [&](int half) {
+      const int gi = p.tile * kT + r;
+      float2* colp = p.A + (size_t)(p.k * kT + 64 * half) * p.lda + gi;
+#pragma unroll 1
+      for (int c = 0; c < 4; c++) {
+        float v[16];
+        sm100::tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + 128 + 64 * half + 16 * c, v);  // (the whole warp)
+        if (gi < p.m) {
 #pragma unroll
-        for (int p = 0; p < 3; p++) {
-          const uint32_t b0 = sm100::smem_u32(sb + pa[p] * kHalfBytes), b1 = sm100::smem_u32(sb + pb[p] * kHalfBytes);
-          const uint32_t a0 = sm100::smem_u32(sa + pa[p] * kHalfBytes);
+          for (int j4 = 0; j4 < 4; j4++) {
+            const float4 f = *reinterpret_cast<const float4*>(&bars->xsc[64 * half + 16 * c + 4 * j4]);
+            const float fs[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
-          for (int kk = 0; kk < 4; kk++) {
-            const uint32_t acc = (h | p | kk) != 0;
-            sm100::mma_f16(tmem, sm100::desc_kmajor_sw128(b0 + kk * 32), sm100::desc_kmajor_sw128(b1 + kk * 32), idesc,
-                            acc);
-            if (!is_diag)
-              sm100::mma_f16(tmem + kT, sm100::desc_kmajor_sw128(a0 + kk * 32), sm100::desc_kmajor_sw128(b1 + kk * 32),
-                              idesc, acc);
+            for (int j = 0; j < 4; j++)
+              sm100::st_f2_hint(colp + (size_t)(16 * c + 4 * j4 + j) * p.lda, make_float2(v[4 * j4 + j] * fs[j], 0.f), pol);
           }
         }
+        __syncwarp();
       }
-      sm100::mma_commit(&pbar->done);
-      if (!ok) {
-        atomicExch(err, 6);
-        // copies still in flight land before their memory is reused
-        (void)sm100::mbar_wait(&pbar->full[0], 0, kWaitLimit);
-        (void)sm100::mbar_wait(&pbar->full[1], 0, kWaitLimit);
-      }
-    }
-    // the products read the stage memory: complete before S overwrites it
-    pre_ok = sm100::mbar_wait(&pbar->done, 0, kWaitLimit);
-    sm100::tc_fence_after();
-    pre_ok = __syncthreads_and(pre_ok);  // one decision for the whole CTA (it gates a named barrier below)
-    if (!pre_ok && tid == 0) atomicExch(err, 7);
-  }
-  // Rows [0, nr) of a 128-row part of the panel (columns k0 .. k0 + kb) into
-  // S[roff ..], FP32 (the nearest of each stored double-float; entries past
-  // the part are zero), by 8 warps (w8 = 0 .. 7).  Two rows per 16-byte
-  // load; lane l takes rows 2 (l & 3) + {0, 1} of an 8-row block and column
-  // l >> 2 of an 8-column block, so a warp reads 64-byte runs of 8 columns
-  // and its shared stores hit 32 distinct banks.  Row pairs start even and
-  // lda is a multiple of 32: every load is aligned and stays inside its
-  // column.  16 loads per thread in flight.
-  const size_t ld4 = (size_t)lda / 2;
-  const uint64_t pol = sm100::policy_evict_first();  // read once (BD_DP_EVICT_FIRST)
-  auto load_part = [&](const float2* gbase, int roff, int nr, bool lower, int w8) {
-    const int rr = 2 * (lane & 3), cc = lane >> 2;
-    const float4* g4 = reinterpret_cast<const float4*>(gbase);
-#pragma unroll 1
-    for (int cb = w8; cb < kT / 8; cb += 8) {
-      const int c = 8 * cb + cc;
-      float4 v[16];
+    };
+    float2 old[64];
+    if (has_tile) {
+      const int gi = p.tile * kT + r;
+      float2* colp = p.A + (size_t)(p.k * kT + 64 * ch) * p.lda + gi;
+      const bool in = gi < p.m;
 #pragma unroll
-      for (int i = 0; i < 16; i++) {
-        const int r = 8 * i + rr;
-        const bool in = (!lower || r + 1 >= c) && r < nr && c < kb;
-        v[i] = in ? (BD_DP_EVICT_FIRST ? sm100::ld_f4_hint(g4 + c * ld4 + r / 2, pol) : g4[c * ld4 + r / 2])
-                  : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int i = 0; i < 16; i++) {
-        const int r = 8 * i + rr;
-        S[roff + r][c] = (r < nr && c < kb) ? v[i].x + v[i].y : 0.f;
-        S[roff + r + 1][c] = (r + 1 < nr && c < kb) ? v[i].z + v[i].w : 0.f;
-      }
-    }
-  };
-  // the CTA's D accumulator rows into S: warp w reads TMEM lanes 32 (w % 4) ..
-  auto subtract = [&](bool tile_part) {
-    const int q = warp & 3, r = 32 * q + lane;
-    const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + (tile_part ? (uint32_t)kT : 0u);
-    float* row = tile_part ? S[kT + r - part * rpc] : S[r];
-#pragma unroll 1
-    for (int cc = 0; cc < kT; cc += 32) {
-      float v[32];
-      sm100::tmem_ld32(ta + cc, v);
-#pragma unroll
-      for (int k4 = 0; k4 < 8; k4++) {
-        float4* p4 = reinterpret_cast<float4*>(row + cc + 4 * k4);
-        float4 x = *p4;
-        x.x -= v[4 * k4] * iscale2, x.y -= v[4 * k4 + 1] * iscale2;
-        x.z -= v[4 * k4 + 2] * iscale2, x.w -= v[4 * k4 + 3] * iscale2;
-        *p4 = x;
-      }
-    }
-  };
-  // the diagonal block first (and D0 off it); the tile rows load while the
-  // first 32 x 32 block is factored (below)
-  if (work) load_part(A + (size_t)k0 * lda + k0, 0, kb, true, warp);
-  __syncthreads();
-  if (PSpre && pre_ok && warp < 4) subtract(false);
-  if (PSpre) sm100::tc_fence_before();
-  __syncthreads();
-  DP_MARK(1);
-  const int nb = (kb + 31) >> 5;
-  const int nrt = is_diag ? 0 : rpc;  // tile rows solved (rows past the matrix are zero and stay zero)
-  for (int jb = 0; jb < nb; jb++) {
-    const int c0 = 32 * jb, w = min(32, kb - c0);
-    const int c1 = c0 + 32, w1 = kb - c1;  // the next block column (w1 <= 0: none)
-    const int nd = max(0, w1);             // diagonal-block rows below this block
-    // A: warp 0 factors the 32 x 32 diagonal block; warps 2..9 meanwhile
-    // apply the finished block columns (q < c0) to the next block column
-    if (warp == 0) {
-      float a[32];
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const float4 v = lane < w ? reinterpret_cast<const float4*>(&S[c0 + lane][c0])[k] : make_float4(0.f, 0.f, 0.f, 0.f);
-        a[4 * k] = v.x, a[4 * k + 1] = v.y, a[4 * k + 2] = v.z, a[4 * k + 3] = v.w;
-      }
-#pragma unroll
-      for (int j = 0; j < 32; j++)
-        if (j > lane) a[j] = 0.f;  // upper part: not referenced
-      int neg = 0;
-      if (w == 32) warp_chol32<true>(a, 32, lane, T, neg);
-      else warp_chol32<false>(a, w, lane, T, neg);
-      if (is_diag) {  // L_kk is kept by CTA 0 only; the others need T alone
-        if (neg) atomicAdd(negpiv, 1);
-#pragma unroll
-        for (int j = 0; j < 32; j++)
-          if (lane < w && j <= lane) S[c0 + lane][c0 + j] = a[j];
-      }
-    } else if (warp >= 2 && jb == 0) {
-      // the tile rows (and the previous panel's update of them)
-      if (!is_diag) {
+      for (int j = 0; j < 64; j++) old[j] = sm100::ld_f2_hint_if(colp + (size_t)j * p.lda, pol, in);
+      if (pre) {
+        ok = sm100::mbar_wait(&bars->preDone, 0, kWaitLimit);
         sm100::tc_fence_after();
-        load_part(A + (size_t)k0 * lda + row0, kT, nrows, false, warp - 2);
-        if (PSpre && pre_ok) {
-          asm volatile("bar.sync 1, 256;" ::: "memory");  // warps 2..9: the tile rows loaded
-          if (warp >= 4 && warp < 8 && (32 * (warp & 3)) / rpc == part) subtract(true);
+      }
+      // the tile less panel k - 1's update, as slices of scale^2 / 16 times
+      // it (|A_ij| <= max D_ii: at most 2^14)
+      const float cs = p.scale * p.scale * 0.0625f;
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        float v[16];
+        if (pre) sm100::tmem_ld16(trow + 16 * c, v);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          float x[8];
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            const float2 o = old[16 * c + 8 * h + j];
+            x[j] = (pre ? fmaf(-v[8 * h + j], p.iscale2, o.x) + o.y : o.x + o.y) * cs;
+          }
+          put_slices8(R1, r, 64 * ch + 16 * c + 8 * h, x);
         }
       }
-    } else if (warp >= 2 && w1 > 0 && c0 > 0) {
-      dp_block_update(S, tid - 64, c1, min(32, w1), nd, nd + nrows, 0, c0);
+      sm100::fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) sm100::mbar_arrive(&bars->sReady);
     }
-    if (jb == 0 && PSpre) sm100::tc_fence_before();
-    __syncthreads();
-    if (jb == 0 && PSpre && warp == 1) sm100::tmem_dealloc(tmem, 2 * kT);
-    DP_MARK(2 + 3 * jb);
-    // B: the rows below the block, the rest of the diagonal block, then the
-    // 128 tile rows; a tile row's 32 new entries of L_ik go out at once:
-    // back into A as (L, 0) pairs and as two FP16 slices, pre-swizzled
-    // (consecutive lanes take consecutive rows, so the pair stores are
-    // coalesced)
-    if (tid < nd + nrt) {
+    const int kb = min(kT, p.m - nd * kT);
+    if (CHAIN) {  // the diagonal block's row, under the product
+      const float2* colp = p.A + (size_t)(nd * kT + 64 * ch) * p.lda + nd * kT + r;
+#pragma unroll
+      for (int j = 0; j < 64; j++)
+        old[j] = sm100::ld_f2_hint_if(colp + (size_t)j * p.lda, pol, 64 * ch + j <= r && r < kb);
+    }
+    if (has_tile) {
+      ok = sm100::mbar_wait(&bars->fullW, 0, kWaitLimit) && ok;  // (xsc)
+      ok = sm100::mbar_wait(&bars->xDone, 0, kWaitLimit) && ok;
+      sm100::tc_fence_after();
+#pragma unroll 1
+      for (int c = 0; c < 4; c++) {
+        float v[16], x[16];
+        sm100::tmem_ld16(trow + 128 + 16 * c, v);
+#pragma unroll
+        for (int j4 = 0; j4 < 4; j4++) {
+          const float4 f = *reinterpret_cast<const float4*>(&bars->xsc[64 * ch + 16 * c + 4 * j4]);
+          const float fs[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+          for (int j = 0; j < 4; j++) x[4 * j4 + j] = v[4 * j4 + j] * (fs[j] * p.scale);
+        }
+#pragma unroll
+        for (int j8 = 0; j8 < 2; j8++) {
+          float y[8];
+#pragma unroll
+          for (int j = 0; j < 8; j++) y[j] = x[8 * j8 + j];
+          put_slices8(R0, r, 64 * ch + 16 * c + 8 * j8, y);
+        }
+      }
+      sm100::fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) sm100::mbar_arrive(&bars->lReady);
+      if (!CHAIN) store_l(ch);
+    }
+    if (CHAIN) {
+      if (has_tile) {
+        ok = sm100::mbar_wait(&bars->qDone, 0, kWaitLimit) && ok;
+        sm100::tc_fence_after();
+      }
+      // the diagonal block less its two updates (the part above the diagonal
+      // is never used); rows past the matrix: the unit block
       float x[32];
-      dp_row_solve(&S[tid < nd ? c1 + tid : kT + tid - nd][c0], T, x);
-      if (tid >= nd) dp_emit(x, tid - nd, part * rpc + tid - nd, nrows, c0, w, A + (size_t)(k0 + c0) * lda + row0, lda,
-                             PS + (size_t)tile * kTileBytes, scale);
+#pragma unroll
+      for (int c = 0; c < 8; c++) {
+        float y[8], v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) y[j] = old[8 * c + j].x;
+        if (has_tile) {
+          sm100::tmem_ld8(trow + 256 + 8 * c, v);
+#pragma unroll
+          for (int j = 0; j < 8; j++) y[j] = fmaf(-v[j], p.iscale2, y[j]);
+        }
+        if (pre) {
+          sm100::tmem_ld8(trow + 384 + 8 * c, v);
+#pragma unroll
+          for (int j = 0; j < 8; j++) y[j] = fmaf(-v[j], p.iscale2, y[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          y[j] += old[8 * c + j].y;
+          if (r >= kb) y[j] = 64 * ch + 8 * c + j == r ? 1.f : 0.f;
+        }
+        if (c < 4) {
+#pragma unroll
+          for (int j = 0; j < 8; j++) x[8 * c + j] = y[j];
+        }
+        if (c >= 4 || ch == 1) {  // (the first panel stays in registers)
+          *reinterpret_cast<float4*>(&S[r][64 * ch + 8 * c]) = make_float4(y[0], y[1], y[2], y[3]);
+          *reinterpret_cast<float4*>(&S[r][64 * ch + 8 * c + 4]) = make_float4(y[4], y[5], y[6], y[7]);
+        }
+      }
+      if (ch == 0) {
+        int neg = 0;
+        chol_inv128(S, bars, R0, tmem, x, r, lane, p.scale, neg, ok);
+        if (neg && lane == 0 && q == 0) atomicAdd(p.negpiv, neg);
+      } else {
+        if (has_tile) {
+          store_l(0);
+          store_l(1);
+        }
+#pragma unroll 1
+        for (int P = 0; P < 4; P++) {
+          if (P < 2) chol_help(S, bars, tmem, P, r, lane, ok);
+          chain_store_w(S, bars, lane, 4 * P + (warp - 6), p.scale * p.scale * 0.0625f, sm + kChainW, p.Wn, p.wscn, ok);
+        }
+        if (lane < 2 * kTileSlices) sm100::bulk_store_wait();
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      // L's 8 x 8 diagonal blocks (only this CTA reads or writes the diagonal block in this launch)
+      if (ch == 0 && r < kb) {
+        float2* row = p.A + (size_t)(nd * kT + (r & ~7)) * p.lda + nd * kT + r;
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+          if (j <= (r & 7)) row[(size_t)j * p.lda] = make_float2(bars->dg[r >> 3][r & 7][j], 0.f);
+      }
     }
-    __syncthreads();
-    DP_MARK(3 + 3 * jb);
-    // C: this block column's contribution to the next one
-    if (w1 > 0) {
-      if (work) dp_block_update(S, tid, c1, min(32, w1), nd, nd + nrows, c0, c1);
-      __syncthreads();
-    }
-    DP_MARK(4 + 3 * jb);
   }
-  if (is_diag && work) {
-    // L_kk goes to a side buffer, not into A: panel CTAs of this launch that
-    // start after this one has finished (more CTAs than SMs) still read A_kk
-    for (int e = tid; e < kT * kT; e += kDpThreads) {
-      const int c = e >> 7, r = e & (kT - 1);
-      Ldg[e] = (r >= c && r < kb && c < kb) ? S[r][c] : 0.f;  // column-major
-    }
-  }
-  DP_MARK(15);
+  if (!ok) atomicExch(p.err, 6);
+  sm100::tc_fence_before();
+  __syncthreads();
+  if (warp == 1) sm100::tmem_dealloc(tmem, kCols);
 }
 
 // ------------------------------------------------------------ tensor-core trailing update
@@ -577,7 +756,7 @@ __device__ __forceinline__ void dpanel_body(float4* sm4, float2* A, float* Ldg, 
 #endif
 constexpr int kRestThreads = 320;
 constexpr int kStageBytes = kTileSlices * kHalfBytes;  // one K-half of the two B slices
-constexpr size_t kRestSmem = kPreBarOff + 2 * 1024;
+constexpr size_t kRestSmem = kPanelSmem;
 static_assert(kRestSmem >= (size_t)kTileBytes + 2 * kStageBytes + 1024 + 256, "the update CTAs' operands");
 constexpr int kAccCols = 128;
 
@@ -612,6 +791,9 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
                                           int tlo, int thi, int group, int cta, const unsigned char* __restrict__ PS,
                                           const unsigned char* __restrict__ PS2, const unsigned char* __restrict__ PS3,
                                           int* err, float iscale2) {
+  // (rounded as an integer, not by align1024: with the pointer known to be
+  // shared the compiler places the epilogue's loads worse, 211 against 161 ms
+  // for the factorisation at 3N = 46,200)
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smraw) + 1023) & ~uintptr_t(1023));
   unsigned char* sA = sm;                 // 2 slices x 32 KB
   unsigned char* sB = sm + kTileBytes;    // 2 stages x (2 slices x 16 KB)
@@ -942,41 +1124,38 @@ struct UpdJob {
   int jlo, mode, tlo, thi, group, nctas;
 };
 struct StepArgs {
-  float2* A;
-  float* Ldg;           // this panel's diagonal factor
-  unsigned char* PSp;   // this panel's slice buffer
-  const unsigned char* PSpre;  // the previous panel's slices: its update of this panel's column, or null
-  int* negpiv;
-  int* err;
-  int lda, m, ndp, pk0, pkb;
-  float scale, iscale2;  // the slices hold scale * L; iscale2 = scale^-2 (powers of two)
-  int prows;  // tile rows per panel CTA (128, or 64 when the panel is split over twice the CTAs)
+  PanelArgs pan;  // panel k and the chain's tile
+  int ntile;      // tile CTAs: tile rows k + 2 .. k + 1 + ntile
   UpdJob job[2];
 };
 
-// One launch per step: CTAs [0, ndp) factor panel pk (diagonal block and the
-// tiles below it, writing its slices to PSp); then the CTAs of update job 0,
-// then those of job 1.  The parts of one launch touch disjoint tiles and
-// slice buffers.
+// One launch per step.  CTA 0 is the chain CTA, CTAs 1 .. ntile solve the
+// other tiles of panel k; then the CTAs of update job 0, then those of job 1.
+// The parts of one launch touch disjoint tiles and slice buffers.
 __device__ __forceinline__ void chol_step_body(const StepArgs& a, int b, float4* smem4) {
-  if (b < a.ndp) {
-    dpanel_body(smem4, a.A, a.Ldg, a.lda, a.m, a.pk0, a.pkb, a.pk0 / kT + 1, b, a.PSp, a.negpiv, a.PSpre, a.err,
-                a.prows, a.scale, a.iscale2);
+  unsigned char* sm = reinterpret_cast<unsigned char*>(smem4);
+  if (b == 0) {
+    panel_body<true>(sm, a.pan);
     return;
   }
-  b -= a.ndp;
+  b -= 1;
+  if (b < a.ntile) {
+    PanelArgs p = a.pan;
+    p.tile = a.pan.k + 2 + b;
+    panel_body<false>(sm, p);
+    return;
+  }
+  b -= a.ntile;
   const int jn = b < a.job[0].nctas ? 0 : 1;
   if (jn) b -= a.job[0].nctas;
   const UpdJob& j = a.job[jn];
+  const PanelArgs& p = a.pan;
   if (j.ps3)
-    rest_body<3>(reinterpret_cast<unsigned char*>(smem4), a.A, a.lda, a.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b,
-                 j.ps, j.ps2, j.ps3, a.err, a.iscale2);
+    rest_body<3>(sm, p.A, p.lda, p.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b, j.ps, j.ps2, j.ps3, p.err, p.iscale2);
   else if (j.ps2)
-    rest_body<2>(reinterpret_cast<unsigned char*>(smem4), a.A, a.lda, a.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b,
-                 j.ps, j.ps2, nullptr, a.err, a.iscale2);
+    rest_body<2>(sm, p.A, p.lda, p.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b, j.ps, j.ps2, nullptr, p.err, p.iscale2);
   else
-    rest_body<1>(reinterpret_cast<unsigned char*>(smem4), a.A, a.lda, a.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b,
-                 j.ps, nullptr, nullptr, a.err, a.iscale2);
+    rest_body<1>(sm, p.A, p.lda, p.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b, j.ps, nullptr, nullptr, p.err, p.iscale2);
 }
 
 __global__ void __launch_bounds__(kRestThreads, 1) k_chol_step(const __grid_constant__ StepArgs a) {
@@ -985,44 +1164,25 @@ __global__ void __launch_bounds__(kRestThreads, 1) k_chol_step(const __grid_cons
 }
 
 // The same step for many independent factorisations in one launch (replicas
-// of a batch): factorisation r owns CTAs [off[r], off[r + 1]) and runs its own
-// schedule's step with args[r]; the factorisations share no memory.
+// of a batch): each runs its own schedule's step with args[r].  The nrep
+// chain CTAs come first (they take longest), then factorisation r owns CTAs
+// nrep + [off[r], off[r + 1]); the factorisations share no memory.
 __global__ void __launch_bounds__(kRestThreads, 1) k_chol_step_multi(const StepArgs* __restrict__ args,
                                                                       const int* __restrict__ off, int nrep) {
   extern __shared__ float4 smem4[];
-  const int bid = (int)blockIdx.x;
+  int bid = (int)blockIdx.x;
+  if (bid < nrep) {
+    chol_step_body(args[bid], 0, smem4);
+    return;
+  }
+  bid -= nrep;
   int lo = 0, hi = nrep;  // off[lo] <= bid < off[lo + 1]
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
     if (off[mid] <= bid) lo = mid;
     else hi = mid;
   }
-  chol_step_body(args[lo], bid - off[lo], smem4);
-}
-
-// After the last panel: the diagonal factors L_kk from the side buffer into
-// the lower triangles of A's diagonal blocks, as (L, 0) pairs.
-__device__ __forceinline__ void diag_scatter_body(float2* A, int lda, int m, const float* __restrict__ Ld, int k) {
-  const int k0 = k * kT, kb = min(kT, m - k0);
-  const float* src = Ld + (size_t)k * kT * kT;
-  for (int e = threadIdx.x; e < kT * kT; e += blockDim.x) {
-    const int c = e >> 7, r = e & (kT - 1);
-    if (r >= c && r < kb && c < kb) A[(size_t)(k0 + c) * lda + k0 + r] = make_float2(src[e], 0.f);
-  }
-}
-__global__ void __launch_bounds__(256) k_diag_scatter(float2* A, int lda, int m, const float* __restrict__ Ld) {
-  diag_scatter_body(A, lda, m, Ld, blockIdx.x);
-}
-struct ScatterArgs {
-  float2* A;
-  int lda, m;
-  const float* Ld;
-};
-// every factorisation of a batch (blockIdx.y), diagonal block blockIdx.x
-__global__ void __launch_bounds__(256) k_diag_scatter_multi(const ScatterArgs* __restrict__ sc) {
-  const ScatterArgs a = sc[blockIdx.y];
-  if ((int)blockIdx.x * kT >= a.m) return;
-  diag_scatter_body(a.A, a.lda, a.m, a.Ld, blockIdx.x);
+  chol_step_body(args[lo], bid - off[lo] + 1, smem4);
 }
 
 }  // namespace
@@ -1032,9 +1192,9 @@ namespace bdk {
 // kBufs panel-slice buffers, panel p in buffer p % kBufs: a triple's bulk
 // update reads panels k .. k + 2 while panel k + 3 is written
 constexpr int kBufs = 4;
-size_t mixed_panel_bytes(int m) {  // the slice buffers, then the diagonal factors
-  return kBufs * (size_t)cdiv(m, kT) * kTileBytes + (size_t)cdiv(m, kT) * kT * kT * sizeof(float);
-}
+// the slice buffers, then two buffers for the inverse of a diagonal factor
+// (W_k in buffer k & 1: read by the launch that writes W_k+1), then its factors
+size_t mixed_panel_bytes(int m) { return kBufs * (size_t)cdiv(m, kT) * kTileBytes + 2 * (size_t)kTileBytes + 2 * kT * sizeof(float); }
 int mixed_max_launches(int m) { return 2 * cdiv(m, kT) + 2; }
 int mixed_tiles(int m) { return cdiv(m, kT); }
 
@@ -1056,7 +1216,6 @@ static bool g_attr_done = false;
 
 int set_mixed_attributes() {
   if (g_attr_done) return 0;
-  static_assert(kDpSmem <= kRestSmem, "panel CTAs run inside the update kernel's shared memory");
   cudaError_t e = cudaFuncSetAttribute(k_chol_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRestSmem);
   if (e != cudaSuccess) return 1;
   e = cudaFuncSetAttribute(k_chol_step_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRestSmem);
@@ -1081,30 +1240,26 @@ static int rest_group(int tiles) {
 }
 
 // Right-looking with a lookahead of one panel, on one stream, no two kernels
-// at a time; every launch is one k_chol_step: panel pn in its own CTAs (which
-// first apply panel pn-1's update to column pn themselves) beside up to two
-// update jobs.  Panel p's slices live in buffer p % kBufs, L_kk in a side
-// buffer.  Invariant before the launch of panel k+1: panels <= k are
-// factored and column k+1 holds the updates of panels < k.
-// Single step: panel k+1 beside panel k's update of the tiles right of
-// column k+1 (K = 128).
+// at a time; every launch is one k_chol_step: panel k's tiles solved and
+// diagonal block k + 1 factored (the chain and tile CTAs, which apply panel
+// k - 1's update to column k themselves) beside up to two update jobs.  Panel
+// p's slices live in buffer p % kBufs, W_p in buffer p & 1.  Invariant before
+// the launch of panel k + 1: panels <= k are solved, column k + 1 and diagonal
+// block k + 2 hold the updates of panels < k, and the launch leaves diagonal
+// block k + 2 to its chain CTA (which applies panels k and k + 1).
+// Single step: panel k + 1 beside panel k's update of the tiles right of
+// column k + 1 (K = 128).
 // Pair (k+1, k+2), while the trailing matrix is large: the bulk tiles get
 // both panels in one read-modify-write (K = 256), half the HBM traffic:
-//   1: panel k+1 beside panel k's update of column k+2;
+//   1: panel k+1 beside panel k's update of column k+2 and of diagonal block k+3;
 //   2: panel k+2 beside panels k and k+1 on the tiles right of column k+2.
 // Triple (k+1 .. k+3), while it is larger still (K = 384):
-//   1: panel k+1 beside panel k's update of column k+2;
-//   2: panel k+2 beside panels k and k+1 on column k+3 (K = 256);
+//   1: panel k+1 beside panel k's update of column k+2 and of diagonal block k+3;
+//   2: panel k+2 beside panels k and k+1 on column k+3 (K = 256) and on diagonal block k+4;
 //   3: panel k+3 beside panels k .. k+2 on the tiles right of column k+3.
 // Returns the number of kernel launches.
 #ifndef BD_PAIR_MIN
 #define BD_PAIR_MIN 24  // pair while at least this many tile rows remain right of column k+2 (k: last factored)
-#endif
-#ifndef BD_SPLIT_CTAS
-#define BD_SPLIT_CTAS 151  // panel CTAs allowed when the panel is split in 64-row parts
-#endif
-#ifndef BD_SPLIT_JOB_TILES
-#define BD_SPLIT_JOB_TILES 400  // ... and at most this many update tiles in the launch
 #endif
 #ifndef BD_TRIPLE_MIN
 #define BD_TRIPLE_MIN 40  // three panels per bulk pass while this many tile rows remain right of column k+3
@@ -1114,12 +1269,12 @@ struct Job {
   const unsigned char* ps = nullptr;
   const unsigned char* ps2 = nullptr;
   const unsigned char* ps3 = nullptr;
-  int jlo = 0, mode = kCol, tiles = 0, group = 1;
+  int jlo = 0, mode = kCol, tlo = 0, tiles = 0, group = 1;
 };
 }  // namespace
 
 // The launches of one factorisation: issued on st, or (plan != nullptr)
-// only recorded with their grid sizes, without the final diagonal scatter.
+// only recorded with their grid sizes.
 // max_pass (1..3): most panels one bulk pass carries (K = 128 max_pass).
 // Fewer panels per pass mean fewer FP32 tensor-memory accumulation steps per
 // stored update and more read-modify-write passes: 3 is the fastest, 1 the
@@ -1133,7 +1288,8 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
   int L = 0, timed = 0;
   auto kb_of = [&](int k) { return (m - k * kT < kT) ? m - k * kT : kT; };
   auto psb = [&](int k) { return PS + (size_t)(k % kBufs) * buf; };
-  float* Ld = reinterpret_cast<float*>(PS + kBufs * buf);  // [nt][128 x 128] diagonal factors
+  unsigned char* Wb = PS + kBufs * buf;  // the inverses' slices
+  float* wsc = reinterpret_cast<float*>(Wb + 2 * (size_t)kTileBytes);
   // elements of the lower triangle in tile columns [j0, j1)
   auto elems = [&](int j0, int j1) {
     double e = 0.0;
@@ -1143,48 +1299,46 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
     }
     return e;
   };
-  auto col_job = [&](int p, int J, int npan = 1) {  // panels p .. p + npan - 1 on column J
+  // panels p .. p + npan - 1 on column J below its diagonal block (the chain CTA's)
+  auto col_job = [&](int p, int J, int npan = 1) {
     Job j;
-    j.ps = psb(p), j.ps2 = npan > 1 ? psb(p + 1) : nullptr, j.jlo = J, j.mode = kCol, j.tiles = nt - J, j.group = 1;
+    j.ps = psb(p), j.ps2 = npan > 1 ? psb(p + 1) : nullptr, j.jlo = J, j.mode = kCol, j.tlo = 1, j.tiles = nt - J;
     return j;
   };
-  auto tri_job = [&](int p, int npan, int jlo) {  // panels p .. p + npan - 1 on the triangle from column jlo
+  auto diag_job = [&](int p, int J, int npan = 1) {  // ... on diagonal block J alone
+    Job j;
+    j.ps = psb(p), j.ps2 = npan > 1 ? psb(p + 1) : nullptr, j.jlo = J, j.mode = kCol, j.tiles = 1;
+    return j;
+  };
+  auto tri_job = [&](int p, int npan, int jlo) {  // ... on the triangle from column jlo but its first diagonal block
     Job j;
     const int n = nt - jlo;
     j.ps = psb(p), j.ps2 = npan > 1 ? psb(p + 1) : nullptr, j.ps3 = npan > 2 ? psb(p + 2) : nullptr;
-    j.jlo = jlo, j.mode = kRowTri;
+    j.jlo = jlo, j.mode = kRowTri, j.tlo = 1;
     j.tiles = n > 0 ? n * (n + 1) / 2 : 0;
     j.group = rest_group(j.tiles);
     return j;
   };
-  // pn: the panel factored by this launch (-1: none); pre: panel pn - 1's
-  // update of column pn is applied by the panel CTAs themselves
-  auto launch = [&](int pn, const Job& j0, const Job& j1, bool pre) {
+  // panel k's tiles (k < 0: none) and diagonal block k + 1
+  auto launch = [&](int k, const Job& j0, const Job& j1) {
     StepArgs a{};
-    a.A = A, a.negpiv = negpiv, a.err = err, a.lda = lda, a.m = m;
-    a.scale = scale, a.iscale2 = 1.f / (scale * scale);
-    a.Ldg = Ld, a.PSp = PS, a.PSpre = nullptr, a.prows = kT;
-    if (pn >= 0) {
-      // the panel over twice the CTAs (64 tile rows each) when they fit on
-      // the GPU beside small update jobs: the diagonal work is repeated,
-      // the tile work halved
-      const int jt = (j0.tiles > 0 ? j0.tiles : 0) + (j1.tiles > 0 ? j1.tiles : 0);
-      if (2 * (nt - pn - 1) + 1 <= BD_SPLIT_CTAS && jt <= BD_SPLIT_JOB_TILES) a.prows = kT / 2;
-      a.ndp = 1 + (nt - pn - 1) * (kT / a.prows), a.pk0 = pn * kT, a.pkb = kb_of(pn);
-      a.Ldg = Ld + (size_t)pn * kT * kT, a.PSp = psb(pn);
-      if (pre && pn > 0) a.PSpre = psb(pn - 1);
-    }
+    PanelArgs& p = a.pan;
+    p.A = A, p.lda = lda, p.m = m, p.k = k, p.tile = k < 0 ? -1 : k + 1;
+    p.PSp = psb(k < 0 ? 0 : k), p.PSpre = k > 0 ? psb(k - 1) : nullptr;
+    p.Wk = Wb + (size_t)(k & 1) * kTileBytes, p.wsc = wsc + kT * (k & 1);
+    p.Wn = Wb + (size_t)((k + 1) & 1) * kTileBytes, p.wscn = wsc + kT * ((k + 1) & 1);
+    p.negpiv = negpiv, p.err = err, p.scale = scale, p.iscale2 = 1.f / (scale * scale);
+    a.ntile = k < 0 ? 0 : nt - k - 2;
     const Job* js[2] = {&j0, &j1};
-    int grid = a.ndp;
+    int grid = 1 + a.ntile;
     for (int q = 0; q < 2; q++) {
       const Job& j = *js[q];
       UpdJob& u = a.job[q];
-      u.ps = j.ps, u.ps2 = j.ps2, u.ps3 = j.ps3, u.jlo = j.jlo, u.mode = j.mode, u.tlo = 0, u.thi = j.tiles,
+      u.ps = j.ps, u.ps2 = j.ps2, u.ps3 = j.ps3, u.jlo = j.jlo, u.mode = j.mode, u.tlo = j.tlo, u.thi = j.tiles,
       u.group = j.group;
-      u.nctas = j.tiles > 0 ? cdiv(j.tiles, j.group) : 0;
+      u.nctas = j.tiles > j.tlo ? cdiv(j.tiles - j.tlo, j.group) : 0;
       grid += u.nctas;
     }
-    if (grid == 0) return;
     if (plan) {
       plan->emplace_back(a, grid);
       return;
@@ -1197,39 +1351,39 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
     }
     L++;
     if (kbytes || kflop) {
-      double by = pn >= 0 ? 16.0 * (double)(m - pn * kT) * kb_of(pn) : 0.0;  // panel read and written back
-      double fl = a.PSpre ? 3.0 * 2.0 * kT * kT * kT * (2 * a.ndp - 1) : 0.0;  // the panel CTAs' own products
+      const double tile_fl = 3.0 * 2.0 * kT * kT * kT;
+      double by = 16.0 * (double)(m - (k + 1) * kT) * (k < 0 ? kb_of(0) : kT);  // panel read and written back
+      double fl = k < 0 ? 0.0 : tile_fl * (2.0 * (1 + a.ntile) + 2.0);        // the panel CTAs' own products
       for (int q = 0; q < 2; q++) {
         const Job& j = *js[q];
-        if (j.tiles <= 0) continue;
-        by += 16.0 * elems(j.jlo, j.mode == kCol ? j.jlo + 1 : nt);  // double-float tile read + write
-        fl += 3.0 * 2.0 * kT * kT * kT * j.tiles * (j.ps3 ? 3 : (j.ps2 ? 2 : 1));  // FP16 tensor work issued
+        if (j.tiles <= j.tlo) continue;
+        by += 16.0 * (j.tiles == 1 ? 0.5 * kT * kb_of(j.jlo) : elems(j.jlo, j.mode == kCol ? j.jlo + 1 : nt));
+        fl += tile_fl * (j.tiles - j.tlo) * (j.ps3 ? 3 : (j.ps2 ? 2 : 1));  // FP16 tensor work issued
       }
       if (kbytes) *kbytes += by;
       if (kflop) *kflop += fl;
     }
   };
   const Job none;
-  launch(0, none, none, false);  // panel 0 alone
+  launch(-1, none, none);             // diagonal block 0
+  if (nt > 1) launch(0, none, none);  // panel 0
   int k = 0;
-  while (k + 1 < nt) {
+  while (k + 2 < nt) {
     if (max_pass >= 3 && nt - (k + 4) >= BD_TRIPLE_MIN) {
-      launch(k + 1, col_job(k, k + 2), none, true);
-      launch(k + 2, col_job(k, k + 3, 2), none, true);
-      launch(k + 3, tri_job(k, 3, k + 4), none, true);
+      launch(k + 1, col_job(k, k + 2), diag_job(k, k + 3));
+      launch(k + 2, col_job(k, k + 3, 2), diag_job(k, k + 4, 2));
+      launch(k + 3, tri_job(k, 3, k + 4), none);
       k += 3;
     } else if (max_pass >= 2 && nt - (k + 3) >= BD_PAIR_MIN) {
-      launch(k + 1, col_job(k, k + 2), none, true);
-      launch(k + 2, tri_job(k, 2, k + 3), none, true);
+      launch(k + 1, col_job(k, k + 2), diag_job(k, k + 3));
+      launch(k + 2, tri_job(k, 2, k + 3), none);
       k += 2;
     } else {
-      launch(k + 1, tri_job(k, 1, k + 2), none, true);
+      launch(k + 1, tri_job(k, 1, k + 2), none);
       k += 1;
     }
   }
   if (plan) return L;
-  k_diag_scatter<<<nt, 256, 0, st>>>(A, lda, m, Ld);
-  L++;
   if (kev_pairs) *kev_pairs = timed;
   return L;
 }
@@ -1251,8 +1405,7 @@ struct MixedBatch {
   std::vector<size_t> args_at, off_at;
   StepArgs* d_args = nullptr;
   int* d_off = nullptr;
-  ScatterArgs* d_sc = nullptr;
-  int nrep = 0, max_nt = 0;
+  int nrep = 0;
 };
 
 MixedBatch* mixed_batch_create(int nrep, const int* m, double* const* A, const int* lda, unsigned char* const* PS,
@@ -1261,17 +1414,10 @@ MixedBatch* mixed_batch_create(int nrep, const int* m, double* const* A, const i
   size_t steps = 0;
   MixedBatch* b = new MixedBatch();
   b->nrep = nrep;
-  std::vector<ScatterArgs> sc(nrep);
   for (int r = 0; r < nrep; r++) {
     potrf_mixed_impl(m[r], A[r], lda[r], PS[r], negpiv[r], err[r], nullptr, nullptr, nullptr, nullptr, nullptr,
                      &plans[r], max_pass, scale[r]);
     steps = std::max(steps, plans[r].size());
-    const int nt = cdiv(m[r], kT);
-    b->max_nt = std::max(b->max_nt, nt);
-    sc[r].A = reinterpret_cast<float2*>(A[r]);
-    sc[r].lda = lda[r];
-    sc[r].m = m[r];
-    sc[r].Ld = reinterpret_cast<const float*>(PS[r] + kBufs * (size_t)nt * kTileBytes);
   }
   std::vector<StepArgs> args;
   std::vector<int> off;
@@ -1286,19 +1432,17 @@ MixedBatch* mixed_batch_create(int nrep, const int* m, double* const* A, const i
       if (i < shift || i - shift >= plans[r].size()) continue;
       args.push_back(plans[r][i - shift].first);
       off.push_back(total);
-      total += plans[r][i - shift].second;
+      total += plans[r][i - shift].second - 1;  // its chain CTA is counted apart
       n++;
     }
     off.push_back(total);
     b->nrep_at.push_back(n);
-    b->grid_at.push_back(total);
+    b->grid_at.push_back(n + total);
   }
   bool ok = cudaMalloc(&b->d_args, std::max<size_t>(1, args.size()) * sizeof(StepArgs)) == cudaSuccess &&
             cudaMalloc(&b->d_off, std::max<size_t>(1, off.size()) * sizeof(int)) == cudaSuccess &&
-            cudaMalloc(&b->d_sc, nrep * sizeof(ScatterArgs)) == cudaSuccess &&
             cudaMemcpy(b->d_args, args.data(), args.size() * sizeof(StepArgs), cudaMemcpyHostToDevice) == cudaSuccess &&
-            cudaMemcpy(b->d_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
-            cudaMemcpy(b->d_sc, sc.data(), nrep * sizeof(ScatterArgs), cudaMemcpyHostToDevice) == cudaSuccess;
+            cudaMemcpy(b->d_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess;
   if (!ok) {
     mixed_batch_free(b);
     return nullptr;
@@ -1313,15 +1457,13 @@ int mixed_batch_run(const MixedBatch* b, cudaStream_t st) {
                                                                          b->d_off + b->off_at[i], b->nrep_at[i]);
     L++;
   }
-  k_diag_scatter_multi<<<dim3(b->max_nt, b->nrep), 256, 0, st>>>(b->d_sc);
-  return L + 1;
+  return L;
 }
 
 void mixed_batch_free(MixedBatch* b) {
   if (!b) return;
   if (b->d_args) cudaFree(b->d_args);
   if (b->d_off) cudaFree(b->d_off);
-  if (b->d_sc) cudaFree(b->d_sc);
   delete b;
 }
 

@@ -57,6 +57,20 @@ __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, u
       : "memory");
 }
 
+// 1-D bulk-async copy shared -> global (16-byte aligned, size % 16 == 0), in
+// the thread's bulk group; the generic-proxy writes of the source must be
+// fenced (fence_proxy_async) before.  bulk_store_wait: every copy committed
+// by this thread has been written.
+__device__ __forceinline__ void bulk_s2g(void* gmem_dst, const void* smem_src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gmem_dst), "r"(smem_u32(smem_src)),
+               "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_store_wait() {
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
 // Hint: bring `bytes` (multiple of 16, 16-byte aligned) of global memory into L2.
 __device__ __forceinline__ void prefetch_l2(const void* gmem, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gmem), "r"(bytes) : "memory");
@@ -119,6 +133,17 @@ __device__ __forceinline__ float4 ld_f4_hint(const float4* a, uint64_t pol) {
 __device__ __forceinline__ float2 ld_f2_hint(const float2* a, uint64_t pol) {
   float2 v;
   asm volatile("ld.global.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(a), "l"(pol));
+  return v;
+}
+// The same where `in` holds, else (0, 0); no branch around the load.
+__device__ __forceinline__ float2 ld_f2_hint_if(const float2* a, uint64_t pol, bool in) {
+  float2 v = make_float2(0.f, 0.f);
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.u32 p, %4, 0;\n\t"
+      "@p ld.global.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;\n\t}"
+      : "+f"(v.x), "+f"(v.y)
+      : "l"(a), "l"(pol), "r"((uint32_t)in));
   return v;
 }
 __device__ __forceinline__ void st_f2_hint(float2* a, float2 v, uint64_t pol) {
