@@ -324,18 +324,42 @@ __global__ void k_chain_bonded(DevModel M, DevState X, const double* __restrict_
   Ech[j] = has_hi ? hi[36] : 0.0;
 }
 
-// ------------------------------------------------------------ charge sets
-// Core/core (func.cpp:1489-1566), FP64 path: kCCSplit CTAs per core pair
-// I < J (mixed contexts: k_core_core_mx below, split the same way).
-constexpr int kCCThreads = 256;
+// Past pair_f1's longest cut-off (7 nm) by more than FP32's error, from the
+// double-float mirror: no force, no energy.  Most pairs of the FP64 gathers end
+// here without FP64 arithmetic, whose pipe bounds them (a pair's distance alone
+// is six operations at 16 cycles a warp and SM).  50 nucleosomes with linker
+// histones, chain + tails + LH: 2,042 us with the distance in FP64 and a torque
+// for each pair, 470 now.
+__device__ __forceinline__ bool far(const DevScratch& S, int a, int b) {
+  const float3 z = sepf(ldpf(S, a), ldpf(S, b));
+  const float d2 = fmaf(z.x, z.x, fmaf(z.y, z.y, z.z * z.z));
+  return d2 > 50.f && d2 < 1e30f;
+}
 
-__global__ void __launch_bounds__(kCCThreads) k_core_core(DevModel M, DevState X, double* slots) {
+// ------------------------------------------------------------ charge sets
+// core pair I < J of index t
+__device__ __forceinline__ void core_pair(int t, int& I, int& J) {
+  J = (int)((1.0f + sqrtf(8.f * (float)t + 1.f)) * 0.5f);
+  while (J * (J + 1) / 2 <= t) J++;
+  while (J * (J - 1) / 2 > t) J--;
+  I = t - J * (J - 1) / 2;
+}
+
+// Core/core (func.cpp:1489-1566), FP64 path: kCC64Split CTAs per core pair
+// I < J, each an interleaved share of the charge pairs and its own slot (summed
+// by k_cc_sum).  Bound by the FP64 pipe: 50 operations a charge pair, a warp's
+// each 64 cycles.  Small CTAs, no CTA for pairs I >= J: with 4 of 256 threads
+// in a grid of all I, J the SMs' shares of 66 pairs were uneven.  12
+// nucleosomes: 1,700 us with pow and both torques per charge pair, 858 without,
+// 475 in this split.
+constexpr int kCC64Threads = 128;
+
+__global__ void __launch_bounds__(kCC64Threads) k_core_core(DevModel M, DevState X, double* slots) {
   extern __shared__ double sm[];
-  int I = blockIdx.x, J = blockIdx.y;
-  // gridDim.z CTAs share the pair, each its own interleaved share of the
-  // charge pairs and its own slot (summed by k_cc_sum)
-  double* out = slots + (((size_t)blockIdx.z * M.n_c + I) * M.n_c + J) * 10;
-  if (I >= J) return;
+  int I, J;
+  core_pair(blockIdx.x / kCC64Split, I, J);
+  const int part = blockIdx.x % kCC64Split;
+  double* out = slots + (((size_t)part * M.n_c + I) * M.n_c + J) * 10;
   int i = M.core_bead[I], j = M.core_bead[J];
   V3 ri = ld3(X.r + 3 * i), rj = ld3(X.r + 3 * j);
   double d0 = sqrt((rj.x - ri.x) * (rj.x - ri.x) + (rj.y - ri.y) * (rj.y - ri.y) + (rj.z - ri.z) * (rj.z - ri.z));
@@ -358,56 +382,59 @@ __global__ void __launch_bounds__(kCCThreads) k_core_core(DevModel M, DevState X
   const double* cp = M.core_pos;
   const double* cq = M.core_q;
   const double ke = M.k_e, kap = M.debye, kex = M.k_ex, sg = M.sCC;
-  double v[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-  {
-  for (int p = blockIdx.z * blockDim.x + threadIdx.x; p < Nq * Nq; p += blockDim.x * gridDim.z) {
-      int k = p / Nq, l = p - k * Nq;
-      V3 pk = ld3(si_ + 3 * k), pl = ld3(sj_ + 3 * l);
-      V3 z{pk.x - pl.x, pk.y - pl.y, pk.z - pl.z};
-      double dd = sqrt(z.x * z.x + z.y * z.y + z.z * z.z);
-      double mi = 1.0 / dd;
-      z = V3{mi * z.x, mi * z.y, mi * z.z};
-      double ex = exp(-kap * dd);
-      double g1 = ke * cq[k] * cq[l] * ex * (kap * dd + 1.0) / (dd * dd);
-      v[9] = v[9] + (ke * cq[l] * cq[k] / dd) * ex;
-      double gsum[2] = {g1, 0.0};
-      int ng = 1;
+  // Warp w takes sites k = w, w + nw, ... of core I against all sites of core
+  // J (lanes).  The force on site k is summed over the lane's sites first and
+  // its torque formed once per k; the torque on J is linear in sum f (x) cp_l
+  // (nine sums), turned into J's frame at the end: the reference's
+  // cp x (R^T f), which forms both torques for every charge pair.
+  double F[3] = {0, 0, 0}, TI[3] = {0, 0, 0}, MJ[3][3] = {{0}}, E = 0.0;
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int k = (threadIdx.x >> 5) + nw * part; k < Nq; k += nw * kCC64Split) {
+    const V3 pk = ld3(si_ + 3 * k);
+    const double qk = ke * cq[k];
+    double fk[3] = {0, 0, 0};
+    for (int l = lane; l < Nq; l += 32) {
+      const V3 pl = ld3(sj_ + 3 * l);
+      const double zx = pk.x - pl.x, zy = pk.y - pl.y, zz = pk.z - pl.z;
+      const double dd = sqrt(fma(zx, zx, fma(zy, zy, zz * zz))), mi = 1.0 / dd;
+      double e = qk * cq[l] * mi * exp(-kap * dd);       // k_e q_k q_l e^{-kappa d} / d
+      double g = e * fma(kap, dd, 1.0) * mi;             // ... (kappa d + 1) / d^2
       if (dd <= 8.0) {
-        gsum[1] = kex * ((12.0 / sg) * pow((sg / dd), 13) - (6.0 / sg) * pow((sg / dd), 7));
-        v[9] = v[9] + kex * (pow(sg / dd, 12) - pow(sg / dd, 6));
-        ng = 2;
+        double s6, s12;
+        lj_powers(sg, mi, s6, s12);
+        g = fma(kex * mi, fma(12.0, s12, -6.0 * s6), g);
+        e = fma(kex, s12 - s6, e);
       }
-      for (int q = 0; q < ng; q++) {
-        double gg = gsum[q];
-        v[0] = v[0] + gg * z.x; v[1] = v[1] + gg * z.y; v[2] = v[2] + gg * z.z;
-        double fa = gg * (ai.x * z.x + ai.y * z.y + ai.z * z.z);
-        double fb = gg * (bi.x * z.x + bi.y * z.y + bi.z * z.z);
-        double fc = gg * (ci.x * z.x + ci.y * z.y + ci.z * z.z);
-        v[3] = v[3] + (fc * cp[3 * k + 1] - fb * cp[3 * k + 2]);
-        v[4] = v[4] + (fa * cp[3 * k + 2] - fc * cp[3 * k]);
-        v[5] = v[5] + (fb * cp[3 * k] - fa * cp[3 * k + 1]);
-        fa = -gg * (aj.x * z.x + aj.y * z.y + aj.z * z.z);
-        fb = -gg * (bj.x * z.x + bj.y * z.y + bj.z * z.z);
-        fc = -gg * (cj.x * z.x + cj.y * z.y + cj.z * z.z);
-        v[6] = v[6] + (fc * cp[3 * l + 1] - fb * cp[3 * l + 2]);
-        v[7] = v[7] + (fa * cp[3 * l + 2] - fc * cp[3 * l]);
-        v[8] = v[8] + (fb * cp[3 * l] - fa * cp[3 * l + 1]);
+      E = E + e;
+      const double gz = g * mi, fx = gz * zx, fy = gz * zy, fz = gz * zz;
+      fk[0] = fk[0] + fx, fk[1] = fk[1] + fy, fk[2] = fk[2] + fz;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double p = cp[3 * l + c];
+        MJ[0][c] = fma(fx, p, MJ[0][c]), MJ[1][c] = fma(fy, p, MJ[1][c]), MJ[2][c] = fma(fz, p, MJ[2][c]);
       }
     }
+    F[0] = F[0] + fk[0], F[1] = F[1] + fk[1], F[2] = F[2] + fk[2];
+    const V3 t = torque_rel(V3{fk[0], fk[1], fk[2]}, cp + 3 * k, ai, bi, ci);
+    TI[0] = TI[0] + t.x, TI[1] = TI[1] + t.y, TI[2] = TI[2] + t.z;
   }
+  // f on J is -f: T_J = (R^T (-f)) x ..., component by component of the sums
+  auto dotm = [&](const V3& u, int c) { return u.x * MJ[0][c] + u.y * MJ[1][c] + u.z * MJ[2][c]; };
+  double v[10] = {F[0], F[1], F[2], TI[0], TI[1], TI[2], dotm(bj, 2) - dotm(cj, 1), dotm(cj, 0) - dotm(aj, 2),
+                  dotm(aj, 1) - dotm(bj, 0), E};
   bsum<10>(v, red);
   if (threadIdx.x == 0)
     for (int q = 0; q < 10; q++) out[q] = v[q];
 }
 
-// the FP64 core/core slots: the kCCSplit partials of each pair I < J, summed in order
-__global__ void k_cc_sum(int nc, const double* __restrict__ part, double* __restrict__ slots) {
+// the core/core slots: the nsplit partials of each pair I < J, summed in order
+__global__ void k_cc_sum(int nc, int nsplit, const double* __restrict__ part, double* __restrict__ slots) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nc * nc * 10) return;
   const int pr = e / 10, I = pr / nc, J = pr - I * nc;
   if (I >= J) return;
   double s = 0.0;
-  for (int z = 0; z < kCCSplit; z++) s += part[(size_t)z * nc * nc * 10 + e];
+  for (int z = 0; z < nsplit; z++) s += part[(size_t)z * nc * nc * 10 + e];
   slots[e] = s;
 }
 
@@ -419,15 +446,16 @@ __global__ void k_cc_sum(int nc, const double* __restrict__ part, double* __rest
 // lever x f (lever = R cp) and turned into the body frame once at the end
 // (R^T (lever x f) = cp x (R^T f), the reference's form); sums are FP32 over
 // 32 pairs, then FP64.
+constexpr int kCCThreads = 256;
 constexpr int kCCFlush = 32;
 
 __global__ void __launch_bounds__(kCCThreads) k_core_core_mx(DevModel M, DevState X, DevScratch S, double* slots) {
   extern __shared__ double sm[];
-  const int I = blockIdx.x, J = blockIdx.y;
-  // gridDim.z CTAs share the pair (interleaved sites k of core I), each
+  int I, J;
+  core_pair(blockIdx.x, I, J);
+  // gridDim.y CTAs share the pair (interleaved sites k of core I), each
   // with its own slot, summed in order by k_cc_sum
-  double* out = slots + (((size_t)blockIdx.z * M.n_c + I) * M.n_c + J) * 10;
-  if (I >= J) return;
+  double* out = slots + (((size_t)blockIdx.y * M.n_c + I) * M.n_c + J) * 10;
   const int i = M.core_bead[I], j = M.core_bead[J];
   // far-pair test and the centre offset in FP32, from the double-float mirror
   const float3 oij = sepf(ldpf(S, i), ldpf(S, j));  // r_i - r_j
@@ -477,7 +505,7 @@ __global__ void __launch_bounds__(kCCThreads) k_core_core_mx(DevModel M, DevStat
   // warp w takes sites k = w, w + nw, ... of core I against all sites l of
   // core J (lanes); the force and torque on I are summed per k first
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int k = (threadIdx.x >> 5) + nw * blockIdx.z; k < Nq; k += nw * gridDim.z) {
+  for (int k = (threadIdx.x >> 5) + nw * blockIdx.y; k < Nq; k += nw * gridDim.y) {
     const float sx = sIx[k], sy = sIy[k], sz = sIz[k], qk = qI[k];
     float fkx = 0.f, fky = 0.f, fkz = 0.f;
     for (int l = lane; l < Nq; l += 32) {
@@ -605,35 +633,34 @@ __global__ void k_dna_core(DevModel M, DevState X, DevScratch S, double* slots) 
     }
     for (int q = 0; q < 7; q++) v[q] = (double)a[q];
   } else {
-  for (int k = lane; k < M.Nq; k += 32) {
-      V3 s = body(rc, ac, bc, cc, cp + 3 * k);
-      V3 z{rd_.x - s.x, rd_.y - s.y, rd_.z - s.z};
-      double dd = sqrt(z.x * z.x + z.y * z.y + z.z * z.z);
-      double mi = 1.0 / dd;
-      z = V3{mi * z.x, mi * z.y, mi * z.z};
-      double q = M.core_q[k];
-      double gs[2];
-      int ng = 0;
+    double MC[3][3] = {{0}};  // sum f (x) cp: the torque on the core is linear in it (k_core_core)
+    for (int k = lane; k < M.Nq; k += 32) {
+      const V3 s = body(rc, ac, bc, cc, cp + 3 * k);
+      const double zx = rd_.x - s.x, zy = rd_.y - s.y, zz = rd_.z - s.z;
+      const double dd = sqrt(fma(zx, zx, fma(zy, zy, zz * zz))), mi = 1.0 / dd;
+      const double q = M.core_q[k];
+      double g = 0.0;
       if (adj) {
-        double ex = exp(-kap * dd);
-        gs[ng++] = ke * ql * q * ex * (kap * dd + 1.0) / (dd * dd);
-        v[6] = v[6] + (ke * ql * q / dd) * ex;
+        const double e = ke * ql * q * mi * exp(-kap * dd);
+        g = e * fma(kap, dd, 1.0) * mi;
+        v[6] = v[6] + e;
       }
       if (dd <= 8.0 && q > 0) {
-        gs[ng++] = kex * ((12.0 / sg) * pow((sg / dd), 13) - (6.0 / sg) * pow((sg / dd), 7));
-        v[6] = v[6] + kex * (pow(sg / dd, 12) - pow(sg / dd, 6));
+        double s6, s12;
+        lj_powers(sg, mi, s6, s12);
+        g = fma(kex * mi, fma(12.0, s12, -6.0 * s6), g);
+        v[6] = fma(kex, s12 - s6, v[6]);
       }
-      for (int t = 0; t < ng; t++) {
-        double g1 = gs[t];
-        v[0] = v[0] + g1 * z.x; v[1] = v[1] + g1 * z.y; v[2] = v[2] + g1 * z.z;
-        double fa = -g1 * (ac.x * z.x + ac.y * z.y + ac.z * z.z);
-        double fb = -g1 * (bc.x * z.x + bc.y * z.y + bc.z * z.z);
-        double fc = -g1 * (cc.x * z.x + cc.y * z.y + cc.z * z.z);
-        v[3] = v[3] + (fc * cp[3 * k + 1] - fb * cp[3 * k + 2]);
-        v[4] = v[4] + (fa * cp[3 * k + 2] - fc * cp[3 * k]);
-        v[5] = v[5] + (fb * cp[3 * k] - fa * cp[3 * k + 1]);
+      const double gz = g * mi, fx = gz * zx, fy = gz * zy, fz = gz * zz;
+      v[0] = v[0] + fx, v[1] = v[1] + fy, v[2] = v[2] + fz;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double p = cp[3 * k + c];
+        MC[0][c] = fma(fx, p, MC[0][c]), MC[1][c] = fma(fy, p, MC[1][c]), MC[2][c] = fma(fz, p, MC[2][c]);
       }
     }
+    auto dotm = [&](const V3& u, int c) { return u.x * MC[0][c] + u.y * MC[1][c] + u.z * MC[2][c]; };
+    v[3] = dotm(bc, 2) - dotm(cc, 1), v[4] = dotm(cc, 0) - dotm(ac, 2), v[5] = dotm(ac, 1) - dotm(bc, 0);
   }
   for (int q = 0; q < 7; q++) v[q] = wsum(v[q]);
   if (lane == 0)
@@ -663,18 +690,36 @@ __global__ void k_ghead_core(DevModel M, DevState X, double* slots) {
   const double eps = eps_of(M);
   double v[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   const int ng = M.n_lh_g, Nq = M.Nq;
-  for (int p = lane; p < ng * Nq; p += 32) {
-    int jm = p / Nq, m = p - jm * Nq;
-    V3 g = ld3(X.gpos + 3 * (I * ng + jm));
-    V3 z = body(rl, al, bl, cl, M.core_pos + 3 * m);
-    V3 f1 = pairF<true, true, MX>(M.LH_q[jm], M.core_q[m], eps, M.debye, M.k_ex, M.LH_vdw_hc[jm], g, z, &v[9]);
-    V3 f2{-f1.x, -f1.y, -f1.z};
-    v[0] = v[0] + f1.x; v[1] = v[1] + f1.y; v[2] = v[2] + f1.z;
-    V3 t1 = torque_rel(f1, M.LH_g_pos + 3 * jm, ai, bi, ci);
-    V3 t2 = torque_rel(f2, M.core_pos + 3 * m, al, bl, cl);
-    v[3] = v[3] + t1.x; v[4] = v[4] + t1.y; v[5] = v[5] + t1.z;
-    v[6] = v[6] + t2.x; v[7] = v[7] + t2.y; v[8] = v[8] + t2.z;
+  // lane: charges m of core L, each against every site jm of the head.  The
+  // torques are linear in sum f (x) gp_jm and in sum f (x) cp_m (as in
+  // k_core_core), so no pair forms one in FP64; with two torques and the
+  // charge's position a pair it was 183 us for four cores, now 108.
+  double MI[3][3] = {{0}}, ML[3][3] = {{0}};
+  for (int m = lane; m < Nq; m += 32) {
+    const V3 z = body(rl, al, bl, cl, M.core_pos + 3 * m);
+    double fm[3] = {0, 0, 0};
+    for (int jm = 0; jm < ng; jm++) {
+      const V3 g = ld3(X.gpos + 3 * (I * ng + jm));
+      const V3 f1 = pairF<true, true, MX>(M.LH_q[jm], M.core_q[m], eps, M.debye, M.k_ex, M.LH_vdw_hc[jm], g, z, &v[9]);
+      fm[0] = fm[0] + f1.x, fm[1] = fm[1] + f1.y, fm[2] = fm[2] + f1.z;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double p = M.LH_g_pos[3 * jm + c];
+        MI[0][c] = fma(f1.x, p, MI[0][c]), MI[1][c] = fma(f1.y, p, MI[1][c]), MI[2][c] = fma(f1.z, p, MI[2][c]);
+      }
+    }
+    v[0] = v[0] + fm[0], v[1] = v[1] + fm[1], v[2] = v[2] + fm[2];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const double p = M.core_pos[3 * m + c];
+      ML[0][c] = fma(fm[0], p, ML[0][c]), ML[1][c] = fma(fm[1], p, ML[1][c]), ML[2][c] = fma(fm[2], p, ML[2][c]);
+    }
   }
+  auto dotm = [](const V3& u, const double (&m)[3][3], int c) { return u.x * m[0][c] + u.y * m[1][c] + u.z * m[2][c]; };
+  v[3] = dotm(ci, MI, 1) - dotm(bi, MI, 2), v[4] = dotm(ai, MI, 2) - dotm(ci, MI, 0),
+  v[5] = dotm(bi, MI, 0) - dotm(ai, MI, 1);
+  v[6] = dotm(bl, ML, 2) - dotm(cl, ML, 1), v[7] = dotm(cl, ML, 0) - dotm(al, ML, 2),
+  v[8] = dotm(al, ML, 1) - dotm(bl, ML, 0);  // (the force on L is -f)
   for (int q = 0; q < 10; q++) v[q] = wsum(v[q]);
   if (lane == 0)
     for (int q = 0; q < 10; q++) out[q] = v[q];
@@ -684,70 +729,11 @@ __global__ void k_ghead_core(DevModel M, DevState X, double* slots) {
 // One CTA per chain bead: every remaining contribution to its force and
 // torque, plus the slot reductions; writes the bead's final F, T and its
 // energy share.
-// Block sum of a chain bead's pair terms, then the slot reductions in a
-// fixed order and the bonded terms; thread 0 stores.
+// A chain bead's slot sums, spread over the CTA's threads (FP64, many lanes per
+// instruction: a thread walking the 350 slots of a 50-nucleosome fibre alone
+// held its CTA for 70 us), the block sum of its pair terms and the bonded terms;
+// thread 0 stores.
 __device__ void chain_finish(const DevModel& M, const DevScratch& S, const double* Fm, const double* Tm,
-                             const double* Ech, DevForces& out, double* Eout, int j, V3 F, V3 T, double E,
-                             double* red) {
-  const bool dna = M.type[j] == 0;
-  double v[7] = {F.x, F.y, F.z, T.x, T.y, T.z, E};
-  bsum<7>(v, red);
-  if (threadIdx.x != 0) return;
-  F = V3{v[0], v[1], v[2]};
-  T = V3{v[3], v[4], v[5]};
-  E = v[6];
-  // slot reductions, fixed order
-  if (dna) {
-    const int D = j - M.core_rank[j] - 1;  // linker beads before j
-    for (int J = 0; J < M.n_c; J++) {
-      const double* s = S.dc + ((size_t)D * M.n_c + J) * 7;
-      F.x = F.x + s[0]; F.y = F.y + s[1]; F.z = F.z + s[2];
-    }
-  } else {
-    const int J = M.core_rank[j];
-    for (int K = 0; K < M.n_c; K++) {
-      if (K < J) {
-        const double* s = S.cc + ((size_t)K * M.n_c + J) * 10;
-        F.x = F.x - s[0]; F.y = F.y - s[1]; F.z = F.z - s[2];
-        T.x = T.x + s[6]; T.y = T.y + s[7]; T.z = T.z + s[8];
-      } else if (K > J) {
-        const double* s = S.cc + ((size_t)J * M.n_c + K) * 10;
-        F.x = F.x + s[0]; F.y = F.y + s[1]; F.z = F.z + s[2];
-        T.x = T.x + s[3]; T.y = T.y + s[4]; T.z = T.z + s[5];
-        E = E + s[9];
-      }
-    }
-    for (int D = 0; D < M.n_dna; D++) {
-      const double* s = S.dc + ((size_t)D * M.n_c + J) * 7;
-      F.x = F.x - s[0]; F.y = F.y - s[1]; F.z = F.z - s[2];
-      T.x = T.x + s[3]; T.y = T.y + s[4]; T.z = T.z + s[5];
-      E = E + s[6];
-    }
-    const int lc = M.core_lh[J];
-    for (int I = 0; I < M.n_lhcore; I++) {
-      const double* s = S.gc + ((size_t)I * M.n_c + J) * 10;
-      F.x = F.x - s[0]; F.y = F.y - s[1]; F.z = F.z - s[2];
-      T.x = T.x + s[6]; T.y = T.y + s[7]; T.z = T.z + s[8];
-    }
-    if (lc >= 0) {
-      for (int L = 0; L < M.n_c; L++) {
-        const double* s = S.gc + ((size_t)lc * M.n_c + L) * 10;
-        F.x = F.x + s[0]; F.y = F.y + s[1]; F.z = F.z + s[2];
-        T.x = T.x + s[3]; T.y = T.y + s[4]; T.z = T.z + s[5];
-        E = E + s[9];
-      }
-    }
-  }
-  V3 Fb = ld3(Fm + 3 * j), Tb = ld3(Tm + 3 * j);
-  st3(out.F + 3 * j, V3{Fb.x + F.x, Fb.y + F.y, Fb.z + F.z});
-  st3(out.T + 3 * j, V3{Tb.x + T.x, Tb.y + T.y, Tb.z + T.z});
-  Eout[j] = Ech[j] + E;
-}
-
-// Mixed path: chain_finish with the slot sums spread over the CTA's threads
-// (FP64, many lanes per instruction instead of one thread walking every
-// slot) and folded into the block sum; same terms, another summation order.
-__device__ void chain_finish_mx(const DevModel& M, const DevScratch& S, const double* Fm, const double* Tm,
                                 const double* Ech, DevForces& out, double* Eout, int j, V3 F, V3 T, double E,
                                 double* red) {
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -809,7 +795,6 @@ constexpr int kGatherThreads = 256;
 #endif
 constexpr int kBeadThreads = BD_FP64_BEAD_THREADS;
 
-template <bool MX>
 __global__ void __launch_bounds__(kGatherThreads) k_chain_gather(DevModel M, DevState X, const double* Fm,
                                                                 const double* Tm, const double* Ech,
                                                                 DevScratch S, DevForces out, double* Eout) {
@@ -830,28 +815,15 @@ __global__ void __launch_bounds__(kGatherThreads) k_chain_gather(DevModel M, Dev
         V3 ri = ld3(X.r + 3 * i);
         double d = sqrt((rj.x - ri.x) * (rj.x - ri.x) + (rj.y - ri.y) * (rj.y - ri.y) + (rj.z - ri.z) * (rj.z - ri.z));
         if (d > 25.0) continue;
-        if constexpr (MX) {
-          float zx = (float)(rj.x - ri.x), zy = (float)(rj.y - ri.y), zz = (float)(rj.z - ri.z);
-          float df = sqrtf(zx * zx + zy * zy + zz * zz), mi = 1.f / df;
-          float kap = (float)M.debyell, ex = expf(-kap * df), qf = (float)(M.k_e * qq);
-          float g = qf * ex * (kap * df + 1.f) / (df * df), e = qf * ex / df;
-          if (df <= 8.f) {
-            float sr = (float)M.sDD / df, sr2 = sr * sr, sr6 = sr2 * sr2 * sr2, sr12 = sr6 * sr6;
-            g += (float)M.k_ex * (12.f * sr12 - 6.f * sr6) / df;
-            e += (float)M.k_ex * (sr12 - sr6);
-          }
-          if (j < i) E = E + (double)e;
-          F.x += (double)(g * zx * mi); F.y += (double)(g * zy * mi); F.z += (double)(g * zz * mi);
-          continue;
-        }
-        double mi = 1.0 / d;
+        const double mi = 1.0 / d;
         V3 z{mi * (rj.x - ri.x), mi * (rj.y - ri.y), mi * (rj.z - ri.z)};
-        double g1 = M.k_e * qq * exp(-M.debyell * d) * (M.debyell * d + 1.0) / (d * d);
-        double e = (M.k_e * qq / d) * exp(-M.debyell * d);
+        double e = M.k_e * qq * mi * exp(-M.debyell * d);
+        double g1 = e * fma(M.debyell, d, 1.0) * mi;
         if (d <= 8) {
-          double s1 = M.sDD;
-          g1 = g1 + M.k_ex * ((12.0 / s1) * pow((s1 / d), 13) - (6.0 / s1) * pow((s1 / d), 7));
-          e = e + M.k_ex * (pow(s1 / d, 12) - pow(s1 / d, 6));
+          double s6, s12;
+          lj_powers(M.sDD, mi, s6, s12);
+          g1 = fma(M.k_ex * mi, fma(12.0, s12, -6.0 * s6), g1);
+          e = fma(M.k_ex, s12 - s6, e);
         }
         if (j < i) E = E + e;
         F.x = F.x + g1 * z.x; F.y = F.y + g1 * z.y; F.z = F.z + g1 * z.z;
@@ -859,44 +831,48 @@ __global__ void __launch_bounds__(kGatherThreads) k_chain_gather(DevModel M, Dev
     }
     // tails on this DNA bead (func.cpp:1898-1917); energy on the tail side
     for (int t = tid; t < M.n_tail; t += nt)
-      acc(F, pairF<true, true, MX>(M.q_l, M.t_q[t], eps, M.debye, M.k_ex, M.sTL, rj, ld3(X.r_t + 3 * t), nullptr));
+      if (!far(S, j, S.ot + t))
+        acc(F, pair_f1<true, true>(M.q_l, M.t_q[t], eps, M.debye, M.k_ex, M.sTL, rj, ld3(X.r_t + 3 * t), nullptr));
     // LH beads on this DNA bead (func.cpp:2249-2279); energy on the LH side
     for (int b = tid; b < M.n_LH; b += nt) {
+      if (far(S, j, S.ol + b)) continue;
       int p = lh_param(M, b);
-      acc(F, pairF<true, true, MX>(M.q_l, M.LH_q[p], eps, M.debye, M.k_ex, M.LH_vdw_hl[p], rj, ld3(X.r_lh + 3 * b), nullptr));
+      acc(F, pair_f1<true, true>(M.q_l, M.LH_q[p], eps, M.debye, M.k_ex, M.LH_vdw_hl[p], rj, ld3(X.r_lh + 3 * b), nullptr));
     }
     // globular heads on this DNA bead (func.cpp:2481-2522); energy on the core side
     for (int s = tid; s < M.n_lhcore * M.n_lh_g; s += nt) {
+      if (far(S, j, S.og + s)) continue;
       int m = s % M.n_lh_g;
-      acc(F, pairF<true, true, MX>(M.q_l, M.LH_q[m], eps, M.debye, M.k_ex, M.LH_vdw_hl[m], rj, ld3(X.gpos + 3 * s), nullptr));
+      acc(F, pair_f1<true, true>(M.q_l, M.LH_q[m], eps, M.debye, M.k_ex, M.LH_vdw_hl[m], rj, ld3(X.gpos + 3 * s), nullptr));
     }
   } else {
     const int J = M.core_rank[j];
     const int lc = M.core_lh[J];
     if (lc >= 0) {
-      const int ng = M.n_lh_g;
+      const int ng = M.n_lh_g, hd = S.og + lc * ng;
       // G-head vs linker DNA, tails, LH beads of other LHs, other G-heads
       for (int s = tid; s < ng * M.n; s += nt) {  // func.cpp:2481-2522
         int m = s / M.n, l = s - m * M.n;
-        if (M.type[l] != 0) continue;
+        if (M.type[l] != 0 || far(S, hd + m, l)) continue;
         V3 g = ld3(X.gpos + 3 * (lc * ng + m));
-        V3 f1 = pairF<true, true, MX>(M.LH_q[m], M.q_l, eps, M.debye, M.k_ex, M.LH_vdw_hl[m], g, ld3(X.r + 3 * l), &E);
+        V3 f1 = pair_f1<true, true>(M.LH_q[m], M.q_l, eps, M.debye, M.k_ex, M.LH_vdw_hl[m], g, ld3(X.r + 3 * l), &E);
         acc(F, f1);
         acc(T, torque_rel(f1, M.LH_g_pos + 3 * m, aj, bj, cj));
       }
       for (int s = tid; s < ng * M.n_tail; s += nt) {  // func.cpp:2403-2476
         int m = s / M.n_tail, t = s - m * M.n_tail;
+        if (far(S, hd + m, S.ot + t)) continue;
         V3 g = ld3(X.gpos + 3 * (lc * ng + m));
-        V3 f1 = pairF<true, true, MX>(M.LH_q[m], M.t_q[t], eps, M.debye, M.k_ex, M.LH_vdw_ht[m], g, ld3(X.r_t + 3 * t), &E);
+        V3 f1 = pair_f1<true, true>(M.LH_q[m], M.t_q[t], eps, M.debye, M.k_ex, M.LH_vdw_ht[m], g, ld3(X.r_t + 3 * t), &E);
         acc(F, f1);
         acc(T, torque_rel(f1, M.LH_g_pos + 3 * m, aj, bj, cj));
       }
       for (int s = tid; s < ng * M.n_LH; s += nt) {  // func.cpp:2590-2644
         int m = s / M.n_LH, b = s - m * M.n_LH;
-        if (b / M.nlh == lc) continue;
+        if (b / M.nlh == lc || far(S, hd + m, S.ol + b)) continue;
         int p2 = lh_param(M, b);
         V3 g = ld3(X.gpos + 3 * (lc * ng + m));
-        V3 f1 = pairF<true, true, MX>(M.LH_q[m], M.LH_q[p2], eps, M.debye, M.k_ex, (M.LH_vdw_hh[m] + M.LH_vdw_hh[p2]) / 2,
+        V3 f1 = pair_f1<true, true>(M.LH_q[m], M.LH_q[p2], eps, M.debye, M.k_ex, (M.LH_vdw_hh[m] + M.LH_vdw_hh[p2]) / 2,
                                     g, ld3(X.r_lh + 3 * b), &E);
         acc(F, f1);
         acc(T, torque_rel(f1, M.LH_g_pos + 3 * m, aj, bj, cj));
@@ -904,11 +880,11 @@ __global__ void __launch_bounds__(kGatherThreads) k_chain_gather(DevModel M, Dev
       for (int s = tid; s < ng * M.n_lhcore * ng; s += nt) {  // func.cpp:2649-2719; energy on the lower core
         int m = s / (M.n_lhcore * ng), rest = s - m * (M.n_lhcore * ng);
         int K = rest / ng, m1 = rest - K * ng;
-        if (K == lc) continue;
+        if (K == lc || far(S, hd + m, S.og + rest)) continue;
         V3 g = ld3(X.gpos + 3 * (lc * ng + m));
         V3 g2 = ld3(X.gpos + 3 * (K * ng + m1));
         double e = 0.0;
-        V3 f1 = pairF<true, true, MX>(M.LH_q[m], M.LH_q[m1], eps, M.debye, M.k_ex, (M.LH_vdw_hh[m] + M.LH_vdw_hh[m1]) / 2, g,
+        V3 f1 = pair_f1<true, true>(M.LH_q[m], M.LH_q[m1], eps, M.debye, M.k_ex, (M.LH_vdw_hh[m] + M.LH_vdw_hh[m1]) / 2, g,
                                     g2, &e);
         if (lc < K) E = E + e;
         acc(F, f1);
@@ -951,18 +927,22 @@ __global__ void __launch_bounds__(kGatherThreads) k_chain_gather(DevModel M, Dev
     }
     // LH and G-head forces on this core's anchored tail beads are applied to
     // the core (func.cpp:2361-2391, 2436-2465)
-    for (int t0 = 0; t0 < M.n_tail; t0++) {
+    const int t_lo = M.tails_by_core ? J * M.n_t : 0;
+    const int t_hi = M.tails_by_core ? min((J + 1) * M.n_t, M.n_tail) : M.n_tail;
+    for (int t0 = t_lo; t0 < t_hi; t0++) {
       if (M.t_fix[t0] == 0 || M.t_core_bead[t0] != j) continue;
       V3 rt = ld3(X.r_t + 3 * t0);
       for (int b = tid; b < M.n_LH; b += nt) {
+        if (far(S, S.ot + t0, S.ol + b)) continue;
         int p = lh_param(M, b);
-        V3 f2 = pairF<true, true, MX>(M.t_q[t0], M.LH_q[p], eps, M.debye, M.k_ex, M.LH_vdw_ht[p], rt, ld3(X.r_lh + 3 * b), nullptr);
+        V3 f2 = pair_f1<true, true>(M.t_q[t0], M.LH_q[p], eps, M.debye, M.k_ex, M.LH_vdw_ht[p], rt, ld3(X.r_lh + 3 * b), nullptr);
         acc(F, f2);
         acc(T, torque_abs(f2, rt, rj, aj, bj, cj));
       }
       for (int s = tid; s < M.n_lhcore * M.n_lh_g; s += nt) {
+        if (far(S, S.ot + t0, S.og + s)) continue;
         int m = s % M.n_lh_g;
-        V3 f2 = pairF<true, true, MX>(M.t_q[t0], M.LH_q[m], eps, M.debye, M.k_ex, M.LH_vdw_ht[m], rt, ld3(X.gpos + 3 * s), nullptr);
+        V3 f2 = pair_f1<true, true>(M.t_q[t0], M.LH_q[m], eps, M.debye, M.k_ex, M.LH_vdw_ht[m], rt, ld3(X.gpos + 3 * s), nullptr);
         acc(F, f2);
         acc(T, torque_abs(f2, rt, rj, aj, bj, cj));
       }
@@ -973,8 +953,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_chain_gather(DevModel M, Dev
 
 // ------------------------------------------------------------ tails
 // One warp per tail bead (func.cpp:1809-1917, 2343-2476 for the LH side).
-template <bool MX>
-__global__ void k_tail_gather(DevModel M, DevState X, DevForces out, double* Eout) {
+__global__ void k_tail_gather(DevModel M, DevState X, DevScratch S, DevForces out, double* Eout) {
   int lane = threadIdx.x & 31;
   int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t >= M.n_tail) return;
@@ -1010,27 +989,30 @@ __global__ void k_tail_gather(DevModel M, DevState X, DevForces out, double* Eou
   }
   // tail/tail electrostatics (func.cpp:1863-1891); energy on the lower index
   for (int u = lane; u < nt; u += 32) {
-    if (u == t) continue;
+    if (u == t || far(S, S.ot + t, S.ot + u)) continue;
     int lo = t < u ? t : u, hi = t < u ? u : t;
     if (!(grp[lo] != grp[hi] || hi > lo + 2)) continue;
     double e = 0.0;
-    acc(F, pairF<true, false, MX>(M.t_q[t], M.t_q[u], eps, M.debye, 0.0, 0.0, rt, ld3(X.r_t + 3 * u), &e));
+    acc(F, pair_f1<true, false>(M.t_q[t], M.t_q[u], eps, M.debye, 0.0, 0.0, rt, ld3(X.r_t + 3 * u), &e));
     if (t < u) E = E + e;
   }
   // linker DNA (func.cpp:1898-1917); energy here
   for (int q = lane; q < M.n_dna; q += 32) {
     int j = M.dna_bead[q];
-    acc(F, pairF<true, true, MX>(M.t_q[t], M.q_l, eps, M.debye, M.k_ex, M.sTL, rt, ld3(X.r + 3 * j), &E));
+    if (far(S, S.ot + t, j)) continue;
+    acc(F, pair_f1<true, true>(M.t_q[t], M.q_l, eps, M.debye, M.k_ex, M.sTL, rt, ld3(X.r + 3 * j), &E));
   }
   if (M.t_fix[t] == 0) {
     // LH beads and globular heads act on free tail beads (energies on their side)
     for (int b = lane; b < M.n_LH; b += 32) {
+      if (far(S, S.ot + t, S.ol + b)) continue;
       int p = lh_param(M, b);
-      acc(F, pairF<true, true, MX>(M.t_q[t], M.LH_q[p], eps, M.debye, M.k_ex, M.LH_vdw_ht[p], rt, ld3(X.r_lh + 3 * b), nullptr));
+      acc(F, pair_f1<true, true>(M.t_q[t], M.LH_q[p], eps, M.debye, M.k_ex, M.LH_vdw_ht[p], rt, ld3(X.r_lh + 3 * b), nullptr));
     }
     for (int s = lane; s < M.n_lhcore * M.n_lh_g; s += 32) {
+      if (far(S, S.ot + t, S.og + s)) continue;
       int m = s % M.n_lh_g;
-      acc(F, pairF<true, true, MX>(M.t_q[t], M.LH_q[m], eps, M.debye, M.k_ex, M.LH_vdw_ht[m], rt, ld3(X.gpos + 3 * s), nullptr));
+      acc(F, pair_f1<true, true>(M.t_q[t], M.LH_q[m], eps, M.debye, M.k_ex, M.LH_vdw_ht[m], rt, ld3(X.gpos + 3 * s), nullptr));
     }
   }
   F.x = wsum(F.x); F.y = wsum(F.y); F.z = wsum(F.z); E = wsum(E);
@@ -1042,8 +1024,7 @@ __global__ void k_tail_gather(DevModel M, DevState X, DevForces out, double* Eou
 
 // ------------------------------------------------------------ LH beads
 // One warp per mobile LH bead (func.cpp:2109-2398, 2588-2644, 2725-2777).
-template <bool MX>
-__global__ void k_lh_gather(DevModel M, DevState X, DevForces out, double* Eout) {
+__global__ void k_lh_gather(DevModel M, DevState X, DevScratch S, DevForces out, double* Eout) {
   int lane = threadIdx.x & 31;
   int bI = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (bI >= M.n_LH) return;
@@ -1088,32 +1069,34 @@ __global__ void k_lh_gather(DevModel M, DevState X, DevForces out, double* Eout)
   }
   // LH/LH (func.cpp:2190-2244); energy on the lower index
   for (int u = lane; u < nL; u += 32) {
-    if (u == bI) continue;
+    if (u == bI || far(S, S.ol + bI, S.ol + u)) continue;
     int pu = lh_param(M, u);
     double e = 0.0;
     double sig = (M.LH_vdw_hh[pb] + M.LH_vdw_hh[pu]) / 2;
     if (bI / nlh == u / nlh) {
       int lo = bI < u ? bI : u, hi = bI < u ? u : bI;
       if (!(hi > lo + 1)) continue;
-      acc(F, pairF<false, true, MX>(0.0, 0.0, eps, M.debye, M.k_ex, sig, rb, ld3(X.r_lh + 3 * u), &e));
+      acc(F, pair_f1<false, true>(0.0, 0.0, eps, M.debye, M.k_ex, sig, rb, ld3(X.r_lh + 3 * u), &e));
     } else {
-      acc(F, pairF<true, true, MX>(M.LH_q[pb], M.LH_q[pu], eps, M.debye, M.k_ex, sig, rb, ld3(X.r_lh + 3 * u), &e));
+      acc(F, pair_f1<true, true>(M.LH_q[pb], M.LH_q[pu], eps, M.debye, M.k_ex, sig, rb, ld3(X.r_lh + 3 * u), &e));
     }
     if (bI < u) E = E + e;
   }
   // linker DNA and tails (func.cpp:2249-2398); energies here
   for (int q = lane; q < M.n_dna; q += 32) {
     int j = M.dna_bead[q];
-    acc(F, pairF<true, true, MX>(M.LH_q[pb], M.q_l, eps, M.debye, M.k_ex, M.LH_vdw_hl[pb], rb, ld3(X.r + 3 * j), &E));
+    if (far(S, S.ol + bI, j)) continue;
+    acc(F, pair_f1<true, true>(M.LH_q[pb], M.q_l, eps, M.debye, M.k_ex, M.LH_vdw_hl[pb], rb, ld3(X.r + 3 * j), &E));
   }
   for (int t = lane; t < M.n_tail; t += 32)
-    acc(F, pairF<true, true, MX>(M.LH_q[pb], M.t_q[t], eps, M.debye, M.k_ex, M.LH_vdw_ht[pb], rb, ld3(X.r_t + 3 * t), &E));
+    if (!far(S, S.ol + bI, S.ot + t))
+      acc(F, pair_f1<true, true>(M.LH_q[pb], M.t_q[t], eps, M.debye, M.k_ex, M.LH_vdw_ht[pb], rb, ld3(X.r_t + 3 * t), &E));
   // globular heads of the other LHs (func.cpp:2588-2644); energy on the core
   const int own = bI / nlh;
   for (int s = lane; s < M.n_lhcore * M.n_lh_g; s += 32) {
     int K = s / M.n_lh_g, m = s - K * M.n_lh_g;
-    if (K == own) continue;
-    acc(F, pairF<true, true, MX>(M.LH_q[pb], M.LH_q[m], eps, M.debye, M.k_ex, (M.LH_vdw_hh[m] + M.LH_vdw_hh[pb]) / 2, rb,
+    if (K == own || far(S, S.ol + bI, S.og + s)) continue;
+    acc(F, pair_f1<true, true>(M.LH_q[pb], M.LH_q[m], eps, M.debye, M.k_ex, (M.LH_vdw_hh[m] + M.LH_vdw_hh[pb]) / 2, rb,
                                ld3(X.gpos + 3 * s), nullptr));
   }
   F.x = wsum(F.x); F.y = wsum(F.y); F.z = wsum(F.z); E = wsum(E);
@@ -1659,7 +1642,7 @@ __global__ void __launch_bounds__(kGatherCoreThreads) k_chain_gather_mx(DevModel
   T.x += aj.x * A.s[3] + aj.y * A.s[4] + aj.z * A.s[5];
   T.y += bj.x * A.s[3] + bj.y * A.s[4] + bj.z * A.s[5];
   T.z += cj.x * A.s[3] + cj.y * A.s[4] + cj.z * A.s[5];
-  chain_finish_mx(M, S, Fm, Tm, Ech, out, Eout, j, F, T, E, red);
+  chain_finish(M, S, Fm, Tm, Ech, out, Eout, j, F, T, E, red);
 }
 
 // Total energy: chain, tail and LH shares in a fixed order.
@@ -1687,12 +1670,10 @@ int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& S, int mi
 #define KSEL(name) (mixed ? name<true> : name<false>)
   auto k_dna_coreX = KSEL(k_dna_core);
   auto k_ghead_coreX = KSEL(k_ghead_core);
-  auto k_tail_gatherX = KSEL(k_tail_gather);
-  auto k_lh_gatherX = KSEL(k_lh_gather);
-  auto k_chain_gatherX = KSEL(k_chain_gather);
 #undef KSEL
   if (M.n_lhcore > 0) { k_gpos<<<cdiv(M.n_lhcore * M.n_lh_g, 128), 128, 0, st>>>(M, X); L++; }
-  if (mixed) { k_mirror<<<cdiv(S.npos, 128), 128, 0, st>>>(M, X, S.ph, S.pl, S.npos); L++; }
+  k_mirror<<<cdiv(S.npos, 128), 128, 0, st>>>(M, X, S.ph, S.pl, S.npos);
+  L++;
   if (M.n > 1) {
     k_chain_bonds<<<cdiv(M.n - 1, kBeadThreads), kBeadThreads, 0, st>>>(M, X, S.bonds);
     L++;
@@ -1702,16 +1683,13 @@ int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& S, int mi
   if (M.n_c > 1) {
     if (mixed) {
       size_t sm = (size_t)((14 * M.Nq + 1) / 2 + 32 * 10) * sizeof(double);
-      k_core_core_mx<<<dim3(M.n_c, M.n_c, kCCSplit), kCCThreads, sm, st>>>(M, X, S, S.ccp);
-      k_cc_sum<<<cdiv(M.n_c * M.n_c * 10, 256), 256, 0, st>>>(M.n_c, S.ccp, S.cc);
-      L++;
+      k_core_core_mx<<<dim3(M.n_c * (M.n_c - 1) / 2, kCCSplit), kCCThreads, sm, st>>>(M, X, S, S.ccp);
     } else {
       size_t sm = (size_t)(6 * M.Nq + 32 * 10) * sizeof(double);
-      k_core_core<<<dim3(M.n_c, M.n_c, kCCSplit), kCCThreads, sm, st>>>(M, X, S.ccp);
-      k_cc_sum<<<cdiv(M.n_c * M.n_c * 10, 256), 256, 0, st>>>(M.n_c, S.ccp, S.cc);
-      L++;
+      k_core_core<<<M.n_c * (M.n_c - 1) / 2 * kCC64Split, kCC64Threads, sm, st>>>(M, X, S.ccp);
     }
-    L++;
+    k_cc_sum<<<cdiv(M.n_c * M.n_c * 10, 256), 256, 0, st>>>(M.n_c, mixed ? kCCSplit : kCC64Split, S.ccp, S.cc);
+    L += 2;
   }
   if (M.n_dna > 0 && M.n_c > 0) { k_dna_coreX<<<cdiv(M.n_dna * M.n_c * 32, 256), 256, 0, st>>>(M, X, S, S.dc); L++; }
   if (M.n_lhcore > 0) { k_ghead_coreX<<<cdiv(M.n_lhcore * M.n_c * 32, 256), 256, 0, st>>>(M, X, S.gc); L++; }
@@ -1724,9 +1702,9 @@ int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& S, int mi
     if (M.n_c > 0) k_chain_gather_mx<<<M.n_c, kGatherCoreThreads, 0, st>>>(M, X, Fm, Tm, Ebond, S, out, Ech, M.core_bead);
     L += (M.n_dna > 0) + (M.n_c > 0) - 1;  // one chain launch is counted below
   } else {
-    if (M.n_tail > 0) { k_tail_gatherX<<<cdiv(M.n_tail * 32, 256), 256, 0, st>>>(M, X, out, Et); L++; }
-    if (M.n_LH > 0) { k_lh_gatherX<<<cdiv(M.n_LH * 32, 256), 256, 0, st>>>(M, X, out, El); L++; }
-    k_chain_gatherX<<<M.n, kGatherThreads, 0, st>>>(M, X, Fm, Tm, Ebond, S, out, Ech);
+    if (M.n_tail > 0) { k_tail_gather<<<cdiv(M.n_tail * 32, 256), 256, 0, st>>>(M, X, S, out, Et); L++; }
+    if (M.n_LH > 0) { k_lh_gather<<<cdiv(M.n_LH * 32, 256), 256, 0, st>>>(M, X, S, out, El); L++; }
+    k_chain_gather<<<M.n, kGatherThreads, 0, st>>>(M, X, Fm, Tm, Ebond, S, out, Ech);
   }
   k_energy<<<1, 256, 0, st>>>(M.n + M.n_tail + M.n_LH, S.ebuf, out.E);
   return L + 2;
