@@ -89,140 +89,167 @@ __global__ void __launch_bounds__(256) k_rpy_mx(int nD, const float4* __restrict
 }
 
 // ------------------------------------------------------------ Cholesky
-constexpr int kNB = 64;
+// Blocks of 64 columns, factored as two panels of kNB = 32: the FP64 pipe (two
+// lanes a clock per SM) makes a diagonal block of 64 on one SM and row solves
+// of 64 columns on a few SMs the serial part of a small factorisation.
+constexpr int kNB = 32;
 
-// Factor the kb x kb diagonal block at (k0,k0) in shared memory.
-__global__ void __launch_bounds__(256) k_potrf_diag(double* A, int lda, int k0, int kb, int* negpiv) {
-  __shared__ double S[kNB][kNB + 1];
-  const int tid = threadIdx.x;
-  for (int e = tid; e < kb * kb; e += blockDim.x) {
-    int c = e / kb, rr = e - c * kb;  // column-major walk
-    S[rr][c] = (rr >= c) ? A[(size_t)(k0 + c) * lda + k0 + rr] : 0.0;
+// 1 / sqrt(f), f > 0: from FP32's by one third-order step (22 bits to 2 ulp in
+// five FP64 operations instead of a root and a division)
+__device__ __forceinline__ double rsqrt_nr(double f) {
+  const unsigned e = (unsigned)__double2hiint(f) >> 20;  // sign and exponent
+  if (e < 1023 - 100 || e > 1023 + 100) return 1.0 / sqrt(f);
+  const double y = (double)rsqrtf((float)f);
+  const double d = fma(-f * y, y, 1.0);
+  return fma(y * d, fma(0.375, d, 0.5), y);
+}
+
+// Factor the kb x kb diagonal block at (k0, k0): right-looking, a row per lane,
+// column j in the registers of warp j % 4 (one warp per FP64 pipe: a warp's
+// FP64 operation holds its pipe for 64 cycles), column c to the others through
+// shared memory.  A negative pivot is replaced by its absolute value and
+// counted (func.cpp:827-833).  Bound by the pivots' chain (ten dependent FP64
+// operations and a barrier each): 64 columns by 256 threads with three
+// barriers a column took 119 us, 32 by one warp 69, by four 25 (3N = 912:
+// 5.1 -> 1.7 ms in all, 1,944: 13.3 -> 5.2, 11,700: 499 -> 458).
+__global__ void __launch_bounds__(128) k_potrf_diag(double* A, int lda, int k0, int kb, int* negpiv) {
+  __shared__ double T[kNB][kNB];  // T[c][j] = L_jc (below the diagonal)
+  __shared__ double piv[kNB];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double* col = A + (size_t)k0 * lda + k0 + lane;
+  double a[kNB / 4];
+#pragma unroll
+  for (int i = 0; i < kNB / 4; i++) {
+    const int j = 4 * i + w;
+    a[i] = (lane < kb && j <= lane) ? col[(size_t)j * lda] : (j == lane ? 1.0 : 0.0);
   }
-  __syncthreads();
-  // the pivot's reciprocal, formed once per column by thread 0 beside its
-  // square root, scales the column (one FP64 division per column instead of
-  // one per element on the column's critical path)
-  __shared__ double rpiv;
-  for (int c = 0; c < kb; c++) {
-    if (tid == 0) {
-      double f = S[c][c];
-      if (f < 0) {
+#pragma unroll
+  for (int c = 0; c < kNB; c++) {
+    if (w == (c & 3)) {
+      double f = __shfl_sync(0xffffffffu, a[c >> 2], c);
+      if (__double2hiint(f) < 0 && f < 0) {
         f = -f;
-        atomicAdd(negpiv, 1);
+        if (lane == 0) atomicAdd(negpiv, 1);
       }
-      const double d = sqrt(f);
-      S[c][c] = d;
-      rpiv = 1.0 / d;
+      T[c][lane] = a[c >> 2] *= rsqrt_nr(f);
+      if (lane == c) piv[c] = f;
     }
     __syncthreads();
-    const double rp = rpiv;
-    for (int rr = c + 1 + tid; rr < kb; rr += blockDim.x) S[rr][c] = S[rr][c] * rp;
-    __syncthreads();
-    // rank-1 update of the remaining lower triangle
-    int rem = kb - c - 1;
-    for (int e = tid; e < rem * rem; e += blockDim.x) {
-      int q = e / rem, rr = e - q * rem;
-      int col = c + 1 + q, row = c + 1 + rr;
-      if (row >= col) S[row][col] = S[row][col] - S[row][c] * S[col][c];
-    }
-    __syncthreads();
+    const double l = T[c][lane];
+#pragma unroll
+    for (int i = c >> 2; i < kNB / 4; i++)  // column c + 1 first, of the warp that takes it off next
+      if (4 * i + w > c) a[i] = fma(-l, T[c][4 * i + w], a[i]);  // (rows above the diagonal: not used)
   }
-  for (int e = tid; e < kb * kb; e += blockDim.x) {
-    int c = e / kb, rr = e - c * kb;
-    if (rr >= c) A[(size_t)(k0 + c) * lda + k0 + rr] = S[rr][c];
+#pragma unroll
+  for (int i = 0; i < kNB / 4; i++) {
+    const int j = 4 * i + w;
+    if (lane < kb && j < lane) col[(size_t)j * lda] = a[i];
   }
+  if (w == 0 && lane < kb) col[(size_t)lane * lda] = sqrt(piv[lane]);
 }
 
-// Panel solve: rows [k0+kb, m) of columns [k0, k0+kb): X L_kk^T = A, a
-// row per thread (64 dependent column steps on the FP64 pipe), 128 rows per
-// CTA (32 per CTA spread the rows over more SMs but staged L_kk four times
-// longer per thread: 229 vs 210 us per panel at 3N = 1,944)
-constexpr int kTrsmThreads = 128;
-__global__ void __launch_bounds__(kTrsmThreads) k_trsm_panel(double* A, int lda, int m, int k0, int kb) {
-  __shared__ double Lkk[kNB][kNB + 1];
-  __shared__ double rdiag[kNB];  // 1 / L_cc: the row solves multiply instead of dividing
-  for (int e = threadIdx.x; e < kb * kb; e += blockDim.x) {
-    int c = e / kb, rr = e - c * kb;
-    Lkk[rr][c] = (rr >= c) ? A[(size_t)(k0 + c) * lda + k0 + rr] : 0.0;
+// Panel solve: rows [k0+kb, m) of columns [k0, k0+kb): X L_kk^T = A,
+// right-looking in registers.  A warp takes 8 rows, lane 8 g + r the columns
+// 4 i + g of row r: four times as many warps as with a row per lane, so that
+// the rows of a small matrix reach all FP64 pipes.  64 columns left-looking
+// with a row per thread: 188 us at 3N = 1,944; 32 columns with a row per lane
+// 24 us; now 16.
+__global__ void __launch_bounds__(128) k_trsm_panel(double* A, int lda, int m, int k0, int kb) {
+  __shared__ double L[kNB][kNB];  // L[c][j] = L_jc, j > c; else 0
+  __shared__ double rd[kNB];
+  const int lane = threadIdx.x & 31, g = lane >> 3;
+  const int r = k0 + kb + blockIdx.x * 32 + (threadIdx.x >> 5) * 8 + (lane & 7);
+  double* col = A + (size_t)k0 * lda + r;
+  double x[kNB / 4];
+#pragma unroll
+  for (int i = 0; i < kNB / 4; i++) x[i] = (r < m && 4 * i + g < kb) ? col[(size_t)(4 * i + g) * lda] : 0.0;
+  for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
+    const int c = e / kNB, j = e % kNB;
+    const double v = (j < kb && c <= j) ? A[(size_t)(k0 + c) * lda + k0 + j] : 0.0;
+    if (c == j) rd[c] = j < kb ? 1.0 / v : 0.0;
+    L[c][j] = c < j ? v : 0.0;
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < kb; c += blockDim.x) rdiag[c] = 1.0 / Lkk[c][c];
-  __syncthreads();
-  int r = k0 + kb + blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= m) return;
-  double x[kNB];
 #pragma unroll
   for (int c = 0; c < kNB; c++) {
-    if (c < kb) x[c] = A[(size_t)(k0 + c) * lda + r];
+    const double xc = __shfl_sync(0xffffffffu, x[c >> 2], (lane & 7) + 8 * (c & 3)) * rd[c];
+    if (g == (c & 3)) x[c >> 2] = xc;
+#pragma unroll
+    for (int i = c >> 2; i < kNB / 4; i++) x[i] = fma(-xc, L[c][4 * i + g], x[i]);
   }
+  if (r < m)
 #pragma unroll
-  for (int c = 0; c < kNB; c++) {
-    if (c < kb) {
-      double v = x[c];
-#pragma unroll
-      for (int q = 0; q < kNB; q++)
-        if (q < c) v = v - x[q] * Lkk[c][q];
-      x[c] = v * rdiag[c];
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < kNB; c++)
-    if (c < kb) A[(size_t)(k0 + c) * lda + r] = x[c];
+    for (int i = 0; i < kNB / 4; i++)
+      if (4 * i + g < kb) col[(size_t)(4 * i + g) * lda] = x[i];
 }
 
-// Trailing update of the lower triangle of A[t0:, t0:] (t0 = k0 + kb):
-// A_ij -= P_i P_j^T with P = A[:, k0:k0+kb].  64 x 64 output tile per CTA,
-// 256 threads each owning a 4 x 4 register block.
-constexpr int kTM = 64;
+// Update of the lower triangle of A[t0:, t0:jend] by the kb columns from k0:
+// A_ij -= P_i P_j^T with P = A[:, k0:k0+kb].  TM x TN output tile per CTA (a
+// triangle of square ones, or one column of them), each thread an MR x NR
+// register block, at least four warps: one per FP64 pipe of the SM, which
+// bounds it.
 constexpr int kKC = 16;  // panel columns staged per pass
 
-__global__ void __launch_bounds__(256) k_syrk_update(double* A, int lda, int m, int k0, int kb) {
-  const int t0 = k0 + kb;
-  const int bi = blockIdx.y, bj = blockIdx.x;
-  if (bj > bi) return;
-  const int row0 = t0 + bi * kTM, col0 = t0 + bj * kTM;
-  __shared__ double Pr[kKC][kTM + 1];  // [k][row]
-  __shared__ double Pc[kKC][kTM + 1];  // [k][col]
+// tile (bi, bj <= bi) of a triangle from its row-major index t (a grid without
+// the triangle's empty half: the SMs' shares of the tiles are then even)
+__device__ __forceinline__ void tri_tile(int t, int& bi, int& bj) {
+  bi = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
+  while ((bi + 1) * (bi + 2) / 2 <= t) bi++;
+  while (bi * (bi + 1) / 2 > t) bi--;
+  bj = t - bi * (bi + 1) / 2;
+}
+
+template <int TM, int TN, int MR, int NR>
+__global__ void __launch_bounds__(TM * TN / (MR * NR)) k_syrk_update(double* A, int lda, int m, int k0, int kb, int t0, int jend) {
+  constexpr int NT = TM * TN / (MR * NR);
+  int bi = blockIdx.x, bj = 0;  // TM != TN: one column of tiles
+  if (TM == TN) tri_tile(blockIdx.x, bi, bj);
+  const int row0 = t0 + bi * TM, col0 = t0 + bj * TN;
+  __shared__ double Pr[kKC][TM + 1];  // [k][row]
+  __shared__ double Pc[kKC][TN + 1];  // [k][col]
   const int tid = threadIdx.x;
-  const int tr = (tid & 15) * 4, tc = (tid >> 4) * 4;
-  double acc[4][4];
+  const int tr = (tid % (TM / MR)) * MR, tc = (tid / (TM / MR)) * NR;
+  double acc[MR][NR];
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int a = 0; a < MR; a++)
 #pragma unroll
-    for (int b = 0; b < 4; b++) acc[a][b] = 0.0;
+    for (int b = 0; b < NR; b++) acc[a][b] = 0.0;
   for (int kc = 0; kc < kb; kc += kKC) {
     const int kn = kb - kc < kKC ? kb - kc : kKC;
-    for (int e = tid; e < kKC * kTM; e += blockDim.x) {
-      int k = e / kTM, q = e - k * kTM;
-      int rr = row0 + q, cc = col0 + q;
-      bool in = k < kn;
-      Pr[k][q] = (in && rr < m) ? A[(size_t)(k0 + kc + k) * lda + rr] : 0.0;
-      Pc[k][q] = (in && cc < m) ? A[(size_t)(k0 + kc + k) * lda + cc] : 0.0;
+    for (int e = tid; e < kKC * TM; e += NT) {
+      const int k = e / TM, q = e - k * TM;
+      Pr[k][q] = (k < kn && row0 + q < m) ? A[(size_t)(k0 + kc + k) * lda + row0 + q] : 0.0;
+    }
+    for (int e = tid; e < kKC * TN; e += NT) {
+      const int k = e / TN, q = e - k * TN;
+      Pc[k][q] = (k < kn && col0 + q < jend) ? A[(size_t)(k0 + kc + k) * lda + col0 + q] : 0.0;
     }
     __syncthreads();
 #pragma unroll 4
     for (int k = 0; k < kKC; k++) {
-      double pr[4], pc[4];
+      double a4[MR], b4[NR];
 #pragma unroll
-      for (int a = 0; a < 4; a++) { pr[a] = Pr[k][tr + a]; pc[a] = Pc[k][tc + a]; }
+      for (int q = 0; q < MR; q++) a4[q] = Pr[k][tr + q];
 #pragma unroll
-      for (int a = 0; a < 4; a++)
+      for (int q = 0; q < NR; q++) b4[q] = Pc[k][tc + q];
 #pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = fma(pr[a], pc[b], acc[a][b]);
+      for (int a = 0; a < MR; a++)
+#pragma unroll
+        for (int b = 0; b < NR; b++) acc[a][b] = fma(a4[a], b4[b], acc[a][b]);
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int b = 0; b < 4; b++) {
-    int cc = col0 + tc + b;
-    if (cc >= m) continue;
+  for (int b = 0; b < NR; b++) {
+    const int cc = col0 + tc + b;
+    if (cc >= jend) continue;
 #pragma unroll
-    for (int a = 0; a < 4; a++) {
-      int rr = row0 + tr + a;
-      if (rr >= m || rr < cc) continue;
-      double* p = A + (size_t)cc * lda + rr;
-      *p = *p - acc[a][b];
+    for (int a = 0; a < MR; a++) {
+      const int rr = row0 + tr + a;
+      if (rr < m && rr >= cc) {
+        double* p = A + (size_t)cc * lda + rr;
+        *p = *p - acc[a][b];
+      }
     }
   }
 }
@@ -304,19 +331,38 @@ void rpy_assemble(int nD, const double* r_all, const double* rad, double a1, dou
     k_rpy<<<dim3(nt, nt), dim3(kRpyTile, 8), 0, st>>>(nD, r_all, rad, a1, a2, A, lda);
 }
 
+// Blocks of 2 kNB columns: panel, the second panel's columns updated by the
+// first, panel, then the trailing triangle by both (K = 64, half the passes
+// over it).  The triangle's tiles are 32 wide: a tile takes 17 us on its SM's
+// FP64 pipe and 64-wide ones 69, which leave SMs idle in a last wave and gain
+// nothing at any size (3N = 3,888: 23.1 ms, 22.5 with 32).
 int potrf_fp64(int m, double* A, int lda, double* /*rd_acc*/, const double* /*p*/, double /*s2dt*/, int* d_negpiv,
                cudaStream_t st) {
   int launches = 0;
-  for (int k0 = 0; k0 < m; k0 += kNB) {
-    int kb = m - k0 < kNB ? m - k0 : kNB;
-    k_potrf_diag<<<1, 256, 0, st>>>(A, lda, k0, kb, d_negpiv);
+  auto panel = [&](int k0) {  // returns its width
+    const int kb = m - k0 < kNB ? m - k0 : kNB;
+    k_potrf_diag<<<1, 128, 0, st>>>(A, lda, k0, kb, d_negpiv);
     launches++;
-    int rest = m - k0 - kb;
+    const int rest = m - k0 - kb;
+    if (rest > 0) {
+      k_trsm_panel<<<cdiv(rest, 32), 128, 0, st>>>(A, lda, m, k0, kb);
+      launches++;
+    }
+    return kb;
+  };
+  for (int k0 = 0; k0 < m; k0 += 2 * kNB) {
+    int kb = panel(k0);
+    const int k1 = k0 + kb;
+    if (k1 >= m) break;
+    const int jend = k1 + kNB < m ? k1 + kNB : m;
+    k_syrk_update<16, 32, 2, 2><<<cdiv(m - k1, 16), 128, 0, st>>>(A, lda, m, k0, kb, k1, jend);
+    launches++;
+    kb += panel(k1);
+    const int t0 = k0 + kb, rest = m - t0;
     if (rest <= 0) break;
-    k_trsm_panel<<<cdiv(rest, kTrsmThreads), kTrsmThreads, 0, st>>>(A, lda, m, k0, kb);
-    int nt = cdiv(rest, kTM);
-    k_syrk_update<<<dim3(nt, nt), 256, 0, st>>>(A, lda, m, k0, kb);
-    launches += 2;
+    const int nt = cdiv(rest, 32);
+    k_syrk_update<32, 32, 4, 2><<<nt * (nt + 1) / 2, 128, 0, st>>>(A, lda, m, k0, kb, t0, m);
+    launches++;
   }
   return launches;
 }
