@@ -241,9 +241,16 @@ __global__ void __launch_bounds__(128) k_adj_dnacore(DevModel M, const double* _
 }
 
 // ------------------------------------------------------------ core-core
-// one CTA per core pair; threads over the first core's charges, the second
-// core's sites (position, torque-adjoint terms) staged in shared memory
-constexpr int kCcThreads = 64;  // core i's sites per CTA of a core pair
+// A warp takes 32 of the first core's sites against a quarter of the second
+// core's, staged in shared memory (position, torque-adjoint terms).  The force
+// is G(d) z, so its vector-Jacobian products are G fbar + (G'/d)(fbar.z) z and
+// dG/dkappa (fbar.z): 60 operations a charge pair where four-wide dual numbers
+// took 300.  Bound by the FP64 pipe; one-warp CTAs and the split over the
+// second core's sites put the few pairs of a small fibre on all of them (two
+// warps per 64 sites filled a quarter): 6 nucleosomes, 15 pairs: 2,582 us with
+// dual numbers, 345 now.
+constexpr int kCcThreads = 32;  // core i's sites per CTA of a core pair
+constexpr int kCcSplit = 4;     // CTAs over core j's sites
 
 template <class R>
 __global__ void __launch_bounds__(kCcThreads) k_adj_corecore(DevModel M, const double* __restrict__ x,
@@ -268,10 +275,10 @@ __global__ void __launch_bounds__(kCcThreads) k_adj_corecore(DevModel M, const d
     Ti[q] = R(fb[n3 + 3 * i + q]);
     Tj[q] = R(fb[n3 + 3 * j + q]);
   }
-  const int Nq = M.Nq;
-  for (int l = threadIdx.x; l < Nq; l += blockDim.x) {
+  const int Nq = M.Nq, l0 = Nq * blockIdx.z / kCcSplit, l1 = Nq * (blockIdx.z + 1) / kCcSplit;
+  for (int l = l0 + threadIdx.x; l < l1; l += blockDim.x) {
     R cp[3] = {R(M.core_pos[3 * l]), R(M.core_pos[3 * l + 1]), R(M.core_pos[3 * l + 2])};
-    R* e = sl + 13 * l;  // core j's sites, staged by every CTA of the pair
+    R* e = sl + 13 * (l - l0);  // core j's sites of this CTA
     for (int q = 0; q < 3; q++) e[q] = xj[q] + xj[3 + q] * cp[0] + xj[6 + q] * cp[1] + xj[9 + q] * cp[2];
     R Q[3];
     cross3(Tj, cp, Q);
@@ -286,8 +293,6 @@ __global__ void __launch_bounds__(kCcThreads) k_adj_corecore(DevModel M, const d
   R acc[25];
   for (int q = 0; q < 25; q++) acc[q] = R(0);  // bead i: r a b c (12), bead j: r a b c (12), kappa
   const R ke = R(M.k_e), kex = R(M.k_ex), sg = R(M.sCC);
-  // this CTA's slice of core i's sites: one per thread (the pair spread over
-  // gridDim.y small CTAs, so the pairs of a step balance across the SMs)
   const int kend = min(Nq, (int)(blockIdx.y + 1) * (int)blockDim.x);
   for (int k = blockIdx.y * blockDim.x + threadIdx.x; k < kend; k += blockDim.x) {
     const R cp[3] = {R(M.core_pos[3 * k]), R(M.core_pos[3 * k + 1]), R(M.core_pos[3 * k + 2])};
@@ -298,29 +303,32 @@ __global__ void __launch_bounds__(kCcThreads) k_adj_corecore(DevModel M, const d
     for (int q = 0; q < 3; q++) Ki[q] = Qi[0] * xi[3 + q] + Qi[1] * xi[6 + q] + Qi[2] * xi[9 + q];
     R sumf[3] = {R(0), R(0), R(0)}, sumz[3] = {R(0), R(0), R(0)}, kap = R(0);
     R rj[3] = {R(0), R(0), R(0)}, aj[3] = {R(0), R(0), R(0)}, bj[3] = {R(0), R(0), R(0)}, cj3[3] = {R(0), R(0), R(0)};
-    for (int l = 0; l < Nq; l++) {
-      const R* e = sl + 13 * l;
-      using D = Dual<R, 4>;
-      D zd[3], f[3];
+    const R kd = R(M.debye);
+    for (int l = l0; l < l1; l++) {
+      const R* e = sl + 13 * (l - l0);
+      R z[3], fbar[3];
       for (int q = 0; q < 3; q++) {
-        zd[q] = D(pk[q] - e[q]);
-        zd[q].d[q] = R(1);
+        z[q] = pk[q] - e[q];
+        fbar[q] = Fi[q] - Fj[q] + Ki[q] - e[6 + q];
       }
-      D kk(M.debye);
-      kk.d[3] = R(1);
-      pair_site(ke * qk * e[12], true, true, kex, sg, zd, kk, f);
-      R fbar[3];
-      for (int q = 0; q < 3; q++) fbar[q] = Fi[q] - Fj[q] + Ki[q] - e[6 + q];
-      R zb[3];
-      for (int g = 0; g < 3; g++) zb[g] = fbar[0] * f[0].d[g] + fbar[1] * f[1].d[g] + fbar[2] * f[2].d[g];
-      kap += fbar[0] * f[0].d[3] + fbar[1] * f[1].d[3] + fbar[2] * f[2].d[3];
+      const R d = norm3(z), mi = R(1) / d, m2 = mi * mi, x1 = kd * d;
+      const R ex = ke * qk * e[12] * vexp(-x1) * mi * m2;
+      R G = ex * (x1 + R(1)), H = -ex * m2 * (x1 * (x1 + R(3)) + R(3));  // H = G' / d
+      if (val(d) <= 8.0) {
+        const R u = sg * mi, u2 = u * u, s6 = u2 * u2 * u2, s12 = s6 * s6;
+        G += kex * m2 * (R(12) * s12 - R(6) * s6);
+        H += kex * m2 * m2 * (R(48) * s6 - R(168) * s12);
+      }
+      const R fz = fbar[0] * z[0] + fbar[1] * z[1] + fbar[2] * z[2];
+      kap -= ex * x1 * d * fz;
       for (int q = 0; q < 3; q++) {
-        sumf[q] += f[q].v;
-        sumz[q] += zb[q];
-        rj[q] -= zb[q];
-        aj[q] += -e[3] * f[q].v - e[9] * zb[q];
-        bj[q] += -e[4] * f[q].v - e[10] * zb[q];
-        cj3[q] += -e[5] * f[q].v - e[11] * zb[q];
+        const R f = G * z[q], zb = G * fbar[q] + H * fz * z[q];
+        sumf[q] += f;
+        sumz[q] += zb;
+        rj[q] -= zb;
+        aj[q] += -e[3] * f - e[9] * zb;
+        bj[q] += -e[4] * f - e[10] * zb;
+        cj3[q] += -e[5] * f - e[11] * zb;
       }
     }
     for (int q = 0; q < 3; q++) {
@@ -973,8 +981,9 @@ int forces_vjp(bd_ctx* c, const double* x, const double* fbar, double* lamOut, d
                                                                                                    lamOut, th);
   k_adj_dnadna<R><<<cdiv((long)n * n, 128), 128, 0, st>>>(M, x, fbar, lamOut, th);
   if (M.n_dna > 0) k_adj_dnacore<R><<<M.n_dna * M.n_c, 128, 0, st>>>(M, x, fbar, lamOut, th);
-  k_adj_corecore<R><<<dim3(M.n_c * M.n_c, cdiv(M.Nq, kCcThreads)), kCcThreads, 13 * M.Nq * sizeof(R), st>>>(
-      M, x, fbar, lamOut, th);
+  if (M.n_c > 1)
+    k_adj_corecore<R><<<dim3(M.n_c * M.n_c, cdiv(M.Nq, kCcThreads), kCcSplit), kCcThreads,
+                        13 * cdiv(M.Nq, kCcSplit) * sizeof(R), st>>>(M, x, fbar, lamOut, th);
   L += 4;
   if (nt > 0) {
     k_adj_tail_bonded<double, R><<<cdiv(nt, 128), 128, 0, st>>>(M, x, fbar, lamOut);
