@@ -147,6 +147,14 @@ static int step_phases(bd_ctx* c, const double* d_rr, const double* d_p, double*
   const bool krylov = c->noise_mode == BD_NOISE_KRYLOV;
   // a Krylov step needs D itself: rebuilt when A holds a factor
   bool rebuild = (c->step_count % c->freq_rp) == 0 || (krylov && c->a_holds_factor) || c->need_rebuild;
+  // A whole step's first force pass needs the positions alone: it runs on a side
+  // stream beside the tensor, its factor and the noise displacement, which leave
+  // most SMs idle at small sizes.  Not when phases are timed, nor in a batch,
+  // whose replicas already fill the GPU beside each other.
+  const bool overlap = phases == (kPre | kChol | kPost) && !c->timing && !c->in_batch;
+  const bdk::Side* side = overlap ? &c->side : nullptr;
+  if (overlap) CK(cudaEventRecord(c->side.e[0], st));
+  auto join = [&]() { return !overlap || cudaStreamWaitEvent(st, c->side.e[1], 0) == cudaSuccess; };
   if (phases & kPre) {
     record(c, 0);
     bdk::gather_rall(M, c->X, c->r_all, mixed ? &c->S : nullptr, st);
@@ -160,6 +168,11 @@ static int step_phases(bd_ctx* c, const double* d_rr, const double* d_p, double*
       c->need_rebuild = false;
     }
     record(c, 1);
+  }
+  if (overlap) {
+    CK(cudaStreamWaitEvent(c->side.s[0], c->side.e[0], 0));
+    L += bdk::forces(M, c->X, c->F0, c->S, c->precision, c->side.s[0]);
+    CK(cudaEventRecord(c->side.e[1], c->side.s[0]));
   }
   if ((phases & kChol) && rebuild && !krylov) {
     c->a_holds_factor = true;
@@ -183,14 +196,18 @@ static int step_phases(bd_ctx* c, const double* d_rr, const double* d_p, double*
     rc = bdk::krylov_sqrt(c->m, mixed ? nullptr : c->A, c->lda, mixed, c->S.qh, c->S.ql, M.a1, M.a2, d_p, M.s2dt,
                           c->krylov_tol, c->krylov_kmax, c->rd, c->kscratch, st, &c->krylov_iters, &c->krylov_change,
                           &c->kgraphs);
-    if (rc) return set_error(rc, "bd_step: Krylov noise displacement failed");
+    if (rc) {
+      join();
+      return set_error(rc, "bd_step: Krylov noise displacement failed");
+    }
     L += 10 * c->krylov_iters + 4;
   } else {
     bdk::trmv_lower_ws(c->m, c->A, c->lda, d_p, M.s2dt, c->rd, c->rd_part, st, mixed);
     L += 2;
   }
   record(c, 3);
-  L += bdk::forces(M, c->X, c->F0, c->S, c->precision, st);
+  if (!overlap) L += bdk::forces(M, c->X, c->F0, c->S, c->precision, st);
+  else if (!join()) return set_error(BD_ERR_CUDA, "bd_step: joining the force pass");
   record(c, 4);
   bdk::rotate_translate(M, c->X, c->Y, c->F0, d_rr, c->rd, c->r_all, c->precision, c->S, st);
   L += mixed ? 3 : 2;
@@ -200,7 +217,7 @@ static int step_phases(bd_ctx* c, const double* d_rr, const double* d_p, double*
   L += 2;
   if (saves && (rc = pack_ns(c, c->Y, saves[1]))) return rc;
   record(c, 6);
-  L += bdk::forces(M, c->Y, c->F1, c->S, c->precision, st);
+  L += bdk::forces(M, c->Y, c->F1, c->S, c->precision, st, side);
   record(c, 7);
   bdk::average_forces(M, c->F0, c->F1, c->Fa, st);
   bdk::rotate_translate(M, c->X, c->Y, c->Fa, d_rr, c->rd, c->r_all, c->precision, c->S, st);
@@ -301,6 +318,12 @@ extern "C" int bd_create(const bd_model* m, const bd_state* s, const bd_options*
     }
     c->own_stream = true;
   }
+  for (auto& s : c->side.s)
+    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess)
+      return fail(set_error(BD_ERR_CUDA, "bd_create: stream creation failed"));
+  for (auto& ev : c->side.e)
+    if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess)
+      return fail(set_error(BD_ERR_CUDA, "bd_create: event creation failed"));
   DevModel& M = c->M;
   M.n = m->n; M.n_c = m->n_c; M.Nq = m->Nq; M.n_t = m->n_t; M.n_tail = m->n_tail;
   M.n_lh_n = m->n_lh_n; M.n_lh_g = m->n_lh_g; M.n_lh_c = m->n_lh_c; M.n_LH = m->n_LH;
@@ -559,6 +582,10 @@ extern "C" int bd_destroy(bd_ctx* c) {
   c->kgraphs.clear();
   if (c->kscratch) cudaFree(c->kscratch);
   if (c->arena_base) cudaFree(c->arena_base);
+  for (auto ev : c->side.e)
+    if (ev) cudaEventDestroy(ev);
+  for (auto s : c->side.s)
+    if (s) cudaStreamDestroy(s);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return BD_OK;
@@ -652,7 +679,7 @@ extern "C" int bd_step_reference(bd_ctx* c, int step, int number_of_steps, int f
 
 extern "C" int bd_forces(bd_ctx* c, double* F, double* T, double* tF, double* lF, double* E) {
   if (!c) return set_error(BD_ERR_ARG, "bd_forces: null context");
-  bdk::forces(c->M, c->X, c->F0, c->S, c->precision, c->stream);
+  bdk::forces(c->M, c->X, c->F0, c->S, c->precision, c->stream, &c->side);
   CK(cudaGetLastError());
   cudaStream_t st = c->stream;
   size_t n3 = 3 * (size_t)c->M.n;

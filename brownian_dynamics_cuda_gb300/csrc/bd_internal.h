@@ -138,7 +138,15 @@ void average_forces(const DevModel& M, const DevForces& A, const DevForces& B, D
 void gather_rall(const DevModel& M, const DevState& X, double* r_all, const DevScratch* S, cudaStream_t st);
 // forces.cu
 // returns the number of kernels launched
-int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& scr, int mixed, cudaStream_t st);
+// Streams beside a context's own and the events that fork to and join from them
+struct Side {
+  cudaStream_t s[2] = {};
+  cudaEvent_t e[7] = {};
+};
+// side: the pass's independent parts go beside each other, forked from and
+// joined to st
+int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& scr, int mixed, cudaStream_t st,
+           const Side* side = nullptr);
 // rpy_chol.cu
 // qh, ql (mixed path): the positions as double-float pairs (gather_rall's
 // mirror); FP32 RPY blocks stored as double-float pairs (value, 0)
@@ -259,6 +267,7 @@ struct bd_ctx {
   int m_cap = 0;       // largest m the buffers hold: every core with a linker histone
   double *r_all = nullptr, *rd = nullptr, *p = nullptr, *rr = nullptr, *rd_part = nullptr, *energy = nullptr;
   int* negpiv = nullptr;
+  bdk::Side side;  // a step's forces beside its factorisation, and a force pass's parts beside each other
   cudaGraphExec_t graph = nullptr;
   int last_launches = 0;
   int host_negpiv = 0;

@@ -668,21 +668,22 @@ __global__ void k_dna_core(DevModel M, DevState X, DevScratch S, double* slots) 
 }
 
 // Globular head of LH core I against the charges of core L != I
-// (func.cpp:2524-2586): one warp per (I, L).  Slot: force on I (3), torque
+// (func.cpp:2524-2586): one CTA per (I, L).  Slot: force on I (3), torque
 // on I (3), torque on L (3), energy.  Pairs beyond the 7 nm cut-off add
 // exact zeros, so far object pairs are skipped.
+constexpr int kGheadThreads = 256;
+
 template <bool MX>
-__global__ void k_ghead_core(DevModel M, DevState X, double* slots) {
-  int lane = threadIdx.x & 31;
-  int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (w >= M.n_lhcore * M.n_c) return;
-  int I = w / M.n_c, L = w - I * M.n_c;
-  double* out = slots + (size_t)w * 10;
+__global__ void __launch_bounds__(kGheadThreads) k_ghead_core(DevModel M, DevState X, double* slots) {
+  __shared__ double red[32 * 10];
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int I = blockIdx.x / M.n_c, L = blockIdx.x - I * M.n_c;
+  double* out = slots + (size_t)blockIdx.x * 10;
   int i = M.lh_core_bead[I], l = M.core_bead[L];
   V3 ri = ld3(X.r + 3 * i), rl = ld3(X.r + 3 * l);
   double d0 = dist3(ri, rl);
   if (i == l || d0 > 7.0 + M.gmax + M.qmax_core + 1e-6) {
-    if (lane < 10) out[lane] = 0.0;
+    if (threadIdx.x < 10) out[threadIdx.x] = 0.0;
     return;
   }
   V3 ai = ld3(X.a + 3 * i), bi = ld3(X.b + 3 * i), ci = ld3(X.c + 3 * i);
@@ -690,15 +691,17 @@ __global__ void k_ghead_core(DevModel M, DevState X, double* slots) {
   const double eps = eps_of(M);
   double v[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   const int ng = M.n_lh_g, Nq = M.Nq;
-  // lane: charges m of core L, each against every site jm of the head.  The
+  // Warp w: a quarter (w % 4) of core L's charges m against every second site jm of
+  // the head; one warp for all of a pair held 12 SMs of a four-core pass for 108 us.  The
   // torques are linear in sum f (x) gp_jm and in sum f (x) cp_m (as in
   // k_core_core), so no pair forms one in FP64; with two torques and the
-  // charge's position a pair it was 183 us for four cores, now 108.
+  // charge's position a pair it was 183 us for four cores; by one
+  // warp without 108.
   double MI[3][3] = {{0}}, ML[3][3] = {{0}};
-  for (int m = lane; m < Nq; m += 32) {
+  for (int m = lane + 32 * (wp & 3); m < Nq; m += 128) {
     const V3 z = body(rl, al, bl, cl, M.core_pos + 3 * m);
     double fm[3] = {0, 0, 0};
-    for (int jm = 0; jm < ng; jm++) {
+    for (int jm = wp >> 2; jm < ng; jm += 2) {
       const V3 g = ld3(X.gpos + 3 * (I * ng + jm));
       const V3 f1 = pairF<true, true, MX>(M.LH_q[jm], M.core_q[m], eps, M.debye, M.k_ex, M.LH_vdw_hc[jm], g, z, &v[9]);
       fm[0] = fm[0] + f1.x, fm[1] = fm[1] + f1.y, fm[2] = fm[2] + f1.z;
@@ -720,8 +723,8 @@ __global__ void k_ghead_core(DevModel M, DevState X, double* slots) {
   v[5] = dotm(bi, MI, 0) - dotm(ai, MI, 1);
   v[6] = dotm(bl, ML, 2) - dotm(cl, ML, 1), v[7] = dotm(cl, ML, 0) - dotm(al, ML, 2),
   v[8] = dotm(al, ML, 1) - dotm(bl, ML, 0);  // (the force on L is -f)
-  for (int q = 0; q < 10; q++) v[q] = wsum(v[q]);
-  if (lane == 0)
+  bsum<10>(v, red);
+  if (threadIdx.x == 0)
     for (int q = 0; q < 10; q++) out[q] = v[q];
 }
 
@@ -1658,7 +1661,20 @@ __global__ void k_energy(int n0, const double* e0, double* E) {
 
 namespace bdk {
 
-int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& S, int mixed, cudaStream_t st) {
+// With side streams the independent parts of a pass run beside each other (all
+// of them are a few CTAs or bound by one bead's serial chain, 15-40 us each on
+// a few SMs): bonded terms, G-heads and the linker beads' sums on s0; tails and
+// linker histones on s1.  4 nucleosomes with linker histones, mixed, bd_forces:
+// 0.39 ms in a row, 0.22 so (with k_ghead_core's split).
+int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& S, int mixed, cudaStream_t st,
+           const Side* side) {
+  cudaStream_t s0 = side ? side->s[0] : st, s1 = side ? side->s[1] : st;
+  auto rec = [&](int e, cudaStream_t a) {
+    if (side) cudaEventRecord(side->e[e], a);
+  };
+  auto wait = [&](cudaStream_t b, int e) {
+    if (side) cudaStreamWaitEvent(b, side->e[e], 0);
+  };
   // energy layout in S.ebuf: [0,n) chain, [n, n+n_tail) tails, then LH
   double* Ech = S.ebuf;
   double* Et = S.ebuf + M.n;
@@ -1674,12 +1690,28 @@ int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& S, int mi
   if (M.n_lhcore > 0) { k_gpos<<<cdiv(M.n_lhcore * M.n_lh_g, 128), 128, 0, st>>>(M, X); L++; }
   k_mirror<<<cdiv(S.npos, 128), 128, 0, st>>>(M, X, S.ph, S.pl, S.npos);
   L++;
+  rec(2, st);
+  wait(s0, 2);
+  wait(s1, 2);
   if (M.n > 1) {
-    k_chain_bonds<<<cdiv(M.n - 1, kBeadThreads), kBeadThreads, 0, st>>>(M, X, S.bonds);
+    k_chain_bonds<<<cdiv(M.n - 1, kBeadThreads), kBeadThreads, 0, s0>>>(M, X, S.bonds);
     L++;
   }
-  k_chain_bonded<<<cdiv(M.n, kBeadThreads), kBeadThreads, 0, st>>>(M, X, S.bonds, Fm, Tm, Ebond);
+  k_chain_bonded<<<cdiv(M.n, kBeadThreads), kBeadThreads, 0, s0>>>(M, X, S.bonds, Fm, Tm, Ebond);
   L++;
+  if (M.n_lhcore > 0) { k_ghead_coreX<<<M.n_lhcore * M.n_c, kGheadThreads, 0, s0>>>(M, X, S.gc); L++; }
+  rec(3, s0);
+  if (mixed) {
+    if (M.n_tail > 0) { k_tail_bonded_mx<<<cdiv(M.n_tail, kBeadThreads), kBeadThreads, 0, s1>>>(M, X, S); L++; }
+    if (M.n_LH > 0) { k_lh_bonded_mx<<<cdiv(M.n_LH, kBeadThreads), kBeadThreads, 0, s1>>>(M, X, S); L++; }
+    if (M.n_tail > 0) { k_tail_gather_mx<<<cdiv(M.n_tail * 32, 256), 256, 0, s1>>>(M, X, S, out, Et); L++; }
+    if (M.n_LH > 0) { k_lh_gather_mx<<<cdiv(M.n_LH * 32, 256), 256, 0, s1>>>(M, X, S, out, El); L++; }
+  } else {
+    if (M.n_tail > 0) { k_tail_gather<<<cdiv(M.n_tail * 32, 256), 256, 0, s1>>>(M, X, S, out, Et); L++; }
+    if (M.n_LH > 0) { k_lh_gather<<<cdiv(M.n_LH * 32, 256), 256, 0, s1>>>(M, X, S, out, El); L++; }
+  }
+  if (M.n_dna > 0 && M.n_c > 0) { k_dna_coreX<<<cdiv(M.n_dna * M.n_c * 32, 256), 256, 0, st>>>(M, X, S, S.dc); L++; }
+  rec(4, st);
   if (M.n_c > 1) {
     if (mixed) {
       size_t sm = (size_t)((14 * M.Nq + 1) / 2 + 32 * 10) * sizeof(double);
@@ -1691,21 +1723,19 @@ int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& S, int mi
     k_cc_sum<<<cdiv(M.n_c * M.n_c * 10, 256), 256, 0, st>>>(M.n_c, mixed ? kCCSplit : kCC64Split, S.ccp, S.cc);
     L += 2;
   }
-  if (M.n_dna > 0 && M.n_c > 0) { k_dna_coreX<<<cdiv(M.n_dna * M.n_c * 32, 256), 256, 0, st>>>(M, X, S, S.dc); L++; }
-  if (M.n_lhcore > 0) { k_ghead_coreX<<<cdiv(M.n_lhcore * M.n_c * 32, 256), 256, 0, st>>>(M, X, S.gc); L++; }
+  wait(st, 3);
   if (mixed) {
-    if (M.n_tail > 0) { k_tail_bonded_mx<<<cdiv(M.n_tail, kBeadThreads), kBeadThreads, 0, st>>>(M, X, S); L++; }
-    if (M.n_LH > 0) { k_lh_bonded_mx<<<cdiv(M.n_LH, kBeadThreads), kBeadThreads, 0, st>>>(M, X, S); L++; }
-    if (M.n_tail > 0) { k_tail_gather_mx<<<cdiv(M.n_tail * 32, 256), 256, 0, st>>>(M, X, S, out, Et); L++; }
-    if (M.n_LH > 0) { k_lh_gather_mx<<<cdiv(M.n_LH * 32, 256), 256, 0, st>>>(M, X, S, out, El); L++; }
-    if (M.n_dna > 0) k_chain_gather_mx<<<M.n_dna, kGatherThreads, 0, st>>>(M, X, Fm, Tm, Ebond, S, out, Ech, M.dna_bead);
+    wait(s0, 4);
+    if (M.n_dna > 0) k_chain_gather_mx<<<M.n_dna, kGatherThreads, 0, s0>>>(M, X, Fm, Tm, Ebond, S, out, Ech, M.dna_bead);
     if (M.n_c > 0) k_chain_gather_mx<<<M.n_c, kGatherCoreThreads, 0, st>>>(M, X, Fm, Tm, Ebond, S, out, Ech, M.core_bead);
     L += (M.n_dna > 0) + (M.n_c > 0) - 1;  // one chain launch is counted below
   } else {
-    if (M.n_tail > 0) { k_tail_gather<<<cdiv(M.n_tail * 32, 256), 256, 0, st>>>(M, X, S, out, Et); L++; }
-    if (M.n_LH > 0) { k_lh_gather<<<cdiv(M.n_LH * 32, 256), 256, 0, st>>>(M, X, S, out, El); L++; }
     k_chain_gather<<<M.n, kGatherThreads, 0, st>>>(M, X, Fm, Tm, Ebond, S, out, Ech);
   }
+  rec(5, s0);
+  rec(6, s1);
+  wait(st, 5);
+  wait(st, 6);
   k_energy<<<1, 256, 0, st>>>(M.n + M.n_tail + M.n_LH, S.ebuf, out.E);
   return L + 2;
 }
