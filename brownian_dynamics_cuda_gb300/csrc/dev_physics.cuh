@@ -204,55 +204,30 @@ __device__ __forceinline__ V3 torque_rel(const V3& F, const double* comp, const 
 __device__ __forceinline__ void acc(V3& s, const V3& v) { s.x = s.x + v.x; s.y = s.y + v.y; s.z = s.z + v.z; }
 __device__ __forceinline__ void dec(V3& s, const V3& v) { s.x = s.x - v.x; s.y = s.y - v.y; s.z = s.z - v.z; }
 
-// RPY tensor element (row 3i+k, column 3j+l) for a bead pair i != j, with
-// sij = r_i - r_j (either sign).  func.cpp:753-799 writes each off-diagonal
-// element twice, leaving the value computed with the larger component
-// index first; this returns that value.
-__device__ __forceinline__ double rpy_elem(const V3& sij, double ssq, double s, double radi, double radj, double a1,
-                                           double a2, int k, int l) {
-  int kk = k > l ? k : l, ll = k > l ? l : k;
-  double sk = c3(sij, kk), sl = c3(sij, ll);
-  if (s >= radi + radj) {
-    double f = (radi * radi + radj * radj) / ssq;
-    double f1 = 1.0 + f / 3, f2 = 1.0 - f;
-    if (k == l) return (a2 / s) * (f1 + f2 * sk * sk / ssq);
-    return (a2 / s) * (f2 * sk * sl / ssq);
-  }
-  double se = pow((radi * radi * radi + radj * radj * radj) / 2.0, 1.0 / 3);
-  if (k == l) return (a1 / se) * (1.0 - 9.0 * sqrt(ssq) / (32 * se) + 3.0 * sk * sk / (32.0 * se * sqrt(ssq)));
-  return (a1 / se) * (3.0 * sk * sl / (32.0 * se * sqrt(ssq)));
-}
-
-// The full 3 x 3 block (same per-element expressions as rpy_elem, shared
-// subexpressions evaluated once): out[k][l].
+// RPY tensor block (rows 3i+k, columns 3j+l) for a bead pair i != j, with
+// sij = r_i - r_j (either sign; func.cpp:753-799).  out[k][l]: one root and one
+// division (nine divisions with each element formed as the reference does: 170
+// FP64 operations a pair, 60 here; the FP64 pipe bounds tensor and drift).  3N =
+// 1,944: tensor 139 -> 41 us, drift 216 -> 54.
 __device__ __forceinline__ void rpy_block(const V3& sij, double ssq, double s, double radi, double radj, double a1,
                                           double a2, double (&out)[3][3]) {
-  const double sv[3] = {sij.x, sij.y, sij.z};
+  const double sv[3] = {sij.x, sij.y, sij.z}, mi = 1.0 / s;
+  double dg, c;  // out = dg I + c s s^T
   if (s >= radi + radj) {
-    double f = (radi * radi + radj * radj) / ssq;
-    double f1 = 1.0 + f / 3, f2 = 1.0 - f;
-    double as = a2 / s;
-#pragma unroll
-    for (int k = 0; k < 3; k++) out[k][k] = as * (f1 + f2 * sv[k] * sv[k] / ssq);
-    double o10 = as * (f2 * sv[1] * sv[0] / ssq);
-    double o20 = as * (f2 * sv[2] * sv[0] / ssq);
-    double o21 = as * (f2 * sv[2] * sv[1] / ssq);
-    out[1][0] = out[0][1] = o10;
-    out[2][0] = out[0][2] = o20;
-    out[2][1] = out[1][2] = o21;
-    return;
+    const double m2 = mi * mi, f = (radi * radi + radj * radj) * m2, as = a2 * mi;
+    dg = as * fma(f, 1.0 / 3, 1.0);
+    c = as * (1.0 - f) * m2;
+  } else {
+    const double ise = 1.0 / cbrt((radi * radi * radi + radj * radj * radj) * 0.5), as = a1 * ise;
+    dg = as * fma(-9.0 / 32 * s, ise, 1.0);
+    c = as * (3.0 / 32) * ise * mi;
   }
-  double se = pow((radi * radi * radi + radj * radj * radj) / 2.0, 1.0 / 3);
-  double as = a1 / se;
-  double rs = sqrt(ssq);
 #pragma unroll
-  for (int k = 0; k < 3; k++) out[k][k] = as * (1.0 - 9.0 * rs / (32 * se) + 3.0 * sv[k] * sv[k] / (32.0 * se * rs));
-  double o10 = as * (3.0 * sv[1] * sv[0] / (32.0 * se * rs));
-  double o20 = as * (3.0 * sv[2] * sv[0] / (32.0 * se * rs));
-  double o21 = as * (3.0 * sv[2] * sv[1] / (32.0 * se * rs));
-  out[1][0] = out[0][1] = o10;
-  out[2][0] = out[0][2] = o20;
-  out[2][1] = out[1][2] = o21;
+  for (int k = 0; k < 3; k++) {
+    const double ck = c * sv[k];
+#pragma unroll
+    for (int l = 0; l <= k; l++) out[k][l] = out[l][k] = k == l ? fma(ck, sv[l], dg) : ck * sv[l];
+  }
 }
 
 // FP32 form of rpy_block for the mixed path (drift and tensor; separation

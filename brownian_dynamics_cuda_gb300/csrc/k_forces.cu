@@ -696,7 +696,7 @@ __global__ void __launch_bounds__(kGheadThreads) k_ghead_core(DevModel M, DevSta
   // torques are linear in sum f (x) gp_jm and in sum f (x) cp_m (as in
   // k_core_core), so no pair forms one in FP64; with two torques and the
   // charge's position a pair it was 183 us for four cores; by one
-  // warp without 108.
+  // warp without 108, by eight 43.
   double MI[3][3] = {{0}}, ML[3][3] = {{0}};
   for (int m = lane + 32 * (wp & 3); m < Nq; m += 128) {
     const V3 z = body(rl, al, bl, cl, M.core_pos + 3 * m);

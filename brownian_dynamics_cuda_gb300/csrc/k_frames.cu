@@ -229,7 +229,8 @@ __global__ void k_rotate(DevModel M, const double* __restrict__ T, const double*
   }
 }
 
-// Drift + noise for one bead (a warp per bead): x_new = x + rd + del * D_ss F_s,
+// Drift + noise for one bead (a warp per bead, each its own CTA: the rows even
+// out over the FP64 pipes, which bound it): x_new = x + rd + del * D_ss F_s,
 // D_ss the RPY block of the bead's own species (chain, tails or LH).
 // The lanes split the partner loop; partial sums are combined in a fixed
 // butterfly order so the result is deterministic.
@@ -238,8 +239,7 @@ __global__ void k_translate(DevModel M, const double* __restrict__ r_all, const 
                             const double* __restrict__ r0, const double* __restrict__ rt0,
                             const double* __restrict__ rl0, double* r1, double* rt1, double* rl1) {
   int lane = threadIdx.x & 31;
-  int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (i >= M.n_D) return;
+  int i = blockIdx.x;
   int lo, hi;
   const double* F;
   if (i < M.n) { lo = 0; hi = M.n; F = Fc; }
@@ -252,9 +252,9 @@ __global__ void k_translate(DevModel M, const double* __restrict__ r_all, const 
     const double* f = F + 3 * (j - lo);
     if (j == i) {
       double d = M.a1 / radi;
-      s0 = s0 + M.del * d * f[0];
-      s1 = s1 + M.del * d * f[1];
-      s2 = s2 + M.del * d * f[2];
+      s0 = fma(d, f[0], s0);
+      s1 = fma(d, f[1], s1);
+      s2 = fma(d, f[2], s2);
       continue;
     }
     V3 rj = ld3(r_all + 3 * j);
@@ -264,13 +264,14 @@ __global__ void k_translate(DevModel M, const double* __restrict__ r_all, const 
     double radj = M.rad_all[j];
     double Db[3][3];
     rpy_block(sij, ssq, s, radi, radj, M.a1, M.a2, Db);
+#pragma unroll
     for (int l = 0; l < 3; l++) {
-      double fl = f[l];
-      s0 = s0 + M.del * Db[0][l] * fl;
-      s1 = s1 + M.del * Db[1][l] * fl;
-      s2 = s2 + M.del * Db[2][l] * fl;
+      const double fl = f[l];
+      s0 = fma(Db[0][l], fl, s0);
+      s1 = fma(Db[1][l], fl, s1);
+      s2 = fma(Db[2][l], fl, s2);
     }
-    }
+  }
   for (int o = 16; o > 0; o >>= 1) {
     s0 = s0 + __shfl_xor_sync(0xffffffffu, s0, o);
     s1 = s1 + __shfl_xor_sync(0xffffffffu, s1, o);
@@ -283,9 +284,9 @@ __global__ void k_translate(DevModel M, const double* __restrict__ r_all, const 
     if (i < M.n) { out = r1; x0 = r0; li = i; }
     else if (i < M.n + M.n_tail) { out = rt1; x0 = rt0; li = i - M.n; }
     else { out = rl1; x0 = rl0; li = i - M.n - M.n_tail; }
-    out[3 * li] = x0[3 * li] + rd[3 * i] + s0;
-    out[3 * li + 1] = x0[3 * li + 1] + rd[3 * i + 1] + s1;
-    out[3 * li + 2] = x0[3 * li + 2] + rd[3 * i + 2] + s2;
+    out[3 * li] = x0[3 * li] + rd[3 * i] + M.del * s0;
+    out[3 * li + 1] = x0[3 * li + 1] + rd[3 * i + 1] + M.del * s1;
+    out[3 * li + 2] = x0[3 * li + 2] + rd[3 * i + 2] + M.del * s2;
   }
 }
 
@@ -455,7 +456,7 @@ void rotate_translate(const DevModel& M, const DevState& X, DevState& Y, const D
     k_translate_mx<<<cdiv(M.n_D * 32, 256), 256, 0, st>>>(M, S.qh, S.ql, S.qf, rd, X.r, X.r_t, X.r_lh, Y.r, Y.r_t,
                                                            Y.r_lh);
   } else {
-    k_translate<<<cdiv(M.n_D * 32, 256), 256, 0, st>>>(M, r_all, Fo.F, Fo.tF, Fo.lF, rd, X.r, X.r_t, X.r_lh, Y.r,
+    k_translate<<<M.n_D, 32, 0, st>>>(M, r_all, Fo.F, Fo.tF, Fo.lF, rd, X.r, X.r_t, X.r_lh, Y.r,
                                                         Y.r_t, Y.r_lh);
   }
 }

@@ -13,6 +13,8 @@
 //                  over column chunks with a fixed-order final sum.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "bd_internal.h"
 #include "dev_physics.cuh"
 
@@ -22,13 +24,22 @@ namespace {
 
 inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 
+// tile (bi, bj <= bi) of a triangle from its row-major index t (a grid without
+// the triangle's empty half: the SMs' shares of the tiles are then even)
+__device__ __forceinline__ void tri_tile(int t, int& bi, int& bj) {
+  bi = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
+  while ((bi + 1) * (bi + 2) / 2 <= t) bi++;
+  while (bi * (bi + 1) / 2 > t) bi--;
+  bj = t - bi * (bi + 1) / 2;
+}
+
 // ------------------------------------------------------------ RPY
 constexpr int kRpyTile = 32;
 
 __global__ void __launch_bounds__(256) k_rpy(int nD, const double* __restrict__ r, const double* __restrict__ rad,
                                              double a1, double a2, double* __restrict__ A, int lda) {
-  int bi = blockIdx.y, bj = blockIdx.x;
-  if (bj > bi) return;
+  int bi, bj;
+  tri_tile(blockIdx.x, bi, bj);
   int i = bi * kRpyTile + threadIdx.x;
   if (i >= nD) return;
   V3 ri = ld3(r + 3 * i);
@@ -190,15 +201,6 @@ __global__ void __launch_bounds__(128) k_trsm_panel(double* A, int lda, int m, i
 // bounds it.
 constexpr int kKC = 16;  // panel columns staged per pass
 
-// tile (bi, bj <= bi) of a triangle from its row-major index t (a grid without
-// the triangle's empty half: the SMs' shares of the tiles are then even)
-__device__ __forceinline__ void tri_tile(int t, int& bi, int& bj) {
-  bi = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
-  while ((bi + 1) * (bi + 2) / 2 <= t) bi++;
-  while (bi * (bi + 1) / 2 > t) bi--;
-  bj = t - bi * (bi + 1) / 2;
-}
-
 template <int TM, int TN, int MR, int NR>
 __global__ void __launch_bounds__(TM * TN / (MR * NR)) k_syrk_update(double* A, int lda, int m, int k0, int kb, int t0, int jend) {
   constexpr int NT = TM * TN / (MR * NR);
@@ -256,14 +258,18 @@ __global__ void __launch_bounds__(TM * TN / (MR * NR)) k_syrk_update(double* A, 
 
 // ------------------------------------------------------------ L p
 constexpr int kRdRows = 256;
-constexpr int kRdChunk = 512;
+// Columns a CTA sums: short runs at small sizes, where 512 left a few CTAs of one
+// serial chain each (3N = 912: 8 CTAs, 80 us; 32 columns: 11), long ones where
+// the rows alone fill the GPU and the partial sums would cost a second pass.
+constexpr int kRdChunkMax = 512;
+int rd_chunk(int m) { return m <= 2048 ? 32 : m <= 8192 ? 128 : kRdChunkMax; }
 
 __global__ void __launch_bounds__(kRdRows) k_trmv_part(int m, const double* __restrict__ A, int lda,
-                                                       const double* __restrict__ p, double s2dt,
+                                                       const double* __restrict__ p, double s2dt, int chunk,
                                                        double* __restrict__ part) {
   int i = blockIdx.x * kRdRows + threadIdx.x;
   int kc = blockIdx.y;
-  int k0 = kc * kRdChunk, k1 = min(k0 + kRdChunk, m);
+  int k0 = kc * chunk, k1 = min(k0 + chunk, m);
   double s = 0.0;
   if (i < m) {
     int kend = min(k1, i + 1);
@@ -278,12 +284,12 @@ __global__ void __launch_bounds__(kRdRows) k_trmv_part(int m, const double* __re
 // FP32 hi + lo once per CTA, FMA for the rounding error of L_ik p_hi) and
 // summed with a two-sum into (s, c); ~40 significant bits per partial sum.
 __global__ void __launch_bounds__(kRdRows) k_trmv_part_df(int m, const float2* __restrict__ A, int lda,
-                                                          const double* __restrict__ p, double s2dt,
+                                                          const double* __restrict__ p, double s2dt, int chunk,
                                                           double* __restrict__ part) {
-  __shared__ float2 ps[kRdChunk];
+  __shared__ float2 ps[kRdChunkMax];
   int i = blockIdx.x * kRdRows + threadIdx.x;
   int kc = blockIdx.y;
-  int k0 = kc * kRdChunk, k1 = min(k0 + kRdChunk, m);
+  int k0 = kc * chunk, k1 = min(k0 + chunk, m);
   for (int k = k0 + threadIdx.x; k < k1; k += kRdRows) {
     const double pk = p[k];
     const float h = (float)pk;
@@ -328,7 +334,7 @@ void rpy_assemble(int nD, const double* r_all, const double* rad, double a1, dou
     k_rpy_mx<<<dim3(nt, nt), dim3(kRpyTile, 8), 0, st>>>(nD, qh, ql, (float)a1, (float)a2,
                                                          reinterpret_cast<float2*>(A), lda);
   else
-    k_rpy<<<dim3(nt, nt), dim3(kRpyTile, 8), 0, st>>>(nD, r_all, rad, a1, a2, A, lda);
+    k_rpy<<<nt * (nt + 1) / 2, dim3(kRpyTile, 8), 0, st>>>(nD, r_all, rad, a1, a2, A, lda);
 }
 
 // Blocks of 2 kNB columns: panel, the second panel's columns updated by the
@@ -367,16 +373,20 @@ int potrf_fp64(int m, double* A, int lda, double* /*rd_acc*/, const double* /*p*
   return launches;
 }
 
-size_t trmv_scratch_doubles(int m) { return (size_t)cdiv(m, kRdChunk) * m; }
+// (for every size up to m: a smaller matrix can have more partial sums)
+size_t trmv_scratch_doubles(int m) {
+  auto need = [](int k) { return (size_t)cdiv(k, rd_chunk(k)) * k; };
+  return std::max({need(m), need(std::min(m, 2048)), need(std::min(m, 8192))});
+}
 
 void trmv_lower_ws(int m, const double* A, int lda, const double* p, double s2dt, double* rd, double* part,
                    cudaStream_t st, bool df) {
-  int nchunk = cdiv(m, kRdChunk);
+  const int chunk = rd_chunk(m), nchunk = cdiv(m, chunk);
   if (df)
     k_trmv_part_df<<<dim3(cdiv(m, kRdRows), nchunk), kRdRows, 0, st>>>(m, reinterpret_cast<const float2*>(A), lda, p,
-                                                                       s2dt, part);
+                                                                       s2dt, chunk, part);
   else
-    k_trmv_part<<<dim3(cdiv(m, kRdRows), nchunk), kRdRows, 0, st>>>(m, A, lda, p, s2dt, part);
+    k_trmv_part<<<dim3(cdiv(m, kRdRows), nchunk), kRdRows, 0, st>>>(m, A, lda, p, s2dt, chunk, part);
   k_trmv_sum<<<cdiv(m, 256), 256, 0, st>>>(m, nchunk, part, rd);
 }
 
