@@ -105,24 +105,32 @@ __global__ void __launch_bounds__(256) k_rpy_mx(int nD, const float4* __restrict
 // of 64 columns on a few SMs the serial part of a small factorisation.
 constexpr int kNB = 32;
 
-// 1 / sqrt(f), f > 0: from FP32's by one third-order step (22 bits to 2 ulp in
-// five FP64 operations instead of a root and a division)
-__device__ __forceinline__ double rsqrt_nr(double f) {
-  const unsigned e = (unsigned)__double2hiint(f) >> 20;  // sign and exponent
-  if (e < 1023 - 100 || e > 1023 + 100) return 1.0 / sqrt(f);
-  const double y = (double)rsqrtf((float)f);
-  const double d = fma(-f * y, y, 1.0);
-  return fma(y * d, fma(0.375, d, 0.5), y);
+// A pivot's step: f > 0 and a column entry to a / sqrt(f), from FP32's reciprocal
+// root y by one third-order step, e = 1 - f y^2: a y (1 + e / 2 + 3 e^2 / 8) (22
+// bits to 2 ulp in six FP64 operations, four of them in a row, instead of a root
+// and a division; the seed goes to FP32 and back as bits, off the FP64 pipe).
+__device__ __forceinline__ double over_sqrt(double a, double f) {
+  const int hi = __double2hiint(f);
+  const unsigned e = (unsigned)hi >> 20;  // sign and exponent
+  if (e < 1023 - 100 || e > 1023 + 100) return a * (1.0 / sqrt(f));
+  constexpr int kBias = (1023 - 127) << 20;
+  const int y32 = __float_as_int(
+      rsqrtf(__int_as_float(((hi - kBias) << 3) | ((unsigned)__double2loint(f) >> 29))));
+  const double y = __hiloint2double((y32 >> 3) + kBias, y32 << 29);
+  const double d = fma(-f * y, y, 1.0), ay = a * y;
+  return fma(ay * d, fma(0.375, d, 0.5), ay);
 }
 
 // Factor the kb x kb diagonal block at (k0, k0): right-looking, a row per lane,
 // column j in the registers of warp j % 4 (one warp per FP64 pipe: a warp's
 // FP64 operation holds its pipe for 64 cycles), column c to the others through
-// shared memory.  A negative pivot is replaced by its absolute value and
-// counted (func.cpp:827-833).  Bound by the pivots' chain (ten dependent FP64
-// operations and a barrier each): 64 columns by 256 threads with three
-// barriers a column took 119 us, 32 by one warp 69, by four 25 (3N = 912:
-// 5.1 -> 1.7 ms in all, 1,944: 13.3 -> 5.2, 11,700: 499 -> 458).
+// shared memory.  The warp of column c + 1 takes column c off it alone, scales
+// and publishes it, and makes up for its other columns in the next turn.  A
+// negative pivot is replaced by its absolute value and counted
+// (func.cpp:827-833).  Bound by the pivots' chain (six dependent FP64 operations
+// and a barrier each): 64 columns by 256 threads with three barriers a column
+// took 119 us, 32 by one warp 69, by four 25 without that order, 24 with it (with
+// the rows' split below, 3N = 912: 5.1 -> 1.5 ms in all, 1,944: 13.3 -> 4.8).
 __global__ void __launch_bounds__(128) k_potrf_diag(double* A, int lda, int k0, int kb, int* negpiv) {
   __shared__ double T[kNB][kNB];  // T[c][j] = L_jc (below the diagonal)
   __shared__ double piv[kNB];
@@ -134,22 +142,34 @@ __global__ void __launch_bounds__(128) k_potrf_diag(double* A, int lda, int k0, 
     const int j = 4 * i + w;
     a[i] = (lane < kb && j <= lane) ? col[(size_t)j * lda] : (j == lane ? 1.0 : 0.0);
   }
+  auto pivot = [&](double& ac, int c) {  // column c, updated by all before it
+    double f = __shfl_sync(0xffffffffu, ac, c);
+    if (__double2hiint(f) < 0 && f < 0) {
+      f = -f;
+      if (lane == 0) atomicAdd(negpiv, 1);
+    }
+    T[c][lane] = ac = over_sqrt(ac, f);
+    if (lane == c) piv[c] = f;
+  };
+  if (w == 0) pivot(a[0], 0);
+  __syncthreads();
 #pragma unroll
-  for (int c = 0; c < kNB; c++) {
-    if (w == (c & 3)) {
-      double f = __shfl_sync(0xffffffffu, a[c >> 2], c);
-      if (__double2hiint(f) < 0 && f < 0) {
-        f = -f;
-        if (lane == 0) atomicAdd(negpiv, 1);
+  for (int c = 0; c < kNB - 1; c++) {
+    const double l = T[c][lane];
+    if (w == ((c + 1) & 3)) {
+      a[(c + 1) >> 2] = fma(-l, T[c][c + 1], a[(c + 1) >> 2]);
+      pivot(a[(c + 1) >> 2], c + 1);
+    } else {
+      if (c > 0 && w == (c & 3)) {  // the columns left behind at c - 1
+        const double lp = T[c - 1][lane];
+#pragma unroll
+        for (int i = (c >> 2) + 1; i < kNB / 4; i++) a[i] = fma(-lp, T[c - 1][4 * i + w], a[i]);
       }
-      T[c][lane] = a[c >> 2] *= rsqrt_nr(f);
-      if (lane == c) piv[c] = f;
+#pragma unroll
+      for (int i = c >> 2; i < kNB / 4; i++)
+        if (4 * i + w > c) a[i] = fma(-l, T[c][4 * i + w], a[i]);  // (rows above the diagonal: not used)
     }
     __syncthreads();
-    const double l = T[c][lane];
-#pragma unroll
-    for (int i = c >> 2; i < kNB / 4; i++)  // column c + 1 first, of the warp that takes it off next
-      if (4 * i + w > c) a[i] = fma(-l, T[c][4 * i + w], a[i]);  // (rows above the diagonal: not used)
   }
 #pragma unroll
   for (int i = 0; i < kNB / 4; i++) {
@@ -160,38 +180,47 @@ __global__ void __launch_bounds__(128) k_potrf_diag(double* A, int lda, int k0, 
 }
 
 // Panel solve: rows [k0+kb, m) of columns [k0, k0+kb): X L_kk^T = A,
-// right-looking in registers.  A warp takes 8 rows, lane 8 g + r the columns
-// 4 i + g of row r: four times as many warps as with a row per lane, so that
-// the rows of a small matrix reach all FP64 pipes.  64 columns left-looking
-// with a row per thread: 188 us at 3N = 1,944; 32 columns with a row per lane
-// 24 us; now 16.
+// right-looking in registers, the columns unscaled until the end (row c of L
+// carries 1 / L_cc).  A warp takes 4 rows, lane 4 g + r the columns 8 i + g of
+// row r: eight times as many warps as with a row per lane, so that the rows of
+// a small matrix reach all FP64 pipes.  64 columns left-looking with a row per
+// thread: 188 us at 3N = 1,944; 32 columns with a row per lane 24 us, four
+// lanes a row 16; now 11.5.
+constexpr int kTrsmRows = 16;  // per CTA of four warps
+
 __global__ void __launch_bounds__(128) k_trsm_panel(double* A, int lda, int m, int k0, int kb) {
-  __shared__ double L[kNB][kNB];  // L[c][j] = L_jc, j > c; else 0
+  __shared__ double L[kNB][kNB];  // L[c][j] = L_jc / L_cc, j > c; else 0
   __shared__ double rd[kNB];
-  const int lane = threadIdx.x & 31, g = lane >> 3;
-  const int r = k0 + kb + blockIdx.x * 32 + (threadIdx.x >> 5) * 8 + (lane & 7);
+  const int lane = threadIdx.x & 31, g = lane >> 2;
+  const int r = k0 + kb + blockIdx.x * kTrsmRows + (threadIdx.x >> 5) * 4 + (lane & 3);
   double* col = A + (size_t)k0 * lda + r;
-  double x[kNB / 4];
+  double x[kNB / 8];
 #pragma unroll
-  for (int i = 0; i < kNB / 4; i++) x[i] = (r < m && 4 * i + g < kb) ? col[(size_t)(4 * i + g) * lda] : 0.0;
-  for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
-    const int c = e / kNB, j = e % kNB;
-    const double v = (j < kb && c <= j) ? A[(size_t)(k0 + c) * lda + k0 + j] : 0.0;
-    if (c == j) rd[c] = j < kb ? 1.0 / v : 0.0;
-    L[c][j] = c < j ? v : 0.0;
+  for (int i = 0; i < kNB / 8; i++) x[i] = (r < m && 8 * i + g < kb) ? col[(size_t)(8 * i + g) * lda] : 0.0;
+  double v[kNB / 4];
+#pragma unroll
+  for (int q = 0; q < kNB / 4; q++) {  // warp w: columns w, w + 4, ...; lane: row
+    const int c = (threadIdx.x >> 5) + 4 * q;
+    v[q] = (lane < kb && c <= lane) ? A[(size_t)(k0 + c) * lda + k0 + lane] : 0.0;
+    if (lane == c) rd[c] = lane < kb ? 1.0 / v[q] : 0.0;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < kNB / 4; q++) {
+    const int c = (threadIdx.x >> 5) + 4 * q;
+    L[c][lane] = c < lane ? v[q] * rd[c] : 0.0;
   }
   __syncthreads();
 #pragma unroll
-  for (int c = 0; c < kNB; c++) {
-    const double xc = __shfl_sync(0xffffffffu, x[c >> 2], (lane & 7) + 8 * (c & 3)) * rd[c];
-    if (g == (c & 3)) x[c >> 2] = xc;
+  for (int c = 0; c < kNB - 1; c++) {
+    const double xc = __shfl_sync(0xffffffffu, x[c >> 3], (lane & 3) + 4 * (c & 7));
 #pragma unroll
-    for (int i = c >> 2; i < kNB / 4; i++) x[i] = fma(-xc, L[c][4 * i + g], x[i]);
+    for (int i = c >> 3; i < kNB / 8; i++) x[i] = fma(-xc, L[c][8 * i + g], x[i]);
   }
   if (r < m)
 #pragma unroll
-    for (int i = 0; i < kNB / 4; i++)
-      if (4 * i + g < kb) col[(size_t)(4 * i + g) * lda] = x[i];
+    for (int i = 0; i < kNB / 8; i++)
+      if (8 * i + g < kb) col[(size_t)(8 * i + g) * lda] = x[i] * rd[8 * i + g];
 }
 
 // Update of the lower triangle of A[t0:, t0:jend] by the kb columns from k0:
@@ -319,6 +348,7 @@ __global__ void k_trmv_sum(int m, int nchunk, const double* __restrict__ part, d
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   double s = 0.0;
+#pragma unroll 8
   for (int c = 0; c < nchunk; c++) s = s + part[(size_t)c * m + i];
   rd[i] = s;
 }
@@ -351,7 +381,7 @@ int potrf_fp64(int m, double* A, int lda, double* /*rd_acc*/, const double* /*p*
     launches++;
     const int rest = m - k0 - kb;
     if (rest > 0) {
-      k_trsm_panel<<<cdiv(rest, 32), 128, 0, st>>>(A, lda, m, k0, kb);
+      k_trsm_panel<<<cdiv(rest, kTrsmRows), 128, 0, st>>>(A, lda, m, k0, kb);
       launches++;
     }
     return kb;
