@@ -14,11 +14,11 @@
 //                inverts the factor for the next launch.  A negative pivot is
 //                replaced by its absolute value and counted
 //                (func.cpp:827-833).
-//   update CTAs  trailing update A_IJ -= L_I L_J^T of one or two earlier
+//   update CTAs  trailing update A_IJ -= L_I L_J^T of up to eleven earlier
 //                panels, a run of tiles per CTA, warp-specialised:
 //                bulk-async operand copies, three FP16 products (lo.hi,
-//                hi.lo, hi.hi) per panel into one of two FP32 tensor-memory
-//                accumulators (tcgen05.mma, M = N = 128, K = 16 per
+//                hi.lo, hi.hi) per panel, up to three panels into one of
+//                four FP32 tensor-memory accumulators (tcgen05.mma, M = N = 128, K = 16 per
 //                instruction), tcgen05.ld epilogue subtracting into the
 //                double-float tile.  The dropped product lo.lo is below
 //                2^-24 of the kept ones: FP32-class products.
@@ -720,7 +720,7 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
 //   warp 0 (one lane)  bulk-async copies: the two A slices when I changes,
 //                      the two B slices per tile in two K-halves (two
 //                      32 KB stages), and an L2 prefetch of the FP64 tile;
-//   warp 1 (one lane)  three FP16 products per K-half into one of two TMEM
+//   warp 1 (one lane)  three FP16 products per K-half into one of four TMEM
 //                      accumulators (128 columns each), tcgen05.commit to
 //                      release stages, the accumulator and the A operand;
 //   warps 2-9          epilogue: tcgen05.ld of the accumulator (warp w reads
@@ -738,9 +738,6 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
 #endif
 #ifndef BD_EPI_AHEAD
 #define BD_EPI_AHEAD 8  // chunks of 8 columns whose old values are in flight per epilogue thread (4: 8 % slower bulk)
-#endif
-#ifndef BD_EPI_TMEM_COLS
-#define BD_EPI_TMEM_COLS 8  // accumulator columns per TMEM read of the bulk epilogue (8, 16 or 32)
 #endif
 #ifndef BD_REST_GROUP
 #define BD_REST_GROUP 0  // tiles per CTA; 0: from the tile count
@@ -760,36 +757,66 @@ constexpr size_t kRestSmem = kPanelSmem;
 static_assert(kRestSmem >= (size_t)kTileBytes + 2 * kStageBytes + 1024 + 256, "the update CTAs' operands");
 constexpr int kAccCols = 128;
 
+constexpr int kAccs = 4;       // accumulators in tensor memory (all of its columns)
+constexpr int kFoldPanels = 3;  // panels summed into one of them (K = 384): longer sums truncate more
 struct RestBars {
-  uint64_t fullA, emptyA, fullB[2], emptyB[2], accFull[2], accEmpty[2], done;
+  uint64_t fullA, emptyA, fullB[2], emptyB[2], accFull[kAccs], accEmpty[kAccs], done;
+};
+// Panel slices: panel p in buffer p % bufs, buf bytes apart
+struct Slices {
+  const unsigned char* base;
+  size_t buf;
+  int bufs;
+  __device__ __forceinline__ const unsigned char* at(int p) const { return base + (size_t)(p % bufs) * buf; }
 };
 
 // Tile t of an update job's enumeration, from column jlo:
 //   kRowTri  the triangle I >= J >= jlo row by row (consecutive tiles share I),
+//   kBlkTri  the same by super-columns of kSuper tile columns, each row by row
+//            downward: the tiles in flight read the slices of 32 columns and a
+//            few dozen rows, where six panels' slices of a whole row of a large
+//            matrix are more than L2 holds (3N = 46,200: 142 MB; the
+//            factorisation takes 145 ms row by row, 139 so, 144 with 8 columns),
 //   kCol     column jlo alone (I = jlo + t).
-enum { kRowTri = 0, kCol = 1 };
+enum { kRowTri = 0, kCol = 1, kBlkTri = 2 };
+constexpr int kSuper = 32;
 __device__ __forceinline__ void rest_tile(int t, int jlo, int mode, int nt, int& I, int& J) {
   if (mode == kCol) {
     I = jlo + t;
     J = jlo;
     return;
   }
+  int w = nt - jlo, j0 = jlo;  // rows below (and at) the super-column's first, its width
+  if (mode == kBlkTri) {
+    for (; w > kSuper; w -= kSuper, j0 += kSuper) {
+      const int cnt = kSuper * (kSuper + 1) / 2 + (w - kSuper) * kSuper;
+      if (t < cnt) break;
+      t -= cnt;
+    }
+    w = min(w, kSuper);
+    const int u = t - w * (w + 1) / 2;
+    if (u >= 0) {  // below the super-column's triangle
+      I = j0 + w + u / w;
+      J = j0 + u % w;
+      return;
+    }
+  }
   int Ip = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
   while ((Ip + 1) * (Ip + 2) / 2 <= t) Ip++;
   while (Ip * (Ip + 1) / 2 > t) Ip--;
-  I = jlo + Ip;
-  J = jlo + (t - Ip * (Ip + 1) / 2);
+  I = j0 + Ip;
+  J = j0 + (t - Ip * (Ip + 1) / 2);
 }
 
-// `cta` is the CTA's index among the update CTAs.
-// NPAN = 1: one panel's update, the A operand resident per row of tiles.
-// NPAN = 2, 3: two or three consecutive panels' updates (PS, PS2, PS3) in one
-// read-modify-write of the tile (K = 256, 384): both operands streamed in
-// 2 NPAN chunks of 64 KB per tile (panel, K-half) through the two stages.
-template <int NPAN>
+// `cta` is the CTA's index among the update CTAs.  Panels p0 .. p0 + npan - 1.
+// NF = 0: one panel, the A operand resident per row of tiles.
+// NF = 1, 2, 4: up to 3 NF consecutive panels' updates in one read-modify-write of
+// the tile: both operands streamed in 2 npan chunks of 64 KB per tile (panel,
+// K-half) through the two stages, three panels to an accumulator, NF of them
+// subtracted from the tile one after the other (as NF passes would).
+template <int NF>
 __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int lda, int m, int jlo, int mode,
-                                          int tlo, int thi, int group, int cta, const unsigned char* __restrict__ PS,
-                                          const unsigned char* __restrict__ PS2, const unsigned char* __restrict__ PS3,
+                                          int tlo, int thi, int group, int cta, const Slices& sl, int p0, int npan,
                                           int* err, float iscale2) {
   // (rounded as an integer, not by align1024: with the pointer known to be
   // shared the compiler places the epilogue's loads worse, 211 against 161 ms
@@ -810,6 +837,8 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
     for (int h = 0; h < 2; h++) {
       sm100::mbar_init(&bars->fullB[h], 1);
       sm100::mbar_init(&bars->emptyB[h], 1);
+    }
+    for (int h = 0; h < kAccs; h++) {
       sm100::mbar_init(&bars->accFull[h], 1);
       sm100::mbar_init(&bars->accEmpty[h], 8);
     }
@@ -817,7 +846,7 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
     *abort_flag = 0;
     sm100::fence_mbar_init();
   }
-  if (warp == 1) sm100::tmem_alloc(tslot, 2 * kAccCols);
+  if (warp == 1) sm100::tmem_alloc(tslot, kAccs * kAccCols);
   sm100::tc_fence_before();
   __syncthreads();
   sm100::tc_fence_after();
@@ -826,7 +855,8 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
   if (warp == 0) {
     if (lane == 0) {
       // ---------------- producer
-      if constexpr (NPAN == 1) {
+      const unsigned char* PS = sl.at(p0);  // (NF = 0)
+      if constexpr (NF == 0) {
       int curI = -1;
       uint32_t nA = 0, nfill[2] = {0, 0};
       bool ok = true;
@@ -876,7 +906,7 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
         if (nfill[h] > 0) (void)sm100::mbar_wait(&bars->fullB[h], (nfill[h] - 1) & 1, kWaitLimit);
       if (nA > 0) (void)sm100::mbar_wait(&bars->fullA, (nA - 1) & 1, kWaitLimit);
       } else {
-        // NPAN panels: chunk q = (panel q >> 1, K-half q & 1) of both operands
+        // chunk q = (panel p0 + (q >> 1), K-half q & 1) of both operands
         uint32_t nfill[2] = {0, 0};
         int ctot = 0;
         bool ok = true;
@@ -884,14 +914,14 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
           int I, J;
           rest_tile(t, jlo, mode, nt, I, J);
           const bool dg = I == J;
-          for (int q = 0; q < 2 * NPAN; q++) {
+          for (int q = 0; q < 2 * npan; q++) {
             const int st = ctot & 1;
             if (nfill[st] > 0) ok = sm100::mbar_wait(&bars->emptyB[st], (nfill[st] - 1) & 1, kWaitLimit);
             if (!ok || *abort_flag) {
               ok = false;
               break;
             }
-            const unsigned char* src = (q >> 1) == 0 ? PS : ((q >> 1) == 1 ? PS2 : PS3);
+            const unsigned char* src = sl.at(p0 + (q >> 1));
             const int h = q & 1;
             unsigned char* sa = sm + st * (2 * kStageBytes);
             sm100::mbar_arrive_expect_tx(&bars->fullB[st], dg ? kStageBytes : 2 * kStageBytes);
@@ -918,7 +948,7 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
   } else if (warp == 1) {
     if (lane == 0) {
       // ---------------- MMA issuer
-      if constexpr (NPAN == 1) {
+      if constexpr (NF == 0) {
       const uint32_t idesc = sm100::idesc_f16_f32(128, 128);
       const int pa[3] = {1, 0, 0};  // (A slice, B slice) products, smallest first
       const int pb[3] = {0, 1, 0};
@@ -974,43 +1004,42 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
         const int pa[3] = {1, 0, 0};
         const int pb[3] = {0, 1, 0};
         uint32_t nuse[2] = {0, 0};
-        int ctot = 0;
+        int ctot = 0, nacc = 0;  // chunks, accumulators used
         bool ok = true;
-        int n = 0;
-        for (int t = t0; t < t1; t++, n++) {
+        for (int t = t0; t < t1 && ok; t++) {
           int I, J;
           rest_tile(t, jlo, mode, nt, I, J);
           if (*abort_flag) break;
           const bool dg = I == J;
-          const int acc = n & 1;
-          if (n >= 2) {
-            ok = sm100::mbar_wait(&bars->accEmpty[acc], ((n >> 1) - 1) & 1, kWaitLimit);
-            if (!ok) break;
-          }
-          sm100::tc_fence_after();
-          const uint32_t d = tmem + (uint32_t)(acc * kAccCols);
-          for (int q = 0; q < 2 * NPAN && ok; q++) {
-            const int st = ctot & 1;
-            ok = sm100::mbar_wait(&bars->fullB[st], nuse[st] & 1, kWaitLimit);
+          for (int f = 0; f < NF && ok; f++, nacc++) {
+            const int q0 = 2 * kFoldPanels * f, q1 = min(q0 + 2 * kFoldPanels, 2 * npan), acc = nacc % kAccs;
+            if (nacc >= kAccs) ok = sm100::mbar_wait(&bars->accEmpty[acc], (nacc / kAccs - 1) & 1, kWaitLimit);
             if (!ok) break;
             sm100::tc_fence_after();
-            const unsigned char* sa = sm + st * (2 * kStageBytes);
-            const unsigned char* sb = dg ? sa : sa + kStageBytes;
+            const uint32_t d = tmem + (uint32_t)(acc * kAccCols);
+            for (int q = q0; q < q1; q++) {
+              const int st = ctot & 1;
+              ok = sm100::mbar_wait(&bars->fullB[st], nuse[st] & 1, kWaitLimit);
+              if (!ok) break;
+              sm100::tc_fence_after();
+              const unsigned char* sa = sm + st * (2 * kStageBytes);
+              const unsigned char* sb = dg ? sa : sa + kStageBytes;
 #pragma unroll
-            for (int p = 0; p < 3; p++) {
-              const uint32_t aaddr = sm100::smem_u32(sa + pa[p] * kHalfBytes);
-              const uint32_t baddr = sm100::smem_u32(sb + pb[p] * kHalfBytes);
+              for (int p = 0; p < 3; p++) {
+                const uint32_t aaddr = sm100::smem_u32(sa + pa[p] * kHalfBytes);
+                const uint32_t baddr = sm100::smem_u32(sb + pb[p] * kHalfBytes);
 #pragma unroll
-              for (int kk = 0; kk < 4; kk++)
-                sm100::mma_f16(d, sm100::desc_kmajor_sw128(aaddr + kk * 32),
-                                sm100::desc_kmajor_sw128(baddr + kk * 32), idesc, (q | p | kk) != 0);
+                for (int kk = 0; kk < 4; kk++)
+                  sm100::mma_f16(d, sm100::desc_kmajor_sw128(aaddr + kk * 32),
+                                  sm100::desc_kmajor_sw128(baddr + kk * 32), idesc, ((q - q0) | p | kk) != 0);
+              }
+              sm100::mma_commit(&bars->emptyB[st]);
+              nuse[st]++;
+              ctot++;
             }
-            sm100::mma_commit(&bars->emptyB[st]);
-            nuse[st]++;
-            ctot++;
+            if (!ok) break;
+            sm100::mma_commit(&bars->accFull[acc]);
           }
-          if (!ok) break;
-          sm100::mma_commit(&bars->accFull[acc]);
         }
         if (!ok) {
           atomicExch(err, 4);
@@ -1071,8 +1100,12 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
       float2* ncolp = A;
       int njcnt = 0;
       if (more) row_of(t + 1, ncolp, njcnt);
-      const int acc = n & 1;
-      const bool ok = sm100::mbar_wait(&bars->accFull[acc], (n >> 1) & 1, kWaitLimit);
+      // the tile's accumulators (NF = 0: two in turn)
+      constexpr int kNF = NF ? NF : 1, kRing = NF ? kAccs : 2;
+      bool ok = true;
+#pragma unroll
+      for (int f = 0; f < kNF; f++)
+        ok = ok && sm100::mbar_wait(&bars->accFull[(kNF * n + f) % kRing], ((kNF * n + f) / kRing) & 1, kWaitLimit);
       if (!ok || *abort_flag) {
         if (!ok && lane == 0) {
           atomicExch(err, 5);
@@ -1081,28 +1114,29 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
         break;
       }
       sm100::tc_fence_after();
+      const int acc = kNF * n % kRing;  // (the ring holds a whole number of tiles)
       const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(acc * kAccCols + 64 * ch);
-      // the accumulator is read kEpT columns at a time (one wait per read)
-      constexpr int kEpT = BD_EPI_TMEM_COLS, kEpR = kEpT / kEpC;
-      static_assert(kEpT % kEpC == 0 && kEpN % kEpR == 0, "TMEM reads cover whole chunks");
-      float vt[kEpT];
 #pragma unroll
       for (int c = 0; c < kEpN; c++) {
         const int s2 = c % kEpS;
-        if (c % kEpR == 0) {
-          if (kEpT == 8) sm100::tmem_ld8(ta + kEpC * c, vt);
-          else if (kEpT == 16) sm100::tmem_ld16(ta + kEpC * c, vt);
-          else sm100::tmem_ld32(ta + kEpC * c, vt);
-          if (c + kEpR == kEpN) {  // accumulator read out: hand it back to the MMA issuer
-            sm100::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) sm100::mbar_arrive(&bars->accEmpty[acc]);
-          }
+#pragma unroll
+        for (int f = 0; f < kNF; f++) {
+          if (f > 0 && f * kFoldPanels >= npan) continue;
+          float v[kEpC];
+          sm100::tmem_ld8(ta + f * kAccCols + kEpC * c, v);
+#pragma unroll
+          for (int j = 0; j < kEpC; j++) old[s2][j] = df_sub(old[s2][j], v[j] * iscale2);
         }
-        const float* v = vt + kEpC * (c % kEpR);
+        if (c == kEpN - 1) {  // read out: hand them back to the MMA issuer
+          sm100::tc_fence_before();
+          __syncwarp();
+          if (lane == 0)
+#pragma unroll
+            for (int e = 0; e < kNF; e++) sm100::mbar_arrive(&bars->accEmpty[acc + e]);
+        }
 #pragma unroll
         for (int j = 0; j < kEpC; j++)
-          if (kEpC * c + j < jcnt) st_tile(colp + (size_t)(kEpC * c + j) * lda, df_sub(old[s2][j], v[j] * iscale2));
+          if (kEpC * c + j < jcnt) st_tile(colp + (size_t)(kEpC * c + j) * lda, old[s2][j]);
         if (c + kEpS < kEpN) load_chunk(old[s2], colp, jcnt, c + kEpS);
         else if (more) load_chunk(old[s2], ncolp, njcnt, c + kEpS - kEpN);
       }
@@ -1112,25 +1146,24 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
   }
   sm100::tc_fence_before();
   __syncthreads();
-  if (warp == 1) sm100::tmem_dealloc(tmem, 2 * kAccCols);
+  if (warp == 1) sm100::tmem_dealloc(tmem, kAccs * kAccCols);
 }
 
 // An update job: tiles [tlo, thi) of an enumeration (rest_tile) from column
-// jlo, panel slices ps (and ps2: two panels, K = 256), `group` tiles per CTA.
+// jlo, panels p0 .. p0 + npan - 1, `group` tiles per CTA.
 struct UpdJob {
-  const unsigned char* ps;
-  const unsigned char* ps2;  // second panel (K = 256) or null
-  const unsigned char* ps3;  // third panel (K = 384) or null
-  int jlo, mode, tlo, thi, group, nctas;
+  int p0, npan, jlo, mode, tlo, thi, group, nctas;
 };
+constexpr int kJobs = 3;
 struct StepArgs {
   PanelArgs pan;  // panel k and the chain's tile
   int ntile;      // tile CTAs: tile rows k + 2 .. k + 1 + ntile
-  UpdJob job[2];
+  Slices sl;
+  UpdJob job[kJobs];
 };
 
 // One launch per step.  CTA 0 is the chain CTA, CTAs 1 .. ntile solve the
-// other tiles of panel k; then the CTAs of update job 0, then those of job 1.
+// other tiles of panel k; then the CTAs of the update jobs in turn.
 // The parts of one launch touch disjoint tiles and slice buffers.
 __device__ __forceinline__ void chol_step_body(const StepArgs& a, int b, float4* smem4) {
   unsigned char* sm = reinterpret_cast<unsigned char*>(smem4);
@@ -1146,16 +1179,18 @@ __device__ __forceinline__ void chol_step_body(const StepArgs& a, int b, float4*
     return;
   }
   b -= a.ntile;
-  const int jn = b < a.job[0].nctas ? 0 : 1;
-  if (jn) b -= a.job[0].nctas;
+  int jn = 0;
+  while (jn < kJobs - 1 && b >= a.job[jn].nctas) b -= a.job[jn++].nctas;
   const UpdJob& j = a.job[jn];
   const PanelArgs& p = a.pan;
-  if (j.ps3)
-    rest_body<3>(sm, p.A, p.lda, p.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b, j.ps, j.ps2, j.ps3, p.err, p.iscale2);
-  else if (j.ps2)
-    rest_body<2>(sm, p.A, p.lda, p.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b, j.ps, j.ps2, nullptr, p.err, p.iscale2);
-  else
-    rest_body<1>(sm, p.A, p.lda, p.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b, j.ps, nullptr, nullptr, p.err, p.iscale2);
+  auto run = [&](auto nf) {
+    rest_body<decltype(nf)::value>(sm, p.A, p.lda, p.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b, a.sl, j.p0, j.npan,
+                                   p.err, p.iscale2);
+  };
+  if (j.npan > 2 * kFoldPanels) run(std::integral_constant<int, 4>{});
+  else if (j.npan > kFoldPanels) run(std::integral_constant<int, 2>{});
+  else if (j.npan > 1) run(std::integral_constant<int, 1>{});
+  else run(std::integral_constant<int, 0>{});
 }
 
 __global__ void __launch_bounds__(kRestThreads, 1) k_chol_step(const __grid_constant__ StepArgs a) {
@@ -1189,12 +1224,23 @@ __global__ void __launch_bounds__(kRestThreads, 1) k_chol_step_multi(const StepA
 
 namespace bdk {
 
-// kBufs panel-slice buffers, panel p in buffer p % kBufs: a triple's bulk
-// update reads panels k .. k + 2 while panel k + 3 is written
-constexpr int kBufs = 4;
+// Panels per bulk pass while the trailing matrix is large (max_pass 3).  Six from
+// kWideTiles tile rows on: half the read-modify-writes of three (which with the
+// products' operands fill the SM's shared-memory and L1 path: 13 kcycles a tile
+// and three panels, 6 of them the products'), against column updates by up to
+// eleven panels.  3N = 46,200: 155 ms with three, 136 with six; 24,300: 27.2, 27.7;
+// 17,820: 12.4, 13.1.
+constexpr int kWideTiles = 256;
+static int group_of(int nt) { return nt >= kWideTiles ? 6 : 3; }
+// Slice buffers, panel p in buffer p % bufs: three panels' bulk update reads them
+// while the next is written; six panels' runs beside the next six.
+static int bufs_of(int nt) { return nt >= kWideTiles ? 12 : 4; }
 // the slice buffers, then two buffers for the inverse of a diagonal factor
 // (W_k in buffer k & 1: read by the launch that writes W_k+1), then its factors
-size_t mixed_panel_bytes(int m) { return kBufs * (size_t)cdiv(m, kT) * kTileBytes + 2 * (size_t)kTileBytes + 2 * kT * sizeof(float); }
+size_t mixed_panel_bytes(int m) {
+  const int nt = cdiv(m, kT);
+  return (size_t)bufs_of(nt) * nt * kTileBytes + 2 * (size_t)kTileBytes + 2 * kT * sizeof(float);
+}
 int mixed_max_launches(int m) { return 2 * cdiv(m, kT) + 2; }
 int mixed_tiles(int m) { return cdiv(m, kT); }
 
@@ -1225,8 +1271,8 @@ int set_mixed_attributes() {
 }
 
 // Tiles per CTA of the bulk update: enough CTAs to fill the GPU about three
-// times over, at most 8 tiles each.
-static int rest_group(int tiles) {
+// times over, at most gmax tiles each (8; 4 with six panels a pass, 1 % faster).
+static int rest_group(int tiles, int gmax) {
   if (BD_REST_GROUP > 0) return BD_REST_GROUP;
   static int sms = 0;
   if (!sms) {
@@ -1236,27 +1282,29 @@ static int rest_group(int tiles) {
     if (sms <= 0) sms = 1;
   }
   int g = tiles / (BD_REST_WAVES * sms);
-  return g < BD_REST_GMIN ? BD_REST_GMIN : (g > BD_REST_GMAX ? BD_REST_GMAX : g);
+  return g < BD_REST_GMIN ? BD_REST_GMIN : (g > gmax ? gmax : g);
 }
 
 // Right-looking with a lookahead of one panel, on one stream, no two kernels
 // at a time; every launch is one k_chol_step: panel k's tiles solved and
 // diagonal block k + 1 factored (the chain and tile CTAs, which apply panel
-// k - 1's update to column k themselves) beside up to two update jobs.  Panel
-// p's slices live in buffer p % kBufs, W_p in buffer p & 1.  Invariant before
+// k - 1's update to column k themselves) beside up to three update jobs.  Panel
+// p's slices live in buffer p % bufs, W_p in buffer p & 1.  Invariant before
 // the launch of panel k + 1: panels <= k are solved, column k + 1 and diagonal
 // block k + 2 hold the updates of panels < k, and the launch leaves diagonal
 // block k + 2 to its chain CTA (which applies panels k and k + 1).
-// Single step: panel k + 1 beside panel k's update of the tiles right of
-// column k + 1 (K = 128).
-// Pair (k+1, k+2), while the trailing matrix is large: the bulk tiles get
-// both panels in one read-modify-write (K = 256), half the HBM traffic:
-//   1: panel k+1 beside panel k's update of column k+2 and of diagonal block k+3;
-//   2: panel k+2 beside panels k and k+1 on the tiles right of column k+2.
-// Triple (k+1 .. k+3), while it is larger still (K = 384):
-//   1: panel k+1 beside panel k's update of column k+2 and of diagonal block k+3;
-//   2: panel k+2 beside panels k and k+1 on column k+3 (K = 256) and on diagonal block k+4;
-//   3: panel k+3 beside panels k .. k+2 on the tiles right of column k+3.
+// Groups of g panels k .. k + g - 1 (1, 2, 3 or 6) share one read-modify-write of
+// the tiles right of them (K = 128 g), the more the larger the trailing matrix:
+//   launch k + i, i = 1 .. g - 1: panel k + i beside panels k .. k + i - 1 on
+//     column k + i + 1 and on diagonal block k + i + 2;
+//   launch k + g: panel k + g beside the group on the tiles right of column k + g.
+// Groups of six: that last pass waits for the next group (b .. k - 1 the solved
+// one, k .. k + g - 1 the next):
+//   launch k + i, i = 0 .. g - 1: panel k + i beside panels b .. k + i - 1 on
+//     column k + i + 1 and diagonal block k + i + 2, and a g-th of the solved
+//     group's pass over the tiles right of column k + g;
+// so that the bulk is spread over all launches.  (With three the column updates
+// cost what the spreading gains: 4.97 and 4.99 ms at 3N = 11,700.)
 // Returns the number of kernel launches.
 #ifndef BD_PAIR_MIN
 #define BD_PAIR_MIN 24  // pair while at least this many tile rows remain right of column k+2 (k: last factored)
@@ -1264,12 +1312,12 @@ static int rest_group(int tiles) {
 #ifndef BD_TRIPLE_MIN
 #define BD_TRIPLE_MIN 40  // three panels per bulk pass while this many tile rows remain right of column k+3
 #endif
+#ifndef BD_DEFER_MIN
+#define BD_DEFER_MIN 24  // a group's bulk runs beside the next group's panels while this many tile rows remain
+#endif
 namespace {
 struct Job {
-  const unsigned char* ps = nullptr;
-  const unsigned char* ps2 = nullptr;
-  const unsigned char* ps3 = nullptr;
-  int jlo = 0, mode = kCol, tlo = 0, tiles = 0, group = 1;
+  int p0 = 0, npan = 0, jlo = 0, mode = kCol, tlo = 0, tiles = 0, group = 1;  // tiles: the enumeration's end
 };
 }  // namespace
 
@@ -1287,8 +1335,9 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
   const size_t buf = (size_t)nt * kTileBytes;
   int L = 0, timed = 0;
   auto kb_of = [&](int k) { return (m - k * kT < kT) ? m - k * kT : kT; };
-  auto psb = [&](int k) { return PS + (size_t)(k % kBufs) * buf; };
-  unsigned char* Wb = PS + kBufs * buf;  // the inverses' slices
+  const int bufs = bufs_of(nt);
+  auto psb = [&](int k) { return PS + (size_t)(k % bufs) * buf; };
+  unsigned char* Wb = PS + bufs * buf;  // the inverses' slices
   float* wsc = reinterpret_cast<float*>(Wb + 2 * (size_t)kTileBytes);
   // elements of the lower triangle in tile columns [j0, j1)
   auto elems = [&](int j0, int j1) {
@@ -1302,25 +1351,25 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
   // panels p .. p + npan - 1 on column J below its diagonal block (the chain CTA's)
   auto col_job = [&](int p, int J, int npan = 1) {
     Job j;
-    j.ps = psb(p), j.ps2 = npan > 1 ? psb(p + 1) : nullptr, j.jlo = J, j.mode = kCol, j.tlo = 1, j.tiles = nt - J;
+    j.p0 = p, j.npan = npan, j.jlo = J, j.mode = kCol, j.tlo = 1, j.tiles = nt - J;
     return j;
   };
   auto diag_job = [&](int p, int J, int npan = 1) {  // ... on diagonal block J alone
     Job j;
-    j.ps = psb(p), j.ps2 = npan > 1 ? psb(p + 1) : nullptr, j.jlo = J, j.mode = kCol, j.tiles = 1;
+    j.p0 = p, j.npan = npan, j.jlo = J, j.mode = kCol, j.tiles = J < nt ? 1 : 0;
     return j;
   };
-  auto tri_job = [&](int p, int npan, int jlo) {  // ... on the triangle from column jlo but its first diagonal block
+  // ... on part `part` of `parts` of the triangle from column jlo but its first diagonal block
+  auto tri_job = [&](int p, int npan, int jlo, int part = 0, int parts = 1) {
     Job j;
-    const int n = nt - jlo;
-    j.ps = psb(p), j.ps2 = npan > 1 ? psb(p + 1) : nullptr, j.ps3 = npan > 2 ? psb(p + 2) : nullptr;
-    j.jlo = jlo, j.mode = kRowTri, j.tlo = 1;
-    j.tiles = n > 0 ? n * (n + 1) / 2 : 0;
-    j.group = rest_group(j.tiles);
+    const long n = nt - jlo, all = n > 0 ? n * (n + 1) / 2 - 1 : 0;
+    j.p0 = p, j.npan = npan, j.jlo = jlo, j.mode = npan > kFoldPanels ? kBlkTri : kRowTri;
+    j.tlo = 1 + (int)(all * part / parts), j.tiles = 1 + (int)(all * (part + 1) / parts);
+    j.group = rest_group(j.tiles - j.tlo, npan > kFoldPanels ? 4 : BD_REST_GMAX);
     return j;
   };
   // panel k's tiles (k < 0: none) and diagonal block k + 1
-  auto launch = [&](int k, const Job& j0, const Job& j1) {
+  auto launch = [&](int k, const Job& j0, const Job& j1 = Job(), const Job& j2 = Job()) {
     StepArgs a{};
     PanelArgs& p = a.pan;
     p.A = A, p.lda = lda, p.m = m, p.k = k, p.tile = k < 0 ? -1 : k + 1;
@@ -1329,13 +1378,13 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
     p.Wn = Wb + (size_t)((k + 1) & 1) * kTileBytes, p.wscn = wsc + kT * ((k + 1) & 1);
     p.negpiv = negpiv, p.err = err, p.scale = scale, p.iscale2 = 1.f / (scale * scale);
     a.ntile = k < 0 ? 0 : nt - k - 2;
-    const Job* js[2] = {&j0, &j1};
+    a.sl = Slices{PS, buf, bufs};
+    const Job* js[kJobs] = {&j0, &j1, &j2};
     int grid = 1 + a.ntile;
-    for (int q = 0; q < 2; q++) {
+    for (int q = 0; q < kJobs; q++) {
       const Job& j = *js[q];
       UpdJob& u = a.job[q];
-      u.ps = j.ps, u.ps2 = j.ps2, u.ps3 = j.ps3, u.jlo = j.jlo, u.mode = j.mode, u.tlo = j.tlo, u.thi = j.tiles,
-      u.group = j.group;
+      u.p0 = j.p0, u.npan = j.npan, u.jlo = j.jlo, u.mode = j.mode, u.tlo = j.tlo, u.thi = j.tiles, u.group = j.group;
       u.nctas = j.tiles > j.tlo ? cdiv(j.tiles - j.tlo, j.group) : 0;
       grid += u.nctas;
     }
@@ -1354,34 +1403,36 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
       const double tile_fl = 3.0 * 2.0 * kT * kT * kT;
       double by = 16.0 * (double)(m - (k + 1) * kT) * (k < 0 ? kb_of(0) : kT);  // panel read and written back
       double fl = k < 0 ? 0.0 : tile_fl * (2.0 * (1 + a.ntile) + 2.0);        // the panel CTAs' own products
-      for (int q = 0; q < 2; q++) {
+      for (int q = 0; q < kJobs; q++) {
         const Job& j = *js[q];
         if (j.tiles <= j.tlo) continue;
-        by += 16.0 * (j.tiles == 1 ? 0.5 * kT * kb_of(j.jlo) : elems(j.jlo, j.mode == kCol ? j.jlo + 1 : nt));
-        fl += tile_fl * (j.tiles - j.tlo) * (j.ps3 ? 3 : (j.ps2 ? 2 : 1));  // FP16 tensor work issued
+        const double all = nt - j.jlo;  // a part of the triangle: its share of the elements
+        by += 16.0 * (j.mode == kCol ? (j.tiles == 1 ? 0.5 * kT * kb_of(j.jlo) : elems(j.jlo, j.jlo + 1))
+                                     : elems(j.jlo, nt) * (j.tiles - j.tlo) / (0.5 * all * (all + 1)));
+        fl += tile_fl * (j.tiles - j.tlo) * j.npan;  // FP16 tensor work issued
       }
       if (kbytes) *kbytes += by;
       if (kflop) *kflop += fl;
     }
   };
-  const Job none;
-  launch(-1, none, none);             // diagonal block 0
-  if (nt > 1) launch(0, none, none);  // panel 0
+  launch(-1, Job());             // diagonal block 0
+  if (nt > 1) launch(0, Job());  // panel 0
+  const int G = group_of(nt);
   int k = 0;
   while (k + 2 < nt) {
-    if (max_pass >= 3 && nt - (k + 4) >= BD_TRIPLE_MIN) {
-      launch(k + 1, col_job(k, k + 2), diag_job(k, k + 3));
-      launch(k + 2, col_job(k, k + 3, 2), diag_job(k, k + 4, 2));
-      launch(k + 3, tri_job(k, 3, k + 4), none);
-      k += 3;
-    } else if (max_pass >= 2 && nt - (k + 3) >= BD_PAIR_MIN) {
-      launch(k + 1, col_job(k, k + 2), diag_job(k, k + 3));
-      launch(k + 2, tri_job(k, 2, k + 3), none);
-      k += 2;
-    } else {
-      launch(k + 1, tri_job(k, 1, k + 2), none);
-      k += 1;
+    const int g = max_pass >= 3 && nt - (k + 1 + G) >= BD_TRIPLE_MIN ? G
+                  : max_pass >= 2 && nt - (k + 3) >= BD_PAIR_MIN     ? 2
+                                                                     : 1;
+    for (int i = 1; i < g; i++) launch(k + i, col_job(k, k + i + 1, i), diag_job(k, k + i + 2, i));
+    int b = k;
+    k += g;  // panels b .. k - 1 are solved, their update right of column k is not made
+    while (g > kFoldPanels && nt - (k + g + 1) >= BD_DEFER_MIN) {
+      for (int i = 0; i < g; i++)
+        launch(k + i, col_job(b, k + i + 1, g + i), diag_job(b, k + i + 2, g + i), tri_job(b, g, k + g + 1, i, g));
+      b = k;
+      k += g;
     }
+    launch(k, tri_job(b, g, k + 1));
   }
   if (plan) return L;
   if (kev_pairs) *kev_pairs = timed;
