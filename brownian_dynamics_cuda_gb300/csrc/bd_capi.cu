@@ -200,7 +200,7 @@ static int step_phases(bd_ctx* c, const double* d_rr, const double* d_p, double*
       join();
       return set_error(rc, "bd_step: Krylov noise displacement failed");
     }
-    L += 10 * c->krylov_iters + 4;
+    L += (mixed ? 6 : 7) * c->krylov_iters + 3;
   } else {
     bdk::trmv_lower_ws(c->m, c->A, c->lda, d_p, M.s2dt, c->rd, c->rd_part, st, mixed);
     L += 2;

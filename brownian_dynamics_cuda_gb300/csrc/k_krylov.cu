@@ -112,122 +112,143 @@ __global__ void k_symv_sum(int m, int nt, const double* __restrict__ P, double* 
   y[r] = s;
 }
 
-// Matrix-free product y = D x for mixed contexts: no tensor in memory.  A
-// warp per bead i; the other beads (double-float positions qh/ql with the
-// radius in w, and x as float4) staged through shared memory; the FP32 RPY
-// block of every pair (rpy_block_f, the mixed tensor's own formula) applied
-// to x_j; runs of 32 terms in FP32, the runs added with Kahan compensation;
-// lanes summed in FP64 in a fixed order.
-constexpr int kMvTile = 256;
-constexpr int kMvB = 2;   // beads per warp: each staged bead j serves both
-constexpr int kMvW = 8;   // warps per CTA (4 measured slower: the staging is per CTA)
+// Double-float (hi, lo) addition in FP32 (two-sum, then renormalised).
+__device__ __forceinline__ void df_add(float& h, float& l, float h2, float l2) {
+  const float s = h + h2, bb = s - h, e = (h - (s - bb)) + (h2 - bb);
+  const float t = e + l + l2;
+  h = s + t;
+  l = t - (h - s);
+}
+
+// 1/sqrt of a squared distance (nm^2), without rsqrtf's scaling of denormals
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// Matrix-free product y = D x for mixed contexts: no tensor in memory.  A CTA
+// per kMvB beads; lane l takes beads j = l, l + 32, ... (double-float positions
+// qh/ql with the radius in w, and x as float4); the FP32 RPY block of every pair
+// (rpy_block_f, the mixed tensor's own formula) applied to x_j; runs of 32 terms
+// in FP32, a run per warp, the runs added in order with Kahan compensation; lanes
+// summed in double-float in a fixed order.  Bound by FP32 issue.  n_D = 3,900: 55
+// us with two beads and all runs a warp, eight warps a CTA (244 CTAs: three or
+// four warps a scheduler), FP64 lane sums and a test for the own bead in every
+// pair; 43 in this split, 36 with the far form of all four beads first.
+constexpr int kMvB = 4;    // beads per CTA: each bead j that is read serves all
+constexpr int kMvW = 4;    // warps per CTA
+constexpr int kMvRun = 32;
 __global__ void __launch_bounds__(32 * kMvW) k_rpy_mv(int nD, const float4* __restrict__ qh, const float4* __restrict__ ql,
                                                 const float4* __restrict__ xf, float a1f, float a2f,
                                                 double* __restrict__ y) {
-  __shared__ float4 sh[kMvTile], sl[kMvTile], sx[kMvTile];
+  constexpr int kV = 3 * kMvB, kMine = kV / kMvW;  // values, of them a warp's
+  __shared__ float runs[kMvW][kV][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int i0 = (blockIdx.x * kMvW + warp) * kMvB;
+  const int i0 = blockIdx.x * kMvB;
   float4 hi[kMvB], lo[kMvB];
-  bool act[kMvB];
 #pragma unroll
   for (int b = 0; b < kMvB; b++) {
-    const int i = i0 + b;
-    act[b] = i < nD;
-    hi[b] = act[b] ? qh[i] : make_float4(0.f, 0.f, 0.f, 1.f);
-    lo[b] = act[b] ? ql[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int i = min(i0 + b, nD - 1);  // (past the end: not stored)
+    hi[b] = qh[i];
+    lo[b] = ql[i];
   }
-  float run[kMvB][3], ks[kMvB][3], kc[kMvB][3];
+  float ks[kMine], kc[kMine];
 #pragma unroll
-  for (int b = 0; b < kMvB; b++)
+  for (int q = 0; q < kMine; q++) ks[q] = kc[q] = 0.f;
+  for (int base = 0; base < nD; base += 32 * kMvRun * kMvW) {
+    float run[kMvB][3];
 #pragma unroll
-    for (int q = 0; q < 3; q++) run[b][q] = ks[b][q] = kc[b][q] = 0.f;
-  int cnt = 0;
-  for (int base = 0; base < nD; base += kMvTile) {
-    __syncthreads();
-    for (int t = threadIdx.x; t < kMvTile && base + t < nD; t += blockDim.x) {
-      sh[t] = qh[base + t];
-      sl[t] = ql[base + t];
-      sx[t] = xf[base + t];
-    }
-    __syncthreads();
-    if (!act[0]) continue;  // warp-uniform: the warp's first bead is past the end
-    const int je = min(nD, base + kMvTile);
-    for (int j = base + lane; j < je; j += 32) {
-      const int t = j - base;
-      const float4 v = sx[t], hj = sh[t], lj = sl[t];
+    for (int b = 0; b < kMvB; b++) run[b][0] = run[b][1] = run[b][2] = 0.f;
+    const int j0 = base + warp * 32 * kMvRun, j1 = min(nD, j0 + 32 * kMvRun);
+    for (int j = j0 + lane; j < j1; j += 32) {
+      const float4 v = xf[j], hj = qh[j], lj = ql[j];
+      // the RPY block of the pair applied to v without forming it: D v = c_d v +
+      // w s (s . v); all beads' far form first (so that their chains overlap),
+      // then the few overlapping pairs
+      float sx[kMvB], sy[kMvB], sz[kMvB], cd[kMvB], w[kMvB];
+      unsigned near = 0;
 #pragma unroll
       for (int b = 0; b < kMvB; b++) {
-        if (j == i0 + b) {
-          const float d = a1f / hi[b].w;
-          run[b][0] += d * v.x;
-          run[b][1] += d * v.y;
-          run[b][2] += d * v.z;
-          continue;
-        }
-        // the RPY block of the pair applied to v without forming it:
-        // D v = c_d v + w s (s . v)
         const float sxv = (hi[b].x - hj.x) + (lo[b].x - lj.x), syv = (hi[b].y - hj.y) + (lo[b].y - lj.y),
                     szv = (hi[b].z - hj.z) + (lo[b].z - lj.z);
         const float ssq = sxv * sxv + syv * syv + szv * szv;
-        const float inv_s = rsqrtf(ssq);
+        const float inv_s = rsqrt_ftz(ssq);
         const float sd = ssq * inv_s;
         const float ri = hi[b].w, rj = hj.w;
-        float cd, w;
-        if (sd >= ri + rj) {
-          const float inv_ssq = inv_s * inv_s;
-          const float f = (ri * ri + rj * rj) * inv_ssq;
-          const float as = a2f * inv_s;
-          cd = as * (1.f + f * (1.f / 3.f));
-          w = as * (1.f - f) * inv_ssq;
-        } else {
-          const float se = cbrtf((ri * ri * ri + rj * rj * rj) / 2.f);
-          const float as = a1f / se;
-          cd = as * (1.f - 9.f * sd / (32.f * se));
-          w = as * 3.f / (32.f * se * sd);
-        }
-        const float sv = w * (sxv * v.x + syv * v.y + szv * v.z);
-        run[b][0] += cd * v.x + sxv * sv;
-        run[b][1] += cd * v.y + syv * sv;
-        run[b][2] += cd * v.z + szv * sv;
+        const float inv_ssq = inv_s * inv_s;
+        const float f = (ri * ri + rj * rj) * inv_ssq;
+        const float as = a2f * inv_s;
+        cd[b] = as * (1.f + f * (1.f / 3.f));
+        w[b] = as * (1.f - f) * inv_ssq;
+        if (!(sd >= ri + rj)) near |= 1u << b;
+        sx[b] = sxv, sy[b] = syv, sz[b] = szv;
       }
-      if (++cnt == 32) {
+      if (near) {
+#pragma unroll 1
+        for (int b = 0; b < kMvB; b++) {
+          if (!(near >> b & 1)) continue;
+          float x = 0.f, y2 = 0.f, z = 0.f, ri = 0.f;
 #pragma unroll
-        for (int b = 0; b < kMvB; b++)
-#pragma unroll
-          for (int q = 0; q < 3; q++) {
-            const float u = run[b][q] - kc[b][q], t2 = ks[b][q] + u;
-            kc[b][q] = (t2 - ks[b][q]) - u;
-            ks[b][q] = t2;
-            run[b][q] = 0.f;
+          for (int e = 0; e < kMvB; e++)
+            if (e == b) x = sx[e], y2 = sy[e], z = sz[e], ri = hi[e].w;
+          const float rj = hj.w;
+          float cn, wn;
+          if (j == i0 + b) {  // the bead itself
+            cn = a1f / ri;
+            wn = 0.f;
+          } else {
+            const float ssq = x * x + y2 * y2 + z * z;
+            const float sd = ssq * rsqrt_ftz(ssq);
+            const float se = cbrtf((ri * ri * ri + rj * rj * rj) / 2.f);
+            const float as = a1f / se;
+            cn = as * (1.f - 9.f * sd / (32.f * se));
+            wn = as * 3.f / (32.f * se * sd);
           }
-        cnt = 0;
+#pragma unroll
+          for (int e = 0; e < kMvB; e++)
+            if (e == b) cd[e] = cn, w[e] = wn;
+        }
+      }
+#pragma unroll
+      for (int b = 0; b < kMvB; b++) {
+        const float sv = w[b] * (sx[b] * v.x + sy[b] * v.y + sz[b] * v.z);
+        run[b][0] += cd[b] * v.x + sx[b] * sv;
+        run[b][1] += cd[b] * v.y + sy[b] * sv;
+        run[b][2] += cd[b] * v.z + sz[b] * sv;
       }
     }
+    if (base > 0) __syncthreads();  // the last round's runs have been added
+#pragma unroll
+    for (int b = 0; b < kMvB; b++)
+#pragma unroll
+      for (int q = 0; q < 3; q++) runs[warp][3 * b + q][lane] = run[b][q];
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kMvW; w++)
+#pragma unroll
+      for (int q = 0; q < kMine; q++) {
+        const float u = runs[w][warp * kMine + q][lane] - kc[q], t2 = ks[q] + u;
+        kc[q] = (t2 - ks[q]) - u;
+        ks[q] = t2;
+      }
   }
 #pragma unroll
-  for (int b = 0; b < kMvB; b++) {
-    double sum[3];
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-      const float u = run[b][q] - kc[b][q], t2 = ks[b][q] + u;
-      sum[q] = (double)t2 - (double)((t2 - ks[b][q]) - u);
-    }
+  for (int q = 0; q < kMine; q++) {
+    float h = ks[q], l = -kc[q];
     for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-      for (int q = 0; q < 3; q++) sum[q] = sum[q] + __shfl_xor_sync(0xffffffffu, sum[q], o);
+      const float h2 = __shfl_xor_sync(0xffffffffu, h, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
+      df_add(h, l, h2, l2);
     }
-    if (act[b] && lane == 0) {
-      const int i = i0 + b;
-      y[3 * i] = sum[0];
-      y[3 * i + 1] = sum[1];
-      y[3 * i + 2] = sum[2];
-    }
+    const int e = 3 * i0 + warp * kMine + q;
+    if (lane == 0 && e < 3 * nD) y[e] = (double)h + (double)l;
   }
 }
 
 // partial dot products of the first ncol basis vectors with w, per block;
 // out[col * nb + block]
 constexpr int kDotB = 256;
+constexpr int kDotBlocks = 8;  // partial sums a column: few, as every block of the projection adds them up
 __global__ void __launch_bounds__(kDotB) k_dots(int m, const double* __restrict__ V, int ncol,
                                                 const double* __restrict__ w, double* __restrict__ out) {
   __shared__ double red[kDotB / 32];
@@ -257,48 +278,74 @@ __global__ void k_combine(int m, const double* __restrict__ V, int ncol, const d
 
 // w -= sum_{l < ncol} h_l V_l with h_l the fixed-order sums of k_dots'
 // partials (block 0, 1, ...), formed by every block into shared memory;
-// block 0 also stores h_{ncol-1} in *alpha when alpha is given
+// block 0 also stores h_{ncol-1} in *alpha when alpha is given; each block's
+// part of |w|^2 goes to nrm2 when given.  32 rows a block, a quarter of the
+// columns a warp: with a row a thread over all columns, 46 partials a column and
+// the norm in a launch of its own 16 us a call at 3N = 11,700 and 30 columns (load
+// latencies in a row), 7 so.
 constexpr int kProjMax = 520;
-__global__ void __launch_bounds__(128) k_sub_proj_sum(int m, const double* __restrict__ V, int ncol, int nb,
-                                                      const double* __restrict__ part, double* __restrict__ w,
-                                                      double* __restrict__ alpha) {
-  __shared__ double hs[kProjMax];
+constexpr int kSubRows = 32, kSubW = 4;
+__global__ void __launch_bounds__(32 * kSubW) k_sub_proj_sum(int m, const double* __restrict__ V, int ncol, int nb,
+                                                             const double* __restrict__ part, double* __restrict__ w,
+                                                             double* __restrict__ alpha, double* __restrict__ nrm2) {
+  __shared__ double hs[kProjMax], red[kSubW][32];
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int r = blockIdx.x * kSubRows + lane;
+  const double w0 = r < m ? w[r] : 0.0;
   for (int col = threadIdx.x; col < ncol; col += blockDim.x) {
     double t = 0.0;
+#pragma unroll 8
     for (int b = 0; b < nb; b++) t += part[(size_t)col * nb + b];
     hs[col] = t;
   }
   __syncthreads();
   if (alpha && blockIdx.x == 0 && threadIdx.x == 0) alpha[0] = hs[ncol - 1];
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= m) return;
-  double s = w[r];
-  for (int l = 0; l < ncol; l++) s -= hs[l] * V[(size_t)l * m + r];
-  w[r] = s;
+  double s = 0.0;
+  if (r < m) {
+#pragma unroll 8
+    for (int l = wp; l < ncol; l += kSubW) s = fma(hs[l], V[(size_t)l * m + r], s);
+  }
+  red[wp][lane] = s;
+  __syncthreads();
+  if (wp > 0) return;
+  double x = w0;
+#pragma unroll
+  for (int k = 0; k < kSubW; k++) x -= red[k][lane];
+  if (r < m) w[r] = x;
+  if (!nrm2) return;
+  x *= x;
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  if (lane == 0) nrm2[blockIdx.x] = x;
 }
 
-// |w| from k_dots' partials (fixed order, in every block), kept in *nrm
+// |w| from nb partial sums of |w|^2 (fixed order, in every block), kept in *nrm
 // and *beta; then, unless v is null, v = w / |w| and, for matrix-free
 // products, its float4 copy per bead (three rows per thread)
-__global__ void __launch_bounds__(256) k_norm_scale(int nD, int nb, const double* __restrict__ part,
+constexpr int kNormB = 64;  // few rows a block: FP64 work spreads over the SMs
+__global__ void __launch_bounds__(kNormB) k_norm_scale(int nD, int nb, const double* __restrict__ part,
                                                     const double* __restrict__ w, double* __restrict__ nrm,
                                                     double* __restrict__ beta, double* __restrict__ v,
                                                     float4* __restrict__ xf) {
   __shared__ double sn;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
     double t = 0.0;
-    for (int b = 0; b < nb; b++) t += part[b];
-    sn = sqrt(t);
-    if (blockIdx.x == 0) {
-      nrm[0] = sn;
-      if (beta) beta[0] = sn;
+#pragma unroll 8
+    for (int b = threadIdx.x; b < nb; b += 32) t += part[b];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (threadIdx.x == 0) {
+      const double n = sqrt(t);
+      sn = 1.0 / n;
+      if (blockIdx.x == 0) {
+        nrm[0] = n;
+        if (beta) beta[0] = n;
+      }
     }
   }
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (!v || i >= nD) return;
-  const double n = sn;
-  const double x = w[3 * i] / n, yv = w[3 * i + 1] / n, z = w[3 * i + 2] / n;
+  const double n = sn;  // 1 / |w|
+  const double x = w[3 * i] * n, yv = w[3 * i + 1] * n, z = w[3 * i + 2] * n;
   v[3 * i] = x;
   v[3 * i + 1] = yv;
   v[3 * i + 2] = z;
@@ -378,9 +425,9 @@ namespace bdk {
 
 size_t krylov_scratch_doubles(int m, int kmax) {
   const int nt = cdivk(m, kKT);
-  const int nb = std::min(cdivk(m, kDotB), 64);
+  const int nb = std::min(cdivk(m, kDotB), kDotBlocks);
   return (size_t)(kmax + 1) * m + (size_t)m + (size_t)nt * nt * kKT + (size_t)(kmax + 1) * nb +
-         3 * (size_t)(kmax + 2) + 8 + 2 * (size_t)cdivk(m, 3) + 2;
+         3 * (size_t)(kmax + 2) + 8 + 2 * (size_t)cdivk(m, 3) + 2 + (size_t)cdivk(m, kSubRows);
 }
 
 // rd = s2dt D^{1/2} p.  The tensor products: with A != nullptr from the
@@ -395,7 +442,7 @@ int krylov_sqrt(int m, const double* A, int lda, bool df, const float4* qh, cons
                 const double* p, double s2dt, double tol, int kmax, double* rd, double* scratch, cudaStream_t st,
                 int* iters, double* change, KrylovGraphs* graphs) {
   const int nt = cdivk(m, kKT), nD = m / 3;
-  const int nb = std::min(cdivk(m, kDotB), 64);
+  const int nb = std::min(cdivk(m, kDotB), kDotBlocks);
   double* V = scratch;
   double* w = V + (size_t)(kmax + 1) * m;
   double* P = w + m;
@@ -405,13 +452,15 @@ int krylov_sqrt(int m, const double* A, int lda, bool df, const float4* qh, cons
   double* beta = alpha + (kmax + 2);           // kmax + 2
   double* nrm = beta + (kmax + 2);             // 8
   // float4 needs 16-byte alignment: start on an even double offset from the (256-aligned) base
-  const size_t xoff = ((size_t)(nrm + 8 - scratch) + 1) & ~(size_t)1;
+  double* nrm2 = nrm + 8;                      // cdivk(m, kSubRows)
+  const int nb2 = cdivk(m, kSubRows);
+  const size_t xoff = ((size_t)(nrm2 + nb2 - scratch) + 1) & ~(size_t)1;
   float4* xf = reinterpret_cast<float4*>(scratch + xoff);
   const int tb = 256, gm = cdivk(m, tb);
   const long tiles = (long)nt * (nt + 1) / 2;
   if (kmax + 1 > kProjMax) return BD_ERR_ARG;
   float4* xfm = A ? nullptr : xf;  // the float4 copy of v_k that matrix-free products read
-  const int gb = cdivk(nD, tb);
+  const int gb = cdivk(nD, kNormB);
   // x = V_k: its float4 copy (matrix-free) was written with it by k_norm_scale
   auto product = [&](const double* x, double* y) {
     if (A) {
@@ -419,12 +468,12 @@ int krylov_sqrt(int m, const double* A, int lda, bool df, const float4* qh, cons
       else k_symv_tiles<false><<<(unsigned)tiles, kKB, 0, st>>>(m, nt, A, lda, x, P);
       k_symv_sum<<<gm, tb, 0, st>>>(m, nt, P, y);
     } else {
-      k_rpy_mv<<<cdivk(nD, kMvW * kMvB), 32 * kMvW, 0, st>>>(nD, qh, ql, xf, (float)a1, (float)a2, y);
+      k_rpy_mv<<<cdivk(nD, kMvB), 32 * kMvW, 0, st>>>(nD, qh, ql, xf, (float)a1, (float)a2, y);
     }
   };
   // v_0 = p / |p|
   k_dots<<<dim3(nb, 1), kDotB, 0, st>>>(m, p, 1, p, part);
-  k_norm_scale<<<gb, tb, 0, st>>>(nD, nb, part, p, nrm, nullptr, V, xfm);
+  k_norm_scale<<<gb, kNormB, 0, st>>>(nD, nb, part, p, nrm, nullptr, V, xfm);
   double pn = 0.0;
   if (cudaMemcpyAsync(&pn, nrm, sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
@@ -436,17 +485,17 @@ int krylov_sqrt(int m, const double* A, int lda, bool df, const float4* qh, cons
     return BD_OK;
   }
   std::vector<double> al, be, c, cprev, hal(kmax + 2), hbe(kmax + 2);
-  // one Lanczos iteration in seven launches: the product, twice the
+  // one Lanczos iteration in six launches: the product, twice the
   // projections on the basis so far (alpha_k from the first), the norm with
   // v_{k+1} = w / |w| (and its float4 copy)
   auto iteration = [&](int k) {
     product(V + (size_t)k * m, w);
     for (int pass = 0; pass < 2; pass++) {
       k_dots<<<dim3(nb, k + 1), kDotB, 0, st>>>(m, V, k + 1, w, part);
-      k_sub_proj_sum<<<cdivk(m, 128), 128, 0, st>>>(m, V, k + 1, nb, part, w, pass == 0 ? alpha + k : nullptr);
+      k_sub_proj_sum<<<nb2, 32 * kSubW, 0, st>>>(m, V, k + 1, nb, part, w, pass == 0 ? alpha + k : nullptr,
+                                            pass == 0 ? nullptr : nrm2);
     }
-    k_dots<<<dim3(nb, 1), kDotB, 0, st>>>(m, w, 1, w, part);
-    k_norm_scale<<<gb, tb, 0, st>>>(nD, nb, part, w, nrm, beta + k + 1, k + 1 < kmax ? V + (size_t)(k + 1) * m : nullptr,
+    k_norm_scale<<<gb, kNormB, 0, st>>>(nD, nb2, nrm2, w, nrm, beta + k + 1, k + 1 < kmax ? V + (size_t)(k + 1) * m : nullptr,
                                     xfm);
   };
   // a block of kCheck iterations is ~100 small launches: captured once per
