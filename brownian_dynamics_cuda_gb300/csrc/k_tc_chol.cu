@@ -14,7 +14,7 @@
 //                inverts the factor for the next launch.  A negative pivot is
 //                replaced by its absolute value and counted
 //                (func.cpp:827-833).
-//   update CTAs  trailing update A_IJ -= L_I L_J^T of up to eleven earlier
+//   update CTAs  trailing update A_IJ -= L_I L_J^T of up to six earlier
 //                panels, a run of tiles per CTA, warp-specialised:
 //                bulk-async operand copies, three FP16 products (lo.hi,
 //                hi.lo, hi.hi) per panel, up to three panels into one of
@@ -762,12 +762,13 @@ constexpr int kFoldPanels = 3;  // panels summed into one of them (K = 384): lon
 struct RestBars {
   uint64_t fullA, emptyA, fullB[2], emptyB[2], accFull[kAccs], accEmpty[kAccs], done;
 };
-// Panel slices: panel p in buffer p % bufs, buf bytes apart
+// Panel slices: panel p in buffer p % kBufs (a group's pass reads its panels' while
+// the next is written), buf bytes apart
+constexpr int kBufs = 7;
 struct Slices {
   const unsigned char* base;
   size_t buf;
-  int bufs;
-  __device__ __forceinline__ const unsigned char* at(int p) const { return base + (size_t)(p % bufs) * buf; }
+  __device__ __forceinline__ const unsigned char* at(int p) const { return base + (size_t)(p % kBufs) * buf; }
 };
 
 // Tile t of an update job's enumeration, from column jlo:
@@ -775,8 +776,8 @@ struct Slices {
 //   kBlkTri  the same by super-columns of kSuper tile columns, each row by row
 //            downward: the tiles in flight read the slices of 32 columns and a
 //            few dozen rows, where six panels' slices of a whole row of a large
-//            matrix are more than L2 holds (3N = 46,200: 142 MB; the
-//            factorisation takes 145 ms row by row, 139 so, 144 with 8 columns),
+//            matrix are more than L2 holds (3N = 46,200: 142 MB; a schedule that
+//            took 145 ms row by row took 139 so, 144 with 8 columns),
 //   kCol     column jlo alone (I = jlo + t).
 enum { kRowTri = 0, kCol = 1, kBlkTri = 2 };
 constexpr int kSuper = 32;
@@ -817,7 +818,7 @@ __device__ __forceinline__ void rest_tile(int t, int jlo, int mode, int nt, int&
 template <int NF>
 __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int lda, int m, int jlo, int mode,
                                           int tlo, int thi, int group, int cta, const Slices& sl, int p0, int npan,
-                                          int* err, float iscale2) {
+                                          int fold, int* err, float iscale2) {
   // (rounded as an integer, not by align1024: with the pointer known to be
   // shared the compiler places the epilogue's loads worse, 211 against 161 ms
   // for the factorisation at 3N = 46,200)
@@ -1012,7 +1013,7 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
           if (*abort_flag) break;
           const bool dg = I == J;
           for (int f = 0; f < NF && ok; f++, nacc++) {
-            const int q0 = 2 * kFoldPanels * f, q1 = min(q0 + 2 * kFoldPanels, 2 * npan), acc = nacc % kAccs;
+            const int q0 = 2 * fold * f, q1 = min(q0 + 2 * fold, 2 * npan), acc = nacc % kAccs;
             if (nacc >= kAccs) ok = sm100::mbar_wait(&bars->accEmpty[acc], (nacc / kAccs - 1) & 1, kWaitLimit);
             if (!ok) break;
             sm100::tc_fence_after();
@@ -1121,7 +1122,7 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
         const int s2 = c % kEpS;
 #pragma unroll
         for (int f = 0; f < kNF; f++) {
-          if (f > 0 && f * kFoldPanels >= npan) continue;
+          if (f > 0 && f * fold >= npan) continue;
           float v[kEpC];
           sm100::tmem_ld8(ta + f * kAccCols + kEpC * c, v);
 #pragma unroll
@@ -1152,9 +1153,9 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
 // An update job: tiles [tlo, thi) of an enumeration (rest_tile) from column
 // jlo, panels p0 .. p0 + npan - 1, `group` tiles per CTA.
 struct UpdJob {
-  int p0, npan, jlo, mode, tlo, thi, group, nctas;
+  int p0, npan, fold, jlo, mode, tlo, thi, group, nctas;
 };
-constexpr int kJobs = 3;
+constexpr int kJobs = 2;
 struct StepArgs {
   PanelArgs pan;  // panel k and the chain's tile
   int ntile;      // tile CTAs: tile rows k + 2 .. k + 1 + ntile
@@ -1185,10 +1186,10 @@ __device__ __forceinline__ void chol_step_body(const StepArgs& a, int b, float4*
   const PanelArgs& p = a.pan;
   auto run = [&](auto nf) {
     rest_body<decltype(nf)::value>(sm, p.A, p.lda, p.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b, a.sl, j.p0, j.npan,
-                                   p.err, p.iscale2);
+                                   j.fold, p.err, p.iscale2);
   };
-  if (j.npan > 2 * kFoldPanels) run(std::integral_constant<int, 4>{});
-  else if (j.npan > kFoldPanels) run(std::integral_constant<int, 2>{});
+  if (j.npan > 2 * j.fold) run(std::integral_constant<int, 4>{});
+  else if (j.npan > j.fold) run(std::integral_constant<int, 2>{});
   else if (j.npan > 1) run(std::integral_constant<int, 1>{});
   else run(std::integral_constant<int, 0>{});
 }
@@ -1224,22 +1225,25 @@ __global__ void __launch_bounds__(kRestThreads, 1) k_chol_step_multi(const StepA
 
 namespace bdk {
 
-// Panels per bulk pass while the trailing matrix is large (max_pass 3).  Six from
-// kWideTiles tile rows on: half the read-modify-writes of three (which with the
-// products' operands fill the SM's shared-memory and L1 path: 13 kcycles a tile
-// and three panels, 6 of them the products'), against column updates by up to
-// eleven panels.  3N = 46,200: 155 ms with three, 136 with six; 24,300: 27.2, 27.7;
-// 17,820: 12.4, 13.1.
-constexpr int kWideTiles = 256;
-static int group_of(int nt) { return nt >= kWideTiles ? 6 : 3; }
-// Slice buffers, panel p in buffer p % bufs: three panels' bulk update reads them
-// while the next is written; six panels' runs beside the next six.
-static int bufs_of(int nt) { return nt >= kWideTiles ? 12 : 4; }
+// Groups of panels that share one read-modify-write of the tiles right of them:
+// `fold` panels to an accumulator (K = 128 fold, summed in FP32 tensor memory: 3
+// while the trailing matrix is large, 2, then 1; at most max_pass), as many
+// accumulators a tile as kGroup says for that fold, each subtracted from the tile
+// by itself, so that the arithmetic is that of one pass per accumulator.  The
+// bulk is bound by the tiles' read-modify-write (their loads and stores share the
+// SM's L1 path with the products' operands, and HBM), the products alone would
+// take half; a group's column updates beside its panels cost less.  One
+// accumulator a pass: 3N = 11,700 5.04 ms, 24,300 27.2, 46,200 155, 24 fibers of
+// 1,992 to 7,836 together 14.9; so: 4.6, 21.7, 122, 11.6.  (Three accumulators of
+// three panels: 4.8 ms at 11,700; four of two: 11.0 and 4.7; the bulk of a group
+// spread over the next group's launches: 131 at 46,200.)
+constexpr int kGroup[4] = {0, 4, 3, 2};  // accumulators by fold
+constexpr int kGroupMin = 4;             // tile rows right of a group (fewer accumulators at the end)
+static_assert(kBufs > kGroup[1] && kBufs > 2 * kGroup[2] && kBufs > 3 * kGroup[3], "a group's panels and the next");
 // the slice buffers, then two buffers for the inverse of a diagonal factor
 // (W_k in buffer k & 1: read by the launch that writes W_k+1), then its factors
 size_t mixed_panel_bytes(int m) {
-  const int nt = cdiv(m, kT);
-  return (size_t)bufs_of(nt) * nt * kTileBytes + 2 * (size_t)kTileBytes + 2 * kT * sizeof(float);
+  return kBufs * (size_t)cdiv(m, kT) * kTileBytes + 2 * (size_t)kTileBytes + 2 * kT * sizeof(float);
 }
 int mixed_max_launches(int m) { return 2 * cdiv(m, kT) + 2; }
 int mixed_tiles(int m) { return cdiv(m, kT); }
@@ -1288,23 +1292,16 @@ static int rest_group(int tiles, int gmax) {
 // Right-looking with a lookahead of one panel, on one stream, no two kernels
 // at a time; every launch is one k_chol_step: panel k's tiles solved and
 // diagonal block k + 1 factored (the chain and tile CTAs, which apply panel
-// k - 1's update to column k themselves) beside up to three update jobs.  Panel
-// p's slices live in buffer p % bufs, W_p in buffer p & 1.  Invariant before
+// k - 1's update to column k themselves) beside up to two update jobs.  Panel
+// p's slices live in buffer p % kBufs, W_p in buffer p & 1.  Invariant before
 // the launch of panel k + 1: panels <= k are solved, column k + 1 and diagonal
 // block k + 2 hold the updates of panels < k, and the launch leaves diagonal
 // block k + 2 to its chain CTA (which applies panels k and k + 1).
-// Groups of g panels k .. k + g - 1 (1, 2, 3 or 6) share one read-modify-write of
-// the tiles right of them (K = 128 g), the more the larger the trailing matrix:
+// Groups of g panels k .. k + g - 1 (kGroup) share one read-modify-write of the
+// tiles right of them (K = 128 g):
 //   launch k + i, i = 1 .. g - 1: panel k + i beside panels k .. k + i - 1 on
 //     column k + i + 1 and on diagonal block k + i + 2;
 //   launch k + g: panel k + g beside the group on the tiles right of column k + g.
-// Groups of six: that last pass waits for the next group (b .. k - 1 the solved
-// one, k .. k + g - 1 the next):
-//   launch k + i, i = 0 .. g - 1: panel k + i beside panels b .. k + i - 1 on
-//     column k + i + 1 and diagonal block k + i + 2, and a g-th of the solved
-//     group's pass over the tiles right of column k + g;
-// so that the bulk is spread over all launches.  (With three the column updates
-// cost what the spreading gains: 4.97 and 4.99 ms at 3N = 11,700.)
 // Returns the number of kernel launches.
 #ifndef BD_PAIR_MIN
 #define BD_PAIR_MIN 24  // pair while at least this many tile rows remain right of column k+2 (k: last factored)
@@ -1312,12 +1309,9 @@ static int rest_group(int tiles, int gmax) {
 #ifndef BD_TRIPLE_MIN
 #define BD_TRIPLE_MIN 40  // three panels per bulk pass while this many tile rows remain right of column k+3
 #endif
-#ifndef BD_DEFER_MIN
-#define BD_DEFER_MIN 24  // a group's bulk runs beside the next group's panels while this many tile rows remain
-#endif
 namespace {
 struct Job {
-  int p0 = 0, npan = 0, jlo = 0, mode = kCol, tlo = 0, tiles = 0, group = 1;  // tiles: the enumeration's end
+  int p0 = 0, npan = 0, fold = 1, jlo = 0, mode = kCol, tlo = 0, tiles = 0, group = 1;  // tiles: the enumeration's end
 };
 }  // namespace
 
@@ -1335,9 +1329,8 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
   const size_t buf = (size_t)nt * kTileBytes;
   int L = 0, timed = 0;
   auto kb_of = [&](int k) { return (m - k * kT < kT) ? m - k * kT : kT; };
-  const int bufs = bufs_of(nt);
-  auto psb = [&](int k) { return PS + (size_t)(k % bufs) * buf; };
-  unsigned char* Wb = PS + bufs * buf;  // the inverses' slices
+  auto psb = [&](int k) { return PS + (size_t)(k % kBufs) * buf; };
+  unsigned char* Wb = PS + kBufs * buf;  // the inverses' slices
   float* wsc = reinterpret_cast<float*>(Wb + 2 * (size_t)kTileBytes);
   // elements of the lower triangle in tile columns [j0, j1)
   auto elems = [&](int j0, int j1) {
@@ -1349,27 +1342,27 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
     return e;
   };
   // panels p .. p + npan - 1 on column J below its diagonal block (the chain CTA's)
-  auto col_job = [&](int p, int J, int npan = 1) {
+  auto col_job = [&](int p, int J, int npan, int fold) {
     Job j;
-    j.p0 = p, j.npan = npan, j.jlo = J, j.mode = kCol, j.tlo = 1, j.tiles = nt - J;
+    j.p0 = p, j.npan = npan, j.fold = fold, j.jlo = J, j.mode = kCol, j.tlo = 1, j.tiles = nt - J;
     return j;
   };
-  auto diag_job = [&](int p, int J, int npan = 1) {  // ... on diagonal block J alone
+  auto diag_job = [&](int p, int J, int npan, int fold) {  // ... on diagonal block J alone
     Job j;
-    j.p0 = p, j.npan = npan, j.jlo = J, j.mode = kCol, j.tiles = J < nt ? 1 : 0;
+    j.p0 = p, j.npan = npan, j.fold = fold, j.jlo = J, j.mode = kCol, j.tiles = J < nt ? 1 : 0;
     return j;
   };
-  // ... on part `part` of `parts` of the triangle from column jlo but its first diagonal block
-  auto tri_job = [&](int p, int npan, int jlo, int part = 0, int parts = 1) {
+  // ... on the triangle from column jlo but its first diagonal block
+  auto tri_job = [&](int p, int npan, int fold, int jlo) {
     Job j;
-    const long n = nt - jlo, all = n > 0 ? n * (n + 1) / 2 - 1 : 0;
-    j.p0 = p, j.npan = npan, j.jlo = jlo, j.mode = npan > kFoldPanels ? kBlkTri : kRowTri;
-    j.tlo = 1 + (int)(all * part / parts), j.tiles = 1 + (int)(all * (part + 1) / parts);
-    j.group = rest_group(j.tiles - j.tlo, npan > kFoldPanels ? 4 : BD_REST_GMAX);
+    const int n = nt - jlo;
+    j.p0 = p, j.npan = npan, j.fold = fold, j.jlo = jlo, j.mode = npan > kFoldPanels ? kBlkTri : kRowTri, j.tlo = 1;
+    j.tiles = n > 0 ? n * (n + 1) / 2 : 0;
+    j.group = rest_group(j.tiles, npan > kFoldPanels ? 4 : BD_REST_GMAX);
     return j;
   };
   // panel k's tiles (k < 0: none) and diagonal block k + 1
-  auto launch = [&](int k, const Job& j0, const Job& j1 = Job(), const Job& j2 = Job()) {
+  auto launch = [&](int k, const Job& j0, const Job& j1 = Job()) {
     StepArgs a{};
     PanelArgs& p = a.pan;
     p.A = A, p.lda = lda, p.m = m, p.k = k, p.tile = k < 0 ? -1 : k + 1;
@@ -1378,13 +1371,13 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
     p.Wn = Wb + (size_t)((k + 1) & 1) * kTileBytes, p.wscn = wsc + kT * ((k + 1) & 1);
     p.negpiv = negpiv, p.err = err, p.scale = scale, p.iscale2 = 1.f / (scale * scale);
     a.ntile = k < 0 ? 0 : nt - k - 2;
-    a.sl = Slices{PS, buf, bufs};
-    const Job* js[kJobs] = {&j0, &j1, &j2};
+    a.sl = Slices{PS, buf};
+    const Job* js[kJobs] = {&j0, &j1};
     int grid = 1 + a.ntile;
     for (int q = 0; q < kJobs; q++) {
       const Job& j = *js[q];
       UpdJob& u = a.job[q];
-      u.p0 = j.p0, u.npan = j.npan, u.jlo = j.jlo, u.mode = j.mode, u.tlo = j.tlo, u.thi = j.tiles, u.group = j.group;
+      u.p0 = j.p0, u.npan = j.npan, u.fold = j.fold, u.jlo = j.jlo, u.mode = j.mode, u.tlo = j.tlo, u.thi = j.tiles, u.group = j.group;
       u.nctas = j.tiles > j.tlo ? cdiv(j.tiles - j.tlo, j.group) : 0;
       grid += u.nctas;
     }
@@ -1406,9 +1399,7 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
       for (int q = 0; q < kJobs; q++) {
         const Job& j = *js[q];
         if (j.tiles <= j.tlo) continue;
-        const double all = nt - j.jlo;  // a part of the triangle: its share of the elements
-        by += 16.0 * (j.mode == kCol ? (j.tiles == 1 ? 0.5 * kT * kb_of(j.jlo) : elems(j.jlo, j.jlo + 1))
-                                     : elems(j.jlo, nt) * (j.tiles - j.tlo) / (0.5 * all * (all + 1)));
+        by += 16.0 * (j.tiles == 1 ? 0.5 * kT * kb_of(j.jlo) : elems(j.jlo, j.mode == kCol ? j.jlo + 1 : nt));
         fl += tile_fl * (j.tiles - j.tlo) * j.npan;  // FP16 tensor work issued
       }
       if (kbytes) *kbytes += by;
@@ -1417,22 +1408,16 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
   };
   launch(-1, Job());             // diagonal block 0
   if (nt > 1) launch(0, Job());  // panel 0
-  const int G = group_of(nt);
   int k = 0;
   while (k + 2 < nt) {
-    const int g = max_pass >= 3 && nt - (k + 1 + G) >= BD_TRIPLE_MIN ? G
-                  : max_pass >= 2 && nt - (k + 3) >= BD_PAIR_MIN     ? 2
-                                                                     : 1;
-    for (int i = 1; i < g; i++) launch(k + i, col_job(k, k + i + 1, i), diag_job(k, k + i + 2, i));
-    int b = k;
-    k += g;  // panels b .. k - 1 are solved, their update right of column k is not made
-    while (g > kFoldPanels && nt - (k + g + 1) >= BD_DEFER_MIN) {
-      for (int i = 0; i < g; i++)
-        launch(k + i, col_job(b, k + i + 1, g + i), diag_job(b, k + i + 2, g + i), tri_job(b, g, k + g + 1, i, g));
-      b = k;
-      k += g;
-    }
-    launch(k, tri_job(b, g, k + 1));
+    const int fold = max_pass >= 3 && nt - (k + 4) >= BD_TRIPLE_MIN ? 3
+                     : max_pass >= 2 && nt - (k + 3) >= BD_PAIR_MIN ? 2
+                                                                    : 1;
+    int g = fold * kGroup[fold];
+    while (g > fold && nt - (k + 1 + g) < kGroupMin) g -= fold;
+    for (int i = 1; i < g; i++) launch(k + i, col_job(k, k + i + 1, i, fold), diag_job(k, k + i + 2, i, fold));
+    launch(k + g, tri_job(k, g, fold, k + g + 1));
+    k += g;
   }
   if (plan) return L;
   if (kev_pairs) *kev_pairs = timed;

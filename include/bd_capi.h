@@ -323,11 +323,12 @@ int bd_batch_phase_times(bd_batch* b, float* out3);
  * launches).  No counterpart in the reference. */
 int bd_batch_launch_count(const bd_batch* b, int* out);
 /* Accuracy/speed setting of the mixed factorisation: at most `passes` (1, 2
- * or 3; default 3) panels per trailing read-modify-write pass.  Each pass
- * accumulates its panels' products in FP32 tensor memory before adding them
- * to the double-float tensor, so fewer panels per pass give a more accurate
- * factor at more HBM traffic (measured at 3N = 11,700: 3 -> 6.9 ms, noise
- * displacement 7.8e-7 from FP64; 2 -> 7.3 ms, 6.3e-7; 1 -> 9.4 ms, 5.4e-7).
+ * or 3; default 3) panels per accumulator of the trailing update.  Each
+ * accumulator sums its panels' products in FP32 tensor memory before they are
+ * added to the double-float tensor (up to four accumulators in one pass over
+ * it), so fewer panels each give a more accurate factor at more work to add
+ * them (measured at 3N = 11,700: 3 -> 4.5 ms, noise displacement 6.9e-7 from
+ * FP64; 2 -> 5.0 ms, 5.8e-7; 1 -> 5.7 ms, 5.0e-7).
  * The next step captures its graph again.  No counterpart in the reference
  * (its factorisation is FP64 cuSOLVER). */
 int bd_set_mixed_passes(bd_ctx* ctx, int passes);
