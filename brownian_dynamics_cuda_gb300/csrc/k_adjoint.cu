@@ -739,54 +739,62 @@ __global__ void __launch_bounds__(64) k_inv_leaf(int mp, const R* __restrict__ U
 
 // C = alpha A op(B) (row-major; op(B) = B or B^T), M, N, K multiples of 64;
 // gridDim.z independent products with operands zstride elements apart.
-// kmode restricts the k range of each 64 x 64 output tile (r0, c0) to
+// kmode restricts the k range of each T x T output tile (r0, c0) to
 // the nonzero band of triangular operands: 1: k >= r0, 2: k >= c0,
-// 4: k < c0 + 64.
-constexpr int kGT = 64, kGK = 16;
+// 4: k < c0 + T.  FP64: 32 x 32 tiles, bound by the FP64 pipe - a 64 x 64 one of
+// K = 1,024 holds an SM's for 1.1 ms, and the products' bands give the tiles very
+// unequal K (order 1,024: 1,480 us the last product, 277 a level's; 801 and 113 with
+// 32).  FP32: 64 x 64, four times the operands' reuse.
+constexpr int kGK = 16;
+template <class R>
+constexpr int kGT = sizeof(R) == 8 ? 32 : 64;
+template <class R>
+constexpr int kGN = sizeof(R) == 8 ? 2 : 4;  // columns a thread (and four rows)
+template <class R>
+constexpr int kGThreads = kGT<R> * kGT<R> / (4 * kGN<R>);
 template <class R, bool TB>
-__global__ void __launch_bounds__(256) k_gemm(int K, R alpha, const R* __restrict__ A, int lda,
+__global__ void __launch_bounds__(kGThreads<R>) k_gemm(int K, R alpha, const R* __restrict__ A, int lda,
                                               const R* __restrict__ B, int ldb, R* C, int ldc, int kmode,
                                               long zstride) {
-  const int r0 = blockIdx.y * kGT, c0 = blockIdx.x * kGT;
+  constexpr int T = kGT<R>, NC = kGN<R>, NT = kGThreads<R>;
+  const int r0 = blockIdx.y * T, c0 = blockIdx.x * T;
   A += blockIdx.z * zstride;  // batch item z: every operand shifted by z * zstride elements
   B += blockIdx.z * zstride;
   C += blockIdx.z * zstride;
   int kb = 0, ke = K;
   if (kmode & 1) kb = max(kb, r0);
   if (kmode & 2) kb = max(kb, c0);
-  if (kmode & 4) ke = min(ke, c0 + kGT);
-  __shared__ R As[kGK][kGT + 4];
-  __shared__ R Bs[kGK][kGT + 4];
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  R acc[4][4];
+  if (kmode & 4) ke = min(ke, c0 + T);
+  __shared__ R As[kGK][T + 4];
+  __shared__ R Bs[kGK][T + 4];
+  const int tx = threadIdx.x % (T / NC), ty = threadIdx.x / (T / NC);
+  R acc[4][NC];
   for (int u = 0; u < 4; u++)
-    for (int v = 0; v < 4; v++) acc[u][v] = R(0);
+    for (int v = 0; v < NC; v++) acc[u][v] = R(0);
   for (int k0 = kb; k0 < ke; k0 += kGK) {
-    for (int e = threadIdx.x; e < kGT * kGK; e += 256) {
+    for (int e = threadIdx.x; e < T * kGK; e += NT) {
       const int rr = e / kGK, kk = e % kGK;
       As[kk][rr] = A[(size_t)(r0 + rr) * lda + k0 + kk];
       if (TB) {
         Bs[kk][rr] = B[(size_t)(c0 + rr) * ldb + k0 + kk];
       } else {
-        const int k2 = e / kGT, cc = e % kGT;
+        const int k2 = e / T, cc = e % T;
         Bs[k2][cc] = B[(size_t)(k0 + k2) * ldb + c0 + cc];
       }
     }
     __syncthreads();
 #pragma unroll
     for (int kk = 0; kk < kGK; kk++) {
-      R a[4], b[4];
-      for (int u = 0; u < 4; u++) {
-        a[u] = As[kk][ty * 4 + u];
-        b[u] = Bs[kk][tx * 4 + u];
-      }
+      R a[4], b[NC];
+      for (int u = 0; u < 4; u++) a[u] = As[kk][ty * 4 + u];
+      for (int v = 0; v < NC; v++) b[v] = Bs[kk][tx * NC + v];
       for (int u = 0; u < 4; u++)
-        for (int v = 0; v < 4; v++) acc[u][v] += a[u] * b[v];
+        for (int v = 0; v < NC; v++) acc[u][v] += a[u] * b[v];
     }
     __syncthreads();
   }
   for (int u = 0; u < 4; u++)
-    for (int v = 0; v < 4; v++) C[(size_t)(r0 + ty * 4 + u) * ldc + c0 + tx * 4 + v] = alpha * acc[u][v];
+    for (int v = 0; v < NC; v++) C[(size_t)(r0 + ty * 4 + u) * ldc + c0 + tx * NC + v] = alpha * acc[u][v];
 }
 
 // Xt[c][i] = s2dt u_i (sum_{j<=i} p_j V[c][j] - p_i V[c][i] / 2): row c of
@@ -826,9 +834,9 @@ __global__ void __launch_bounds__(256) k_build_xt(int m, int mp, const R* __rest
 template <class R>
 int gemm(cudaStream_t st, int M_, int N_, int K_, R alpha, const R* A, int lda, const R* B, int ldb, R* C, int ldc,
          bool tb, int kmode, int batch = 1, long zstride = 0) {
-  dim3 grid(N_ / kGT, M_ / kGT, batch);
-  if (tb) k_gemm<R, true><<<grid, 256, 0, st>>>(K_, alpha, A, lda, B, ldb, C, ldc, kmode, zstride);
-  else k_gemm<R, false><<<grid, 256, 0, st>>>(K_, alpha, A, lda, B, ldb, C, ldc, kmode, zstride);
+  dim3 grid(N_ / kGT<R>, M_ / kGT<R>, batch);
+  if (tb) k_gemm<R, true><<<grid, kGThreads<R>, 0, st>>>(K_, alpha, A, lda, B, ldb, C, ldc, kmode, zstride);
+  else k_gemm<R, false><<<grid, kGThreads<R>, 0, st>>>(K_, alpha, A, lda, B, ldb, C, ldc, kmode, zstride);
   return 0;
 }
 
