@@ -568,6 +568,14 @@ extern "C" int bd_create(const bd_model* m, const bd_state* s, const bd_options*
   return BD_OK;
 }
 
+static void side_free(bd_ctx* c) {
+  for (auto ev : c->side.e)
+    if (ev) cudaEventDestroy(ev);
+  for (auto s : c->side.s)
+    if (s) cudaStreamDestroy(s);
+  c->side = bdk::Side();
+}
+
 extern "C" int bd_destroy(bd_ctx* c) {
   if (!c) return BD_OK;
   if (c->stream) cudaStreamSynchronize(c->stream);
@@ -582,10 +590,7 @@ extern "C" int bd_destroy(bd_ctx* c) {
   c->kgraphs.clear();
   if (c->kscratch) cudaFree(c->kscratch);
   if (c->arena_base) cudaFree(c->arena_base);
-  for (auto ev : c->side.e)
-    if (ev) cudaEventDestroy(ev);
-  for (auto s : c->side.s)
-    if (s) cudaStreamDestroy(s);
+  side_free(c);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return BD_OK;
@@ -679,7 +684,7 @@ extern "C" int bd_step_reference(bd_ctx* c, int step, int number_of_steps, int f
 
 extern "C" int bd_forces(bd_ctx* c, double* F, double* T, double* tF, double* lF, double* E) {
   if (!c) return set_error(BD_ERR_ARG, "bd_forces: null context");
-  bdk::forces(c->M, c->X, c->F0, c->S, c->precision, c->stream, &c->side);
+  bdk::forces(c->M, c->X, c->F0, c->S, c->precision, c->stream, c->in_batch ? nullptr : &c->side);
   CK(cudaGetLastError());
   cudaStream_t st = c->stream;
   size_t n3 = 3 * (size_t)c->M.n;
@@ -1070,6 +1075,7 @@ extern "C" int bd_batch_create(int nrep, const bd_model* models, const bd_state*
       return rc;
     }
     c->in_batch = true;
+    side_free(c);  // replicas run beside each other on the batch's own side streams
     b->ctx.push_back(c);
   }
   *out = b;

@@ -1289,8 +1289,8 @@ static int rest_group(int tiles, int gmax) {
   return g < BD_REST_GMIN ? BD_REST_GMIN : (g > gmax ? gmax : g);
 }
 
-// Right-looking with a lookahead of one panel, on one stream, no two kernels
-// at a time; every launch is one k_chol_step: panel k's tiles solved and
+// Right-looking with a lookahead of one panel, on one stream, one launch
+// after the other; every launch is one k_chol_step: panel k's tiles solved and
 // diagonal block k + 1 factored (the chain and tile CTAs, which apply panel
 // k - 1's update to column k themselves) beside up to two update jobs.  Panel
 // p's slices live in buffer p % kBufs, W_p in buffer p & 1.  Invariant before

@@ -49,7 +49,7 @@ enum {
                          FP32 panels and FP16-pair tensor-core (tcgen05) trailing updates, FP32
                          pair forces with compensated sums; no refinement.  Displacement
                          4e-7 to 8e-7 from the FP64 path on the benchmark fibers; up to
-                         1.3e-6 on 3 of 256 uneven batch replicas (bd_set_mixed_passes) */
+                         1.2e-6 on 2 of 256 uneven batch replicas (bd_set_mixed_passes) */
 };
 
 /* Noise displacement of a step (bd_set_noise_mode). */
