@@ -403,7 +403,7 @@ def run_ours(args):
                 "traffic_source": "DRAM read+write per algorithmic byte of one ncu capture "
                                   "of k_chol_step at 3N = 11,700, times this step's algorithmic bytes",
                 "kernel": "k_chol_step (every launch of the mixed factorisation: next panel in its own CTAs beside "
-                          "tcgen05 column and bulk trailing updates of one or two panels, double-float tile "
+                          "tcgen05 column and bulk trailing updates of up to six panels, double-float tile "
                           "read-modify-write), %d launches/step, avg %.3f ms" % (nk, ms_k / max(nk, 1)),
                 "algorithmic_bytes_per_step": byt,
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)",
@@ -460,11 +460,11 @@ def run_ours(args):
 
 def mixed_schedule_bytes(m: int, kT: int = 128, triple_min: int = 40, pair_min: int = 24) -> float:
     """Algorithmic HBM bytes of one mixed factorisation of a 3N = m tensor: the
-    schedule of bdk::potrf_mixed (one launch per panel; three panels per bulk
-    pass while 40 tile rows remain, two while 24 do), 16 B (double-float read +
-    write) per element of the panel's column and of every trailing tile a bulk
-    pass updates.  Equals the library's own count (bd_kernel_bytes; 12.70 GB at
-    3N = 11,700)."""
+    schedule of bdk::potrf_mixed (one launch per panel; groups of two triples of
+    panels a bulk pass while 40 tile rows remain, three pairs while 24 do, then
+    four single panels), 16 B (double-float read + write) per element of the
+    panel's column and of every tile an update job changes.  Equals the library's
+    own count (bd_kernel_bytes)."""
     nt = -(-m // kT)
     kb = lambda k: m - k * kT if m - k * kT < kT else kT  # noqa: E731
 
@@ -477,29 +477,28 @@ def mixed_schedule_bytes(m: int, kT: int = 128, triple_min: int = 40, pair_min: 
 
     total = 0.0
 
-    def launch(pn, jobs):
+    def launch(k, jobs):
         nonlocal total
-        total += 16.0 * (m - pn * kT) * kb(pn)
-        for mode, jlo in jobs:
-            n = nt - jlo
-            if n > 0:
-                total += 16.0 * elems(jlo, jlo + 1 if mode == "col" else nt)
+        total += 16.0 * (m - (k + 1) * kT) * (kb(0) if k < 0 else kT)
+        for mode, J in jobs:
+            if mode == "diag":
+                total += 8.0 * kT * kb(J) if J < nt else 0.0
+            elif nt - J > 1:
+                total += 16.0 * elems(J, J + 1 if mode == "col" else nt)
 
-    launch(0, [])
+    launch(-1, [])
+    if nt > 1:
+        launch(0, [])
     k = 0
-    while k + 1 < nt:
-        if nt - (k + 4) >= triple_min:
-            launch(k + 1, [("col", k + 2)])
-            launch(k + 2, [("col", k + 3)])
-            launch(k + 3, [("tri", k + 4)])
-            k += 3
-        elif nt - (k + 3) >= pair_min:
-            launch(k + 1, [("col", k + 2)])
-            launch(k + 2, [("tri", k + 3)])
-            k += 2
-        else:
-            launch(k + 1, [("tri", k + 2)])
-            k += 1
+    while k + 2 < nt:
+        fold = 3 if nt - (k + 4) >= triple_min else 2 if nt - (k + 3) >= pair_min else 1
+        g = fold * {1: 4, 2: 3, 3: 2}[fold]
+        while g > fold and nt - (k + 1 + g) < 4:
+            g -= fold
+        for i in range(1, g):
+            launch(k + i, [("col", k + i + 1), ("diag", k + i + 2)])
+        launch(k + g, [("tri", k + g + 1)])
+        k += g
     return total
 
 
@@ -507,7 +506,7 @@ def batch_fp64_comparison(fibers, host, d_rr, d_p, local, stream, passes_list=(3
     """The plain FP64 GPU step on the same replicas and noise: one FP64 batch
     step from the start states (its displacements kept), two timed FP64 batch
     steps (CUDA graph, CUDA events); then, for each mixed schedule (at most
-    `passes` panels per trailing pass; 3 is the default), one mixed batch step
+    `passes` panels per accumulator; 3 is the default), one mixed batch step
     from the same start states — every replica's relative displacement error
     max |dr_mixed - dr_fp64| / max |dr_fp64| over r, r_t, r_lh — and two timed
     mixed steps of that schedule."""
