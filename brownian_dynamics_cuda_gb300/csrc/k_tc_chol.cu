@@ -8,7 +8,7 @@
 // kernel, k_chol_step, runs these kinds of CTA side by side:
 //   panel CTAs   solve panel k's tiles, L_ik = A_ik L_kk^-T, write them back
 //                and split them into two FP16 slices (scaled by one power of
-//                two: hi + lo = the FP32 value to 2^-24), stored pre-swizzled
+//                two: hi + lo = the FP32 value to 2^-23), stored pre-swizzled
 //                in the 128-byte-swizzle K-major layout the MMA reads; one of
 //                them, the chain CTA, then factors diagonal block k + 1 and
 //                inverts the factor for the next launch.  A negative pivot is
@@ -20,18 +20,19 @@
 //                hi.lo, hi.hi) per panel, up to three panels into one of
 //                four FP32 tensor-memory accumulators (tcgen05.mma, M = N = 128, K = 16 per
 //                instruction), tcgen05.ld epilogue subtracting into the
-//                double-float tile.  The dropped product lo.lo is below
-//                2^-24 of the kept ones: FP32-class products.
+//                double-float tile.  The dropped product lo.lo is at most
+//                2^-22 of hi.hi (both values half way between two FP16 ones).
 // Two FP16 slices and three products instead of three BF16 slices and six
 // (which hold the FP32 value exactly): half the tensor work, two thirds of
 // the operand bytes.  3N = 11,700: 7.0 -> 6.1 ms; 3N = 46,200: 202 -> 157 ms.
 // Error of L p against FP64 (2-norm, 13 fibers of 3N 912 .. 11,700):
 // 2.6e-7 .. 5.4e-7 before, 2.6e-7 .. 5.1e-7 now - the sums inside the tensor
-// core set it, not the split.
+// core set it, not the split: FP32-class by that measurement.
 // The launches run on one stream, one at a time (the schedule is at
 // potrf_mixed).  Every mbarrier wait is bounded; on a timeout the kernel
 // records an error code, frees its tensor memory and returns.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <type_traits>
 #include <utility>
@@ -54,6 +55,8 @@ constexpr int kHalfBytes = kSliceBytes / 2;
 constexpr int kTileSlices = 2;
 constexpr int kTileBytes = kTileSlices * kSliceBytes;  // 64 KB per 128-row panel tile
 constexpr uint32_t kWaitLimit = 1u << 24;
+// panel p's slices are in buffer p % kBufs: a group's pass reads its panels' while the next is written
+constexpr int kBufs = 7;
 
 inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 __device__ __forceinline__ int cdiv_d(int a, int b) { return (a + b - 1) / b; }
@@ -64,18 +67,40 @@ __device__ __forceinline__ uint32_t swz_off(int r, int k) {
   return half * kHalfBytes + (r >> 3) * 1024 + (r & 7) * 128 + ((((kk >> 3) ^ (r & 7)) & 7) << 4) + (kk & 7) * 2;
 }
 
-// Two scaled FP32 values as FP16 pairs: x = hi + lo to 2^-24 |x| (two
-// roundings to 11 bits each), low half first.  Values past FP16's range (a
-// factor with replaced negative pivots, see mixed_scale) saturate; NaN stays.
+// Two scaled FP32 values as FP16 pairs: x = hi + lo to 2^-23 |x| (two
+// roundings to 11 bits each), low half first.  A value past FP16's range makes
+// hi infinite and the products NaN: never a finite, wrong factor (see Range).
 __device__ __forceinline__ uint32_t cvt_f16x2(float x0, float x1) {
   uint32_t r;
-  asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(x1), "f"(x0));
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(x1), "f"(x0));
   return r;
 }
 __device__ __forceinline__ void split_f16x2(float x0, float x1, uint32_t& hi, uint32_t& lo) {
   hi = cvt_f16x2(x0, x1);
   const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&hi));
   lo = cvt_f16x2(x0 - hf.x, x1 - hf.y);
+}
+
+// Range.  The slices' common scale (mixed_scale) fits every positive definite
+// tensor.  An indefinite one (its negative pivots are replaced by |f|,
+// func.cpp:827-833) can grow past FP16's range at any row: such a row of a
+// tile gets a power of two of its own, from its largest value (rows that fit
+// keep the common one), so that slices hold whatever FP32 does.  `top`: the
+// largest |hi| of the values split, NaN if one is; past(top): one of them does
+// not fit.
+__device__ __forceinline__ void keep_top(uint32_t& top, uint32_t hi) {
+  const __half2 a = __hmax2_nan(*reinterpret_cast<const __half2*>(&top), __habs2(*reinterpret_cast<const __half2*>(&hi)));
+  top = *reinterpret_cast<const uint32_t*>(&a);
+}
+__device__ __forceinline__ bool past(uint32_t top) { return (top & 0x7fffu) >= 0x7c00u || (top >> 16) >= 0x7c00u; }
+// The power of two that puts m into [2^13, 2^14), and its inverse; false (m
+// zero, infinite or NaN, or the power past 2^+-100): neither is set.
+__device__ __forceinline__ bool own_scale(float m, float& up, float& down) {
+  const int e = 13 + 127 - (int)(__float_as_uint(m) >> 23);
+  if (!(m > 0.f) || isinf(m) || e > 100 || e < -100) return false;
+  up = __uint_as_float((uint32_t)(127 + e) << 23);
+  down = __uint_as_float((uint32_t)(127 - e) << 23);
+  return true;
 }
 
 // (hi, lo) - v in double-float arithmetic: exact two-sums (Knuth), so the
@@ -122,7 +147,12 @@ static_assert(kChainS + kT * kLd * 4 <= kChainW, "the diagonal block lies before
 struct PanelBars {
   uint64_t fullPre, fullW, preDone, sReady, xDone, lReady, qDone, r0Free, trDone[3], trRest[2], helped[2], step[16];
   uint32_t slot;
+  int again, failed;                 // some value does not fit the common scale; some wait ran out
+  int lown, rown;                    // some row of L_ik, of a rank-32 product, has a scale of its own
+  float rmax[2][kT];                 // a row's largest value, by column half
+  float lrow[kT];                    // common scale / the row's own (L_ik)
   float rowf[2][kT];                 // undoes the scales of a row's rank-32 product (panel P in buffer P & 1)
+  float colf[2][kT];                 // ... as a column of it: common scale / the row's own
   alignas(16) float xsc[kT];         // X = D * xsc, by column
   alignas(16) float dg[16][8][8];    // the 8 x 8 diagonal blocks, then L's
 };
@@ -156,10 +186,13 @@ __device__ __forceinline__ void mma_tile(uint32_t d, const unsigned char* sa, co
 }
 
 // 8 consecutive columns (from column c, c % 8 == 0) of row r of a slice pair at `base`
-__device__ __forceinline__ void put_slices8(unsigned char* base, int r, int c, const float (&x)[8]) {
+__device__ __forceinline__ void put_slices8(unsigned char* base, int r, int c, const float (&x)[8], uint32_t& top) {
   uint32_t h[4], l[4];
 #pragma unroll
-  for (int j = 0; j < 4; j++) split_f16x2(x[2 * j], x[2 * j + 1], h[j], l[j]);
+  for (int j = 0; j < 4; j++) {
+    split_f16x2(x[2 * j], x[2 * j + 1], h[j], l[j]);
+    keep_top(top, h[j]);
+  }
   const uint32_t off = swz_off(r, c);
   *reinterpret_cast<uint4*>(base + off) = make_uint4(h[0], h[1], h[2], h[3]);
   *reinterpret_cast<uint4*>(base + kSliceBytes + off) = make_uint4(l[0], l[1], l[2], l[3]);
@@ -271,17 +304,23 @@ __device__ __forceinline__ void chol_inv128(float (*S)[kLd], PanelBars* bars, un
           for (int j = 0; j < 24; j++)
             if (j < (lane & 24)) x[j] = 0.f;
         }
-        if ((r >> 5) <= P) {
-          float m[4] = {0.f, 0.f, 0.f, 0.f};
+        float m[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-          for (int j = 0; j < 32; j++) m[j & 3] = fmaxf(m[j & 3], fabsf(x[j]));
-          m[0] = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
-          int e = 13 + 127 - (int)(__float_as_uint(m[0]) >> 23);
-          if (!(m[0] > 0.f) || isinf(m[0]) || e > 100 || e < -100) e = 0;
-          rho = __uint_as_float((uint32_t)(127 + e) << 23);
-          f = __uint_as_float((uint32_t)(127 - e) << 23) * iscale;
+        for (int j = 0; j < 32; j++) m[j & 3] = fmaxf(m[j & 3], fabsf(x[j]));
+        m[0] = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+        float up = 1.f, down = 1.f, cf = 1.f;
+        const bool set = own_scale(m[0], up, down);
+        if ((r >> 5) <= P) {
+          rho = up;
+          f = down * iscale;
+        } else if (m[0] * scale >= 32768.f && set) {  // a row of L past FP16's range
+          rho = up;
+          f = down * iscale;
+          cf = scale * down;
+          bars->rown = 1;
         }
         bars->rowf[P & 1][r] = f;  // (the buffer's last readers are done: helped[P - 2])
+        bars->colf[P & 1][r] = cf;
       }
       asm volatile("bar.sync 2, 128;" ::: "memory");
       if (lane == 0 && (r >> 5) == 0) {
@@ -339,10 +378,15 @@ __device__ __forceinline__ void chol_inv128(float (*S)[kLd], PanelBars* bars, un
       }
     }
     __syncwarp();
+    const bool own = bars->rown;
     ok = sm100::mbar_wait(&bars->trDone[P], 0, kWaitLimit) && ok;
     sm100::tc_fence_after();
     float v[32];
     sm100::tmem_ld32(trow, v);
+    if (own) {
+#pragma unroll
+      for (int j = 0; j < 32; j++) v[j] *= bars->colf[P & 1][32 * (P + 1) + j];
+    }
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       const float4 o = *reinterpret_cast<const float4*>(&S[r][32 * (P + 1) + 4 * j]);
@@ -366,6 +410,10 @@ __device__ __forceinline__ void chol_help(float (*S)[kLd], PanelBars* bars, uint
   for (int c = 0; c < 64 - 32 * P; c += 16) {
     float v[16];
     sm100::tmem_ld16(trow + 32 + c, v);
+    if (bars->rown) {
+#pragma unroll
+      for (int j = 0; j < 16; j++) v[j] *= bars->colf[P & 1][32 * (P + 2) + c + j];
+    }
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       float4* o = reinterpret_cast<float4*>(&S[r][32 * (P + 2) + c + 4 * j]);
@@ -421,15 +469,15 @@ __device__ __forceinline__ void chain_store_w(const float (*S)[kLd], PanelBars* 
   }
   m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
   m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
-  int e = 13 + 127 - (int)(__float_as_uint(m) >> 23);
-  if (!(m > 0.f) || isinf(m) || e > 100 || e < -100) e = 0;
-  const float sc = __uint_as_float((uint32_t)(127 + e) << 23);
+  float sc = 1.f, isc = 1.f;
+  (void)own_scale(m, sc, isc);
   if (jc == 0) wscn[row] = 1.f / (cs * sc);
+  uint32_t top = 0;  // (scaled by its own maximum: nothing to see)
 #pragma unroll
   for (int t = 0; t < 4; t++) {
 #pragma unroll
     for (int j = 0; j < 8; j++) x[t][j] *= sc;
-    put_slices8(Wo, row, 8 * (jc + 4 * t), x[t]);
+    put_slices8(Wo, row, 8 * (jc + 4 * t), x[t], top);
   }
   sm100::fence_proxy_async();
   __syncwarp();
@@ -452,8 +500,136 @@ struct PanelArgs {
   float* wscn;
   int* negpiv;
   int* err;
+  int* past;                      // [0] the first panel with rows whose scales are their own, [1 + p] panel p is such
+  float* rowk;                    // [nt kT] the common scale / the row's own, of panel k ...
+  const float* rowp;              // ... and of panel k - 1
   float scale, iscale2;
 };
+
+// whether p holds in either of the two warps that share 32 rows (q)
+__device__ __forceinline__ bool pair_any(int q, bool p) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred a, b;\n\t"
+      "setp.ne.u32 a, %1, 0;\n\t"
+      "barrier.cta.red.or.pred b, %2, 64, a;\n\t"
+      "selp.u32 %0, 1, 0, b;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)p), "r"(4 + q)
+      : "memory");
+  return r != 0;
+}
+
+// The 32 rows of warps q where a row of the tile, or of L_ik, does not fit the
+// slices' common scale (the product is then infinite or NaN), or panel k - 1 has
+// rows with scales of their own: the tile less that panel's update, then L_ik by
+// forward substitution in FP32, in A.  Such a row's values can lie further apart
+// than a pair's 40 bits: no one scale holds them, and the product with the
+// inverse would lose the small ones.
+__device__ __forceinline__ void solve_rows(const PanelArgs& p, int q, int ch, int r, bool pre, uint32_t trow) {
+  const bool in = p.tile * kT + r < p.m;
+  float2* row = p.A + (size_t)(p.k * kT) * p.lda + p.tile * kT + r;
+  const float2* L = p.A + (size_t)(p.k * kT) * p.lda + p.k * kT;
+#pragma unroll 1
+  for (int c = 0; c < 64; c += 8) {
+    float v[8];
+    if (pre) sm100::tmem_ld8(trow + c, v);
+    if (in) {
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        float2* a = row + (size_t)(64 * ch + c + j) * p.lda;
+        const float2 o = *a;
+        const float f = pre ? p.iscale2 * p.rowp[p.tile * kT + r] * p.rowp[p.k * kT + 64 * ch + c + j] : 0.f;
+        *a = make_float2((pre ? fmaf(-v[j], f, o.x) : o.x) + o.y, 0.f);
+      }
+    }
+    __syncwarp();
+  }
+  (void)pair_any(q, false);
+  if (ch == 0 && in) {
+#pragma unroll 1
+    for (int c = 0; c < kT; c++) {
+      float s = row[(size_t)c * p.lda].x;
+#pragma unroll 8
+      for (int e = 0; e < c; e++) s = fmaf(-row[(size_t)e * p.lda].x, L[(size_t)e * p.lda + c].x, s);
+      row[(size_t)c * p.lda].x = s / L[(size_t)c * p.lda + c].x;
+    }
+  }
+  __syncwarp();
+  (void)pair_any(q, false);
+}
+
+// The slices of those rows of L_ik: a row past the common scale by a power of two
+// of its own, from its largest value.  Returns the common scale / the row's.
+__device__ __forceinline__ float split_rows(const PanelArgs& p, PanelBars* bars, unsigned char* R0, int q, int ch, int r) {
+  const float2* row = p.A + (size_t)(p.k * kT + 64 * ch) * p.lda + p.tile * kT + r;
+  const bool in = p.tile * kT + r < p.m;
+  float m = 0.f, s = p.scale, lrow = 1.f;
+#pragma unroll 1
+  for (int pass = 0; pass < 2; pass++) {
+#pragma unroll 1
+    for (int c = 0; c < 64; c += 8) {
+      float x[8];
+      uint32_t top = 0;
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        x[j] = in ? row[(size_t)(c + j) * p.lda].x * s : 0.f;
+        m = fmaxf(m, fabsf(x[j]));
+      }
+      if (pass) put_slices8(R0, r, 64 * ch + c, x, top);
+    }
+    if (pass) break;
+    bars->rmax[ch][r] = m;  // of scale * L
+    (void)pair_any(q, false);
+    m = fmaxf(m, bars->rmax[ch ^ 1][r]);
+    float up, down;
+    if (m >= 32768.f && own_scale(m, up, down)) {
+      lrow = down;
+      s *= up;
+      bars->lown = 1;
+      p.past[1 + p.k] = 1;
+      atomicMin(p.past, p.k);
+    }
+  }
+  __syncwarp();
+  return lrow;
+}
+
+// The diagonal block's updates by panels k and (pre) k - 1 whose rows have scales
+// of their own: row r, columns 64 ch .. + 63, in S and (the first 32) in x.
+__device__ __forceinline__ void own_diag(const PanelArgs& p, PanelBars* bars, float (*S)[kLd], float (&x)[32],
+                                         uint32_t trow, bool pre, int ch, int r, bool in) {
+  float4* s4 = reinterpret_cast<float4*>(S[r]);
+  if (ch == 0) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) s4[j] = make_float4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+  }
+  const int t = (p.k + 1) * kT;
+  const float fk = p.iscale2 * bars->lrow[r], fp = pre ? p.iscale2 * p.rowp[t + r] : 0.f;
+#pragma unroll 1
+  for (int c = 64 * ch; c < 64 * ch + 64; c += 8) {
+    float v[8];
+    sm100::tmem_ld8(trow + c, v);
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      if (in) S[r][c + j] = fmaf(-v[j], fk * bars->lrow[c + j], S[r][c + j]);
+    __syncwarp();
+    if (pre) {
+      sm100::tmem_ld8(trow + 128 + c, v);
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+        if (in) S[r][c + j] = fmaf(-v[j], fp * p.rowp[t + c + j], S[r][c + j]);
+      __syncwarp();
+    }
+  }
+  if (ch == 0) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const float4 f = s4[j];
+      x[4 * j] = f.x, x[4 * j + 1] = f.y, x[4 * j + 2] = f.z, x[4 * j + 3] = f.w;
+    }
+  }
+}
 
 // Shared memory: R0 L_i,k-1 then L_ik's slices; R1 L_k,k-1 then the tile's
 // slices (the diagonal block from kChainS on reuses R1 and the start of R2);
@@ -462,8 +638,14 @@ struct PanelArgs {
 // core truncates its sums, so their error grows with the length).
 // Warp 0 copies, warp 1 issues the products, warps 2 .. 9 hold the tile: a
 // thread one row (TMEM lane) and 64 columns.
-template <bool CHAIN>
-__device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs& p) {
+// OWN = false returns true, with nothing written to global memory but past and
+// rowk, where a value does not fit the common scale (it makes its row of the
+// product infinite or NaN) or panel k - 1 has rows with scales of their own.
+// OWN = true then does the work again, with solve_rows, split_rows and own_diag:
+// apart, as those cost every panel 2 us in one body with the rest (registers of
+// the diagonal block, loaded ahead, were waited for and spilled over them).
+template <bool CHAIN, bool OWN>
+__device__ __forceinline__ bool panel_body(unsigned char* smraw, const PanelArgs& p) {
   unsigned char* sm = align1024(smraw);
   unsigned char *R0 = sm, *R1 = sm + kTileBytes, *R2 = sm + 2 * kTileBytes;
   PanelBars* bars = reinterpret_cast<PanelBars*>(sm + kPanelMisc);
@@ -471,7 +653,12 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool has_tile = p.tile >= 0, pre = has_tile && p.PSpre != nullptr;
   constexpr uint32_t kCols = CHAIN ? 512 : 256;
+  if (CHAIN && !has_tile)  // the factorisation's first launch
+    for (int i = tid; i <= cdiv_d(p.m, kT); i += blockDim.x) p.past[i] = i == 0 ? INT_MAX : 0;
   if (tid == 0) {
+    if (OWN)
+      for (uint64_t* b = &bars->fullPre; b < (CHAIN ? bars->step + 16 : &bars->r0Free); b++) sm100::mbar_inval(b);
+    bars->failed = bars->again = bars->lown = bars->rown = 0;
     sm100::mbar_init(&bars->fullPre, 1);
     sm100::mbar_init(&bars->fullW, 2);
     sm100::mbar_init(&bars->preDone, 1);
@@ -490,7 +677,7 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
     }
     sm100::fence_mbar_init();
   }
-  if (warp == 1) sm100::tmem_alloc(&bars->slot, kCols);
+  if (!OWN && warp == 1) sm100::tmem_alloc(&bars->slot, kCols);
   sm100::tc_fence_before();
   __syncthreads();
   sm100::tc_fence_after();
@@ -513,7 +700,8 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
       if (lane == 0) {
         sm100::mbar_arrive(&bars->fullW);
         ok = sm100::mbar_wait(&bars->lReady, 0, kWaitLimit);
-        if (ok) {
+        if (ok && !OWN && bars->again) {
+        } else if (ok) {
           sm100::bulk_s2g(p.PSp + (size_t)p.tile * kTileBytes, R0, kTileBytes);
           sm100::bulk_store_wait();
         } else {  // copies in flight land before the CTA exits
@@ -523,7 +711,7 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
       }
       __syncwarp();
     }
-    if (CHAIN) {
+    if (CHAIN && (OWN || !has_tile || !bars->again)) {
       const int nd = p.k + 1;
       if (lane == 0) sm100::mbar_arrive(&bars->r0Free);
       chain_store_l(S, bars, lane, min(kT, p.m - nd * kT), p.A + (size_t)(nd * kT) * p.lda + nd * kT, p.lda, ok);
@@ -545,8 +733,10 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
       if (CHAIN) {
         ok = ok && sm100::mbar_wait(&bars->lReady, 0, kWaitLimit);
         sm100::tc_fence_after();
-        if (ok) mma_tile(tmem + 256, R0, R0, false);
-        sm100::mma_commit(&bars->qDone);
+        if (OWN || !bars->again) {
+          if (ok) mma_tile(tmem + 256, R0, R0, false);
+          sm100::mma_commit(&bars->qDone);
+        }
       }
       if (!ok) (void)sm100::mbar_wait(&bars->xDone, 0, kWaitLimit);
     }
@@ -555,6 +745,8 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
     const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(64 * ch);
     const uint64_t pol = sm100::policy_evict_first();  // the tile's columns are read again only by the noise product
     const int nd = p.k + 1;  // the diagonal block of the chain CTA (tile row of its tile too)
+    const bool pown = pre && p.past[p.k] != 0;  // rows of panel k - 1 have scales of their own
+    bool subst = false;  // this row (all 32 of the warp) solved by solve_rows, in A
     // 64 columns of the thread's row of L_ik, from tensor memory into A
     auto store_l = [&](int half) {
       const int gi = p.tile * kT + r;
@@ -587,8 +779,9 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
         ok = sm100::mbar_wait(&bars->preDone, 0, kWaitLimit);
         sm100::tc_fence_after();
       }
-      // the tile less panel k - 1's update, as slices of scale^2 / 16 times
-      // it (|A_ij| <= max D_ii: at most 2^14)
+      uint32_t top = 0;  // (what does not fit shows in the product)
+      // the tile less panel k - 1's update, as slices of scale^2 / 16 times it
+      // (positive definite: |A_ij| <= max D_ii, at most 2^14)
       const float cs = p.scale * p.scale * 0.0625f;
 #pragma unroll
       for (int c = 0; c < 4; c++) {
@@ -602,7 +795,7 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
             const float2 o = old[16 * c + 8 * h + j];
             x[j] = (pre ? fmaf(-v[8 * h + j], p.iscale2, o.x) + o.y : o.x + o.y) * cs;
           }
-          put_slices8(R1, r, 64 * ch + 16 * c + 8 * h, x);
+          put_slices8(R1, r, 64 * ch + 16 * c + 8 * h, x, top);
         }
       }
       sm100::fence_proxy_async();
@@ -616,10 +809,12 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
       for (int j = 0; j < 64; j++)
         old[j] = sm100::ld_f2_hint_if(colp + (size_t)j * p.lda, pol, 64 * ch + j <= r && r < kb);
     }
+    bool again = false;
     if (has_tile) {
       ok = sm100::mbar_wait(&bars->fullW, 0, kWaitLimit) && ok;  // (xsc)
       ok = sm100::mbar_wait(&bars->xDone, 0, kWaitLimit) && ok;
       sm100::tc_fence_after();
+      uint32_t top = 0;
 #pragma unroll 1
       for (int c = 0; c < 4; c++) {
         float v[16], x[16];
@@ -636,15 +831,30 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
           float y[8];
 #pragma unroll
           for (int j = 0; j < 8; j++) y[j] = x[8 * j8 + j];
-          put_slices8(R0, r, 64 * ch + 16 * c + 8 * j8, y);
+          put_slices8(R0, r, 64 * ch + 16 * c + 8 * j8, y, top);
         }
+      }
+      float lrow = 1.f;
+      if (!OWN) {
+        if (pown || past(top)) bars->again = 1;
+      } else if (pair_any(q, pown || past(top))) {
+        subst = true;
+        solve_rows(p, q, ch, r, pre, trow);
+        lrow = split_rows(p, bars, R0, q, ch, r);
+      }
+      if (ch == 0) {
+        if (OWN) bars->lrow[r] = lrow;
+        p.rowk[p.tile * kT + r] = lrow;
       }
       sm100::fence_proxy_async();
       __syncwarp();
       if (lane == 0) sm100::mbar_arrive(&bars->lReady);
-      if (!CHAIN) store_l(ch);
+      ok = sm100::mbar_wait(&bars->lReady, 0, kWaitLimit) && ok;  // (again; lown, lrow)
+      again = !OWN && bars->again;
+      if (!CHAIN && !subst && !again) store_l(ch);
     }
-    if (CHAIN) {
+    if (CHAIN && !again) {
+      const bool own = OWN && (pown || bars->lown);  // rows of panel k or k - 1 have scales of their own
       if (has_tile) {
         ok = sm100::mbar_wait(&bars->qDone, 0, kWaitLimit) && ok;
         sm100::tc_fence_after();
@@ -657,12 +867,12 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
         float y[8], v[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) y[j] = old[8 * c + j].x;
-        if (has_tile) {
+        if (has_tile && !own) {
           sm100::tmem_ld8(trow + 256 + 8 * c, v);
 #pragma unroll
           for (int j = 0; j < 8; j++) y[j] = fmaf(-v[j], p.iscale2, y[j]);
         }
-        if (pre) {
+        if (pre && !own) {
           sm100::tmem_ld8(trow + 384 + 8 * c, v);
 #pragma unroll
           for (int j = 0; j < 8; j++) y[j] = fmaf(-v[j], p.iscale2, y[j]);
@@ -681,12 +891,13 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
           *reinterpret_cast<float4*>(&S[r][64 * ch + 8 * c + 4]) = make_float4(y[4], y[5], y[6], y[7]);
         }
       }
+      if (own) own_diag(p, bars, S, x, tmem + ((uint32_t)(32 * q) << 16) + 256, pre, ch, r, r < kb);
       if (ch == 0) {
         int neg = 0;
         chol_inv128(S, bars, R0, tmem, x, r, lane, p.scale, neg, ok);
         if (neg && lane == 0 && q == 0) atomicAdd(p.negpiv, neg);
       } else {
-        if (has_tile) {
+        if (has_tile && !subst) {
           store_l(0);
           store_l(1);
         }
@@ -707,10 +918,15 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
       }
     }
   }
-  if (!ok) atomicExch(p.err, 6);
+  if (!ok) {
+    atomicExch(p.err, 6);
+    bars->failed = 1;
+  }
   sm100::tc_fence_before();
   __syncthreads();
+  if (!OWN && bars->again && !bars->failed) return true;
   if (warp == 1) sm100::tmem_dealloc(tmem, kCols);
+  return false;
 }
 
 // ------------------------------------------------------------ tensor-core trailing update
@@ -754,7 +970,7 @@ __device__ __forceinline__ void panel_body(unsigned char* smraw, const PanelArgs
 constexpr int kRestThreads = 320;
 constexpr int kStageBytes = kTileSlices * kHalfBytes;  // one K-half of the two B slices
 constexpr size_t kRestSmem = kPanelSmem;
-static_assert(kRestSmem >= (size_t)kTileBytes + 2 * kStageBytes + 1024 + 256, "the update CTAs' operands");
+static_assert(kRestSmem >= (size_t)kTileBytes + 2 * kStageBytes + 1024 + 512, "the update CTAs' operands");
 constexpr int kAccCols = 128;
 
 constexpr int kAccs = 4;       // accumulators in tensor memory (all of its columns)
@@ -762,12 +978,9 @@ constexpr int kFoldPanels = 3;  // panels summed into one of them (K = 384): lon
 struct RestBars {
   uint64_t fullA, emptyA, fullB[2], emptyB[2], accFull[kAccs], accEmpty[kAccs], done;
 };
-// Panel slices: panel p in buffer p % kBufs (a group's pass reads its panels' while
-// the next is written), buf bytes apart
-constexpr int kBufs = 7;
 struct Slices {
   const unsigned char* base;
-  size_t buf;
+  size_t buf;  // bytes of one buffer
   __device__ __forceinline__ const unsigned char* at(int p) const { return base + (size_t)(p % kBufs) * buf; }
 };
 
@@ -815,10 +1028,17 @@ __device__ __forceinline__ void rest_tile(int t, int jlo, int mode, int nt, int&
 // the tile: both operands streamed in 2 npan chunks of 64 KB per tile (panel,
 // K-half) through the two stages, three panels to an accumulator, NF of them
 // subtracted from the tile one after the other (as NF passes would).
+// Returns true, with nothing done but the tensor memory's allocation, where one of
+// the panels has rows with scales of their own (own_update's).
 template <int NF>
-__device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int lda, int m, int jlo, int mode,
+__device__ __forceinline__ bool rest_body(unsigned char* smraw, float2* A, int lda, int m, int jlo, int mode,
                                           int tlo, int thi, int group, int cta, const Slices& sl, int p0, int npan,
-                                          int fold, int* err, float iscale2) {
+                                          int fold, int* err, float iscale2, const int* past) {
+  // (loaded ahead of the set-up, looked at behind it.  Looked at by the roles, in
+  // their loops, the compiler places the epilogue's loads worse: 119 against 122 ms
+  // at 3N = 46,200; ahead of the body, 4 us a launch of a batch)
+  int first;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(first) : "l"(past));
   // (rounded as an integer, not by align1024: with the pointer known to be
   // shared the compiler places the epilogue's loads worse, 211 against 161 ms
   // for the factorisation at 3N = 46,200)
@@ -852,6 +1072,11 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
   __syncthreads();
   sm100::tc_fence_after();
   const uint32_t tmem = *tslot;
+  if (first < p0 + npan) {
+    bool own = false;
+    for (int i = 0; i < npan; i++) own = own || past[1 + p0 + i] != 0;
+    if (own) return true;
+  }
 
   if (warp == 0) {
     if (lane == 0) {
@@ -1148,6 +1373,84 @@ __device__ __forceinline__ void rest_body(unsigned char* smraw, float2* A, int l
   sm100::tc_fence_before();
   __syncthreads();
   if (warp == 1) sm100::tmem_dealloc(tmem, kAccs * kAccCols);
+  return false;
+}
+
+static_assert(sizeof(RestBars) + 2 * sizeof(int) <= 256, "own_update's barriers lie behind them");
+
+// The same tiles for panels with rows whose scales are their own (rowf: the
+// common scale / theirs), one panel and one tile at a time.
+__device__ __forceinline__ void own_update(unsigned char* smraw, float2* A, int lda, int m, int jlo, int mode, int t0,
+                                        int t1, const Slices& sl, int p0, int npan, int* err, float iscale2,
+                                        const float* rowf) {
+  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smraw) + 1023) & ~uintptr_t(1023));
+  unsigned char* sB = sm + kTileBytes;
+  RestBars* first = reinterpret_cast<RestBars*>(sB + 2 * kStageBytes);  // rest_body's
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(first + 1);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(first) + 256);  // copies, products
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tslot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nt = cdiv_d(m, kT);
+  if (threadIdx.x == 0) {
+    sm100::mbar_init(&bars[0], 1);
+    sm100::mbar_init(&bars[1], 1);
+    *abort_flag = 0;
+    sm100::fence_mbar_init();
+  }
+  __syncthreads();
+  const uint32_t tmem = *tslot;  // (rest_body's)
+  uint32_t ph = 0;
+  bool ok = true;
+#pragma unroll 1
+  for (int t = t0; t < t1; t++) {
+    int I, J;
+    rest_tile(t, jlo, mode, nt, I, J);
+#pragma unroll 1
+    for (int p = p0; p < p0 + npan; p++, ph ^= 1) {
+      if (threadIdx.x == 0) {
+        const unsigned char* src = sl.at(p);
+        sm100::mbar_arrive_expect_tx(&bars[0], I == J ? kTileBytes : 2 * kTileBytes);
+        sm100::bulk_g2s(sm, src + (size_t)I * kTileBytes, kTileBytes, &bars[0]);
+        if (I != J) sm100::bulk_g2s(sB, src + (size_t)J * kTileBytes, kTileBytes, &bars[0]);
+        if (sm100::mbar_wait(&bars[0], ph, kWaitLimit)) {
+          sm100::tc_fence_after();
+          mma_tile(tmem, sm, I == J ? sm : sB, false);
+        } else {  // the copies in flight land before the CTA exits
+          ok = false;
+          (void)sm100::mbar_wait(&bars[0], ph, kWaitLimit);
+        }
+        sm100::mma_commit(&bars[1]);
+      }
+      __syncwarp();
+      ok = sm100::mbar_wait(&bars[1], ph, kWaitLimit) && ok;
+      sm100::tc_fence_after();
+      if (warp >= 2) {
+        const int q = warp & 3, ch = (warp - 2) >> 2, r = I * kT + 32 * q + lane;
+        const float* f = rowf + (size_t)(p % kBufs) * (nt * kT);
+        const float fr = iscale2 * f[r];
+#pragma unroll 1
+        for (int c = 64 * ch; c < 64 * ch + 64; c += 8) {
+          float v[8];
+          sm100::tmem_ld8(tmem + ((uint32_t)(32 * q) << 16) + c, v);
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            const int col = J * kT + c + j;
+            if (r < m && col <= r) {
+              float2* a = A + (size_t)col * lda + r;
+              *a = df_sub(*a, v[j] * (fr * f[col]));
+            }
+          }
+          __syncwarp();
+        }
+      }
+      if (!ok) *abort_flag = 1;
+      sm100::tc_fence_before();
+      __syncthreads();  // the operands and the accumulator are free
+      if (*abort_flag) t = t1, p = p0 + npan;
+    }
+  }
+  if (!ok) atomicExch(err, 5);
+  if (warp == 1) sm100::tmem_dealloc(tmem, kAccs * kAccCols);
 }
 
 // An update job: tiles [tlo, thi) of an enumeration (rest_tile) from column
@@ -1160,6 +1463,7 @@ struct StepArgs {
   PanelArgs pan;  // panel k and the chain's tile
   int ntile;      // tile CTAs: tile rows k + 2 .. k + 1 + ntile
   Slices sl;
+  const float* rowf;  // [kBufs][nt kT] the rows' factors (PanelArgs) by slice buffer
   UpdJob job[kJobs];
 };
 
@@ -1169,14 +1473,20 @@ struct StepArgs {
 __device__ __forceinline__ void chol_step_body(const StepArgs& a, int b, float4* smem4) {
   unsigned char* sm = reinterpret_cast<unsigned char*>(smem4);
   if (b == 0) {
-    panel_body<true>(sm, a.pan);
+    if (panel_body<true, false>(sm, a.pan)) {
+      __syncthreads();  // (its flags are set anew)
+      (void)panel_body<true, true>(sm, a.pan);
+    }
     return;
   }
   b -= 1;
   if (b < a.ntile) {
     PanelArgs p = a.pan;
     p.tile = a.pan.k + 2 + b;
-    panel_body<false>(sm, p);
+    if (panel_body<false, false>(sm, p)) {
+      __syncthreads();
+      (void)panel_body<false, true>(sm, p);
+    }
     return;
   }
   b -= a.ntile;
@@ -1184,14 +1494,20 @@ __device__ __forceinline__ void chol_step_body(const StepArgs& a, int b, float4*
   while (jn < kJobs - 1 && b >= a.job[jn].nctas) b -= a.job[jn++].nctas;
   const UpdJob& j = a.job[jn];
   const PanelArgs& p = a.pan;
+  bool own = false;  // rows with scales of their own
   auto run = [&](auto nf) {
-    rest_body<decltype(nf)::value>(sm, p.A, p.lda, p.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b, a.sl, j.p0, j.npan,
-                                   j.fold, p.err, p.iscale2);
+    own = rest_body<decltype(nf)::value>(sm, p.A, p.lda, p.m, j.jlo, j.mode, j.tlo, j.thi, j.group, b, a.sl, j.p0, j.npan,
+                                   j.fold, p.err, p.iscale2, p.past);
   };
   if (j.npan > 2 * j.fold) run(std::integral_constant<int, 4>{});
   else if (j.npan > j.fold) run(std::integral_constant<int, 2>{});
   else if (j.npan > 1) run(std::integral_constant<int, 1>{});
   else run(std::integral_constant<int, 0>{});
+  if (own) {
+    const int t0 = j.tlo + b * j.group;
+    own_update(sm, p.A, p.lda, p.m, j.jlo, j.mode, t0, min(t0 + j.group, j.thi), a.sl, j.p0, j.npan, p.err, p.iscale2,
+               a.rowf);
+  }
 }
 
 __global__ void __launch_bounds__(kRestThreads, 1) k_chol_step(const __grid_constant__ StepArgs a) {
@@ -1241,17 +1557,22 @@ constexpr int kGroup[4] = {0, 4, 3, 2};  // accumulators by fold
 constexpr int kGroupMin = 4;             // tile rows right of a group (fewer accumulators at the end)
 static_assert(kBufs > kGroup[1] && kBufs > 2 * kGroup[2] && kBufs > 3 * kGroup[3], "a group's panels and the next");
 // the slice buffers, then two buffers for the inverse of a diagonal factor
-// (W_k in buffer k & 1: read by the launch that writes W_k+1), then its factors
+// (W_k in buffer k & 1: read by the launch that writes W_k+1), then its factors,
+// the rows' scales by slice buffer and a flag a panel (PanelArgs)
 size_t mixed_panel_bytes(int m) {
-  return kBufs * (size_t)cdiv(m, kT) * kTileBytes + 2 * (size_t)kTileBytes + 2 * kT * sizeof(float);
+  const size_t nt = cdiv(m, kT);
+  return kBufs * nt * kTileBytes + 2 * (size_t)kTileBytes + 2 * kT * sizeof(float) + kBufs * nt * kT * sizeof(float) +
+         (nt + 1) * sizeof(int);
 }
 int mixed_max_launches(int m) { return 2 * cdiv(m, kT) + 2; }
 int mixed_tiles(int m) { return cdiv(m, kT); }
 
-// |L_ij| <= sqrt(max D_ii): the slices' largest value is put into [2^8, 2^9),
-// so values down to 2^-34 of it stay in the pair (FP16's smallest subnormal
-// is 2^-24) and a factor with replaced negative pivots has 2^7 of room
-// before the clamp.  Radii that give no finite positive diagonal: 1.
+// Positive definite: |L_ij| <= sqrt(max D_ii), so the slices' largest value is
+// put into [2^8, 2^9): values down to 2^-34 of it stay in the pair (FP16's
+// smallest subnormal is 2^-24), and the tiles' own slices (scale^2 / 16 times the
+// tensor) are at most 2^14.  A factor with replaced negative pivots has 2^7 of
+// room, its tiles 2^2 to 2^4; rows past that: see Range above.  Radii that give no
+// finite positive diagonal: 1.
 float mixed_scale(double a1, const double* rad, int nrad) {
   double dmax = 0.0;
   for (int i = 0; i < nrad; i++) dmax = std::max(dmax, std::fabs(a1 / rad[i]));
@@ -1332,6 +1653,7 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
   auto psb = [&](int k) { return PS + (size_t)(k % kBufs) * buf; };
   unsigned char* Wb = PS + kBufs * buf;  // the inverses' slices
   float* wsc = reinterpret_cast<float*>(Wb + 2 * (size_t)kTileBytes);
+  float* rowf = wsc + 2 * kT;
   // elements of the lower triangle in tile columns [j0, j1)
   auto elems = [&](int j0, int j1) {
     double e = 0.0;
@@ -1369,9 +1691,12 @@ static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int*
     p.PSp = psb(k < 0 ? 0 : k), p.PSpre = k > 0 ? psb(k - 1) : nullptr;
     p.Wk = Wb + (size_t)(k & 1) * kTileBytes, p.wsc = wsc + kT * (k & 1);
     p.Wn = Wb + (size_t)((k + 1) & 1) * kTileBytes, p.wscn = wsc + kT * ((k + 1) & 1);
+    p.rowk = rowf + (size_t)((k < 0 ? 0 : k) % kBufs) * nt * kT, p.rowp = rowf + (size_t)((k > 0 ? k - 1 : 0) % kBufs) * nt * kT;
+    p.past = reinterpret_cast<int*>(rowf + (size_t)kBufs * nt * kT);
     p.negpiv = negpiv, p.err = err, p.scale = scale, p.iscale2 = 1.f / (scale * scale);
     a.ntile = k < 0 ? 0 : nt - k - 2;
     a.sl = Slices{PS, buf};
+    a.rowf = rowf;
     const Job* js[kJobs] = {&j0, &j1};
     int grid = 1 + a.ntile;
     for (int q = 0; q < kJobs; q++) {
