@@ -153,8 +153,11 @@ static int step_phases(bd_ctx* c, const double* d_rr, const double* d_p, double*
   // whose replicas already fill the GPU beside each other.
   const bool overlap = phases == (kPre | kChol | kPost) && !c->timing && !c->in_batch;
   const bdk::Side* side = overlap ? &c->side : nullptr;
-  if (overlap) CK(cudaEventRecord(c->side.e[0], st));
-  auto join = [&]() { return !overlap || cudaStreamWaitEvent(st, c->side.e[1], 0) == cudaSuccess; };
+  auto lost = [&]() {  // a fork or a join failed
+    c->side.drain();
+    return set_error(BD_ERR_CUDA, "bd_step: forking or joining a force pass");
+  };
+  if (overlap && cudaEventRecord(c->side.e[0], st) != cudaSuccess) return lost();
   if (phases & kPre) {
     record(c, 0);
     bdk::gather_rall(M, c->X, c->r_all, mixed ? &c->S : nullptr, st);
@@ -170,9 +173,9 @@ static int step_phases(bd_ctx* c, const double* d_rr, const double* d_p, double*
     record(c, 1);
   }
   if (overlap) {
-    CK(cudaStreamWaitEvent(c->side.s[0], c->side.e[0], 0));
+    if (cudaStreamWaitEvent(c->side.s[0], c->side.e[0], 0) != cudaSuccess) return lost();
     L += bdk::forces(M, c->X, c->F0, c->S, c->precision, c->side.s[0]);
-    CK(cudaEventRecord(c->side.e[1], c->side.s[0]));
+    if (cudaEventRecord(c->side.e[1], c->side.s[0]) != cudaSuccess) return lost();
   }
   if ((phases & kChol) && rebuild && !krylov) {
     c->a_holds_factor = true;
@@ -197,7 +200,7 @@ static int step_phases(bd_ctx* c, const double* d_rr, const double* d_p, double*
                           c->krylov_tol, c->krylov_kmax, c->rd, c->kscratch, st, &c->krylov_iters, &c->krylov_change,
                           &c->kgraphs);
     if (rc) {
-      join();
+      if (overlap) c->side.drain();
       return set_error(rc, "bd_step: Krylov noise displacement failed");
     }
     L += (mixed ? 6 : 7) * c->krylov_iters + 3;
@@ -207,7 +210,7 @@ static int step_phases(bd_ctx* c, const double* d_rr, const double* d_p, double*
   }
   record(c, 3);
   if (!overlap) L += bdk::forces(M, c->X, c->F0, c->S, c->precision, st);
-  else if (!join()) return set_error(BD_ERR_CUDA, "bd_step: joining the force pass");
+  else if (cudaStreamWaitEvent(st, c->side.e[1], 0) != cudaSuccess) return lost();
   record(c, 4);
   bdk::rotate_translate(M, c->X, c->Y, c->F0, d_rr, c->rd, c->r_all, c->precision, c->S, st);
   L += mixed ? 3 : 2;
@@ -217,7 +220,9 @@ static int step_phases(bd_ctx* c, const double* d_rr, const double* d_p, double*
   L += 2;
   if (saves && (rc = pack_ns(c, c->Y, saves[1]))) return rc;
   record(c, 6);
-  L += bdk::forces(M, c->Y, c->F1, c->S, c->precision, st, side);
+  const int nf = bdk::forces(M, c->Y, c->F1, c->S, c->precision, st, side);
+  if (nf < 0) return lost();
+  L += nf;
   record(c, 7);
   bdk::average_forces(M, c->F0, c->F1, c->Fa, st);
   bdk::rotate_translate(M, c->X, c->Y, c->Fa, d_rr, c->rd, c->r_all, c->precision, c->S, st);
@@ -684,7 +689,8 @@ extern "C" int bd_step_reference(bd_ctx* c, int step, int number_of_steps, int f
 
 extern "C" int bd_forces(bd_ctx* c, double* F, double* T, double* tF, double* lF, double* E) {
   if (!c) return set_error(BD_ERR_ARG, "bd_forces: null context");
-  bdk::forces(c->M, c->X, c->F0, c->S, c->precision, c->stream, c->in_batch ? nullptr : &c->side);
+  if (bdk::forces(c->M, c->X, c->F0, c->S, c->precision, c->stream, c->in_batch ? nullptr : &c->side) < 0)
+    return set_error(BD_ERR_CUDA, "bd_forces: forking or joining its parts");
   CK(cudaGetLastError());
   cudaStream_t st = c->stream;
   size_t n3 = 3 * (size_t)c->M.n;

@@ -137,14 +137,20 @@ void average_forces(const DevModel& M, const DevForces& A, const DevForces& B, D
 // r_all: every tensor bead's position; with S (mixed path) also S->qh / S->ql
 void gather_rall(const DevModel& M, const DevState& X, double* r_all, const DevScratch* S, cudaStream_t st);
 // forces.cu
-// returns the number of kernels launched
 // Streams beside a context's own and the events that fork to and join from them
 struct Side {
   cudaStream_t s[2] = {};
   cudaEvent_t e[7] = {};
+  // After a fork or join that failed: nothing is left running on the side
+  // streams, and the error is not found again by the next call's check.
+  void drain() const {
+    for (auto a : s) (void)cudaStreamSynchronize(a);
+    (void)cudaGetLastError();
+  }
 };
-// side: the pass's independent parts go beside each other, forked from and
-// joined to st
+// Returns the number of kernels launched.  side: the pass's independent parts go
+// beside each other, forked from and joined to st; -1: a fork or a join failed
+// (side drained).
 int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& scr, int mixed, cudaStream_t st,
            const Side* side = nullptr);
 // rpy_chol.cu

@@ -1669,11 +1669,14 @@ namespace bdk {
 int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& S, int mixed, cudaStream_t st,
            const Side* side) {
   cudaStream_t s0 = side ? side->s[0] : st, s1 = side ? side->s[1] : st;
-  auto rec = [&](int e, cudaStream_t a) {
-    if (side) cudaEventRecord(side->e[e], a);
-  };
-  auto wait = [&](cudaStream_t b, int e) {
-    if (side) cudaStreamWaitEvent(b, side->e[e], 0);
+  // After a fork or a join that failed nothing more is launched: it would run
+  // beside parts that it needs, or that write what it writes.
+  bool ok = true;
+  auto rec = [&](int e, cudaStream_t a) { ok = ok && (!side || cudaEventRecord(side->e[e], a) == cudaSuccess); };
+  auto wait = [&](cudaStream_t b, int e) { ok = ok && (!side || cudaStreamWaitEvent(b, side->e[e], 0) == cudaSuccess); };
+  auto lost = [&]() {
+    side->drain();
+    return -1;
   };
   // energy layout in S.ebuf: [0,n) chain, [n, n+n_tail) tails, then LH
   double* Ech = S.ebuf;
@@ -1693,6 +1696,7 @@ int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& S, int mi
   rec(2, st);
   wait(s0, 2);
   wait(s1, 2);
+  if (!ok) return lost();
   if (M.n > 1) {
     k_chain_bonds<<<cdiv(M.n - 1, kBeadThreads), kBeadThreads, 0, s0>>>(M, X, S.bonds);
     L++;
@@ -1701,6 +1705,7 @@ int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& S, int mi
   L++;
   if (M.n_lhcore > 0) { k_ghead_coreX<<<M.n_lhcore * M.n_c, kGheadThreads, 0, s0>>>(M, X, S.gc); L++; }
   rec(3, s0);
+  if (!ok) return lost();
   if (mixed) {
     if (M.n_tail > 0) { k_tail_bonded_mx<<<cdiv(M.n_tail, kBeadThreads), kBeadThreads, 0, s1>>>(M, X, S); L++; }
     if (M.n_LH > 0) { k_lh_bonded_mx<<<cdiv(M.n_LH, kBeadThreads), kBeadThreads, 0, s1>>>(M, X, S); L++; }
@@ -1712,6 +1717,7 @@ int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& S, int mi
   }
   if (M.n_dna > 0 && M.n_c > 0) { k_dna_coreX<<<cdiv(M.n_dna * M.n_c * 32, 256), 256, 0, st>>>(M, X, S, S.dc); L++; }
   rec(4, st);
+  if (!ok) return lost();
   if (M.n_c > 1) {
     if (mixed) {
       size_t sm = (size_t)((14 * M.Nq + 1) / 2 + 32 * 10) * sizeof(double);
@@ -1724,8 +1730,9 @@ int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& S, int mi
     L += 2;
   }
   wait(st, 3);
+  if (mixed) wait(s0, 4);
+  if (!ok) return lost();
   if (mixed) {
-    wait(s0, 4);
     if (M.n_dna > 0) k_chain_gather_mx<<<M.n_dna, kGatherThreads, 0, s0>>>(M, X, Fm, Tm, Ebond, S, out, Ech, M.dna_bead);
     if (M.n_c > 0) k_chain_gather_mx<<<M.n_c, kGatherCoreThreads, 0, st>>>(M, X, Fm, Tm, Ebond, S, out, Ech, M.core_bead);
     L += (M.n_dna > 0) + (M.n_c > 0) - 1;  // one chain launch is counted below
@@ -1736,6 +1743,7 @@ int forces(const DevModel& M, DevState& X, DevForces& out, DevScratch& S, int mi
   rec(6, s1);
   wait(st, 5);
   wait(st, 6);
+  if (!ok) return lost();
   k_energy<<<1, 256, 0, st>>>(M.n + M.n_tail + M.n_LH, S.ebuf, out.E);
   return L + 2;
 }
