@@ -10,7 +10,7 @@
 
 #include "../../include/bd_capi.h"
 
-// core/core pairs: each pair's charge pairs over this many CTAs (the slots are sized for the larger)
+// core/core pairs: each pair's charge pairs over this many CTAs
 constexpr int kCCSplit = 4, kCC64Split = 15;  // mixed path, FP64 path
 
 namespace bdh {
@@ -108,7 +108,7 @@ struct DevForces {
 // interacting object pair, reduced per bead in a fixed order).
 struct DevScratch {
   double* cc;    // [n_c * n_c * 10]  core-core: F(3) T_i(3) T_j(3) E
-  double* ccp;   // [kCC64Split * n_c * n_c * 10] core-core partials (a pair over kCC64Split or kCCSplit CTAs)
+  double* ccp;   // [kCC64Split or kCCSplit (FP64, mixed) * n_c * n_c * 10] core-core partials, by CTA
   double* dc;    // [n_dna * n_c * 7] DNA-core: F_on_dna(3) T_core(3) E
   double* gc;    // [n_lhcore * n_c * 10] G-head(core I) - charges(core L): F_I(3) T_I(3) T_L(3) E
   double* ebuf;  // [nE] per-kernel energy partials

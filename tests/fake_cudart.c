@@ -1,6 +1,6 @@
-/* A CUDA runtime without a GPU, preloaded by test_side_streams.py: memory is
- * host memory, kernels do nothing, every launch, event call and stream
- * synchronisation is logged, and one event call can be made to fail. */
+/* A CUDA runtime without a GPU, preloaded by the tests that name it: memory is
+ * host memory, kernels do nothing, every allocation, launch, event call and
+ * stream synchronisation is logged, and one event call can be made to fail. */
 #include <stdlib.h>
 #include <string.h>
 
@@ -30,7 +30,7 @@ int fake_log(char* ops, long* streams, int max) {
   return g_n;
 }
 
-err_t cudaMalloc(void** p, size_t n) { return (*p = calloc(n + 256, 1)) ? 0 : 2; }
+err_t cudaMalloc(void** p, size_t n) { note('M', (void*)n); return (*p = calloc(n + 256, 1)) ? 0 : 2; }
 err_t cudaFree(void* p) { free(p); return 0; }
 err_t cudaMemcpy(void* d, const void* s, size_t n, int k) { memcpy(d, s, n); return 0; }
 err_t cudaMemcpyAsync(void* d, const void* s, size_t n, int k, void* st) { memcpy(d, s, n); return 0; }
