@@ -196,7 +196,7 @@ static int step_phases(bd_ctx* c, const double* d_rr, const double* d_p, double*
   }
   record(c, 2);
   if (krylov) {
-    rc = bdk::krylov_sqrt(c->m, mixed ? nullptr : c->A, c->lda, mixed, c->S.qh, c->S.ql, M.a1, M.a2, d_p, M.s2dt,
+    rc = bdk::krylov_sqrt(c->m, mixed ? nullptr : c->A, c->lda, c->S.qh, c->S.ql, M.a1, M.a2, d_p, M.s2dt,
                           c->krylov_tol, c->krylov_kmax, c->rd, c->kscratch, st, &c->krylov_iters, &c->krylov_change,
                           &c->kgraphs);
     if (rc) {
@@ -773,7 +773,7 @@ extern "C" int bd_noise_displacement(bd_ctx* c, const double* p, double* rd) {
   if (c->noise_mode == BD_NOISE_KRYLOV) {
     assemble_now(c);
     CK(cudaMemcpyAsync(c->p, p, (size_t)c->m * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    int rc = bdk::krylov_sqrt(c->m, mixed ? nullptr : c->A, c->lda, mixed, c->S.qh, c->S.ql, c->M.a1, c->M.a2, c->p,
+    int rc = bdk::krylov_sqrt(c->m, mixed ? nullptr : c->A, c->lda, c->S.qh, c->S.ql, c->M.a1, c->M.a2, c->p,
                               c->M.s2dt, c->krylov_tol, c->krylov_kmax, c->rd, c->kscratch, c->stream,
                               &c->krylov_iters, &c->krylov_change, &c->kgraphs);
     if (rc) return set_error(rc, "bd_noise_displacement: Krylov iteration failed");

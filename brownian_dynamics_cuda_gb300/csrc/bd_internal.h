@@ -198,7 +198,6 @@ struct KrylovGraphs {
   int m = -1, kmax = -1;
   const double* scratch = nullptr;
   const double* A = nullptr;
-  bool df = false;
   double a1 = 0.0, a2 = 0.0;
   std::vector<cudaGraphExec_t> blocks;
   void clear() {
@@ -208,7 +207,7 @@ struct KrylovGraphs {
   }
   ~KrylovGraphs() { clear(); }
 };
-int krylov_sqrt(int m, const double* A, int lda, bool df, const float4* qh, const float4* ql, double a1, double a2,
+int krylov_sqrt(int m, const double* A, int lda, const float4* qh, const float4* ql, double a1, double a2,
                 const double* p, double s2dt, double tol, int kmax, double* rd, double* scratch, cudaStream_t st,
                 int* iters, double* change, struct KrylovGraphs* graphs = nullptr);
 int mixed_max_launches(int m);  // k_chol_step launches of one factorisation, at most

@@ -21,7 +21,6 @@ struct V3 {
 };
 __device__ __forceinline__ V3 ld3(const double* p) { return V3{p[0], p[1], p[2]}; }
 __device__ __forceinline__ void st3(double* p, V3 v) { p[0] = v.x; p[1] = v.y; p[2] = v.z; }
-__device__ __forceinline__ double c3(const V3& v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
 
 __device__ __forceinline__ double clamp09(double v) {
   if (v > 0.9) v = 0.9;
@@ -205,11 +204,11 @@ __device__ __forceinline__ void acc(V3& s, const V3& v) { s.x = s.x + v.x; s.y =
 __device__ __forceinline__ void dec(V3& s, const V3& v) { s.x = s.x - v.x; s.y = s.y - v.y; s.z = s.z - v.z; }
 
 // RPY tensor block (rows 3i+k, columns 3j+l) for a bead pair i != j, with
-// sij = r_i - r_j (either sign; func.cpp:753-799).  out[k][l]: one root and one
+// sij = r_i - r_j (either sign; func.cpp:753-799), s its length.  out[k][l]: one root and one
 // division (nine divisions with each element formed as the reference does: 170
 // FP64 operations a pair, 60 here; the FP64 pipe bounds tensor and drift).  3N =
 // 1,944: tensor 139 -> 41 us, drift 216 -> 54.
-__device__ __forceinline__ void rpy_block(const V3& sij, double ssq, double s, double radi, double radj, double a1,
+__device__ __forceinline__ void rpy_block(const V3& sij, double s, double radi, double radj, double a1,
                                           double a2, double (&out)[3][3]) {
   const double sv[3] = {sij.x, sij.y, sij.z}, mi = 1.0 / s;
   double dg, c;  // out = dg I + c s s^T

@@ -992,7 +992,7 @@ int forces_vjp(bd_ctx* c, const double* x, const double* fbar, double* lamOut, d
   if (M.n_c > 1)
     k_adj_corecore<R><<<dim3(M.n_c * M.n_c, cdiv(M.Nq, kCcThreads), kCcSplit), kCcThreads,
                         13 * cdiv(M.Nq, kCcSplit) * sizeof(R), st>>>(M, x, fbar, lamOut, th);
-  L += 4;
+  L += 3 + (M.n_c > 1);
   if (nt > 0) {
     k_adj_tail_bonded<double, R><<<cdiv(nt, 128), 128, 0, st>>>(M, x, fbar, lamOut);
     k_adj_tail_pairs<R><<<cdiv((long)nt * (nt + n), 256), 256, 0, st>>>(M, x, fbar, lamOut, th);

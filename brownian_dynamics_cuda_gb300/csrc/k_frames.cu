@@ -259,11 +259,10 @@ __global__ void k_translate(DevModel M, const double* __restrict__ r_all, const 
     }
     V3 rj = ld3(r_all + 3 * j);
     V3 sij{ri.x - rj.x, ri.y - rj.y, ri.z - rj.z};
-    double ssq = sij.x * sij.x + sij.y * sij.y + sij.z * sij.z;
-    double s = sqrt(ssq);
+    double s = sqrt(sij.x * sij.x + sij.y * sij.y + sij.z * sij.z);
     double radj = M.rad_all[j];
     double Db[3][3];
-    rpy_block(sij, ssq, s, radi, radj, M.a1, M.a2, Db);
+    rpy_block(sij, s, radi, radj, M.a1, M.a2, Db);
 #pragma unroll
     for (int l = 0; l < 3; l++) {
       const double fl = f[l];

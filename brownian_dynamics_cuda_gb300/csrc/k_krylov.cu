@@ -48,7 +48,6 @@ __device__ __forceinline__ void tile_of(long t, int& I, int& J) {
 
 // P[(I nt + J) 64 + i]: tile (I, J >= ...) contribution to y_I (J <= I: D_IJ x_J;
 // J > I: (D_JI)^T x_J).  Diagonal tiles: the lower part and its mirror.
-template <bool DF>
 __global__ void __launch_bounds__(kKB) k_symv_tiles(int m, int nt, const double* __restrict__ A, int lda,
                                                     const double* __restrict__ x, double* __restrict__ P) {
   __shared__ double xJ[kKT], xI[kKT];
@@ -66,29 +65,17 @@ __global__ void __launch_bounds__(kKB) k_symv_tiles(int m, int nt, const double*
   const bool diag = I == J;
   const double xi = xI[i];
   double rs = 0.0;
-  float rsf = 0.f;
 #pragma unroll 4
   for (int jj = 0; jj < 16; jj++) {
     const int j = g * 16 + jj, col = J * kKT + j;
     const bool in = row < m && col < m && (!diag || i >= j);
-    double cs = 0.0;
-    if (DF) {
-      float d = 0.f;
-      if (in) {
-        const float2 e = reinterpret_cast<const float2*>(A)[(size_t)col * lda + row];
-        d = e.x + e.y;
-      }
-      rsf = fmaf(d, (float)xJ[j], rsf);
-      cs = (!diag || i > j) ? (double)(d * (float)xi) : 0.0;
-    } else {
-      const double d = in ? A[(size_t)col * lda + row] : 0.0;
-      rs = fma(d, xJ[j], rs);
-      cs = (!diag || i > j) ? d * xi : 0.0;
-    }
+    const double d = in ? A[(size_t)col * lda + row] : 0.0;
+    rs = fma(d, xJ[j], rs);
+    double cs = (!diag || i > j) ? d * xi : 0.0;
     for (int o = 16; o > 0; o >>= 1) cs += __shfl_xor_sync(0xffffffffu, cs, o);
     if (lane == 0) cpart[half][j] = cs;
   }
-  rpart[g][i] = DF ? (double)rsf : rs;
+  rpart[g][i] = rs;
   __syncthreads();
   if (tid < kKT) {
     const double yr = ((rpart[0][tid] + rpart[1][tid]) + rpart[2][tid]) + rpart[3][tid];
@@ -431,14 +418,14 @@ size_t krylov_scratch_doubles(int m, int kmax) {
 }
 
 // rd = s2dt D^{1/2} p.  The tensor products: with A != nullptr from the
-// lower-stored tensor (double-float pairs when df); with A == nullptr
+// lower-stored FP64 tensor; with A == nullptr
 // matrix-free from the bead positions (qh, ql: double-float mirror with the
 // radius in w).  p is a device vector.  The coefficients stay on the device;
 // the host reads them back every kCheck iterations (and at kmax) to test
 // convergence, and takes the first iteration that met the tolerance.
 // *iters and *change describe the run.
 constexpr int kCheck = 8;
-int krylov_sqrt(int m, const double* A, int lda, bool df, const float4* qh, const float4* ql, double a1, double a2,
+int krylov_sqrt(int m, const double* A, int lda, const float4* qh, const float4* ql, double a1, double a2,
                 const double* p, double s2dt, double tol, int kmax, double* rd, double* scratch, cudaStream_t st,
                 int* iters, double* change, KrylovGraphs* graphs) {
   const int nt = cdivk(m, kKT), nD = m / 3;
@@ -464,8 +451,7 @@ int krylov_sqrt(int m, const double* A, int lda, bool df, const float4* qh, cons
   // x = V_k: its float4 copy (matrix-free) was written with it by k_norm_scale
   auto product = [&](const double* x, double* y) {
     if (A) {
-      if (df) k_symv_tiles<true><<<(unsigned)tiles, kKB, 0, st>>>(m, nt, A, lda, x, P);
-      else k_symv_tiles<false><<<(unsigned)tiles, kKB, 0, st>>>(m, nt, A, lda, x, P);
+      k_symv_tiles<<<(unsigned)tiles, kKB, 0, st>>>(m, nt, A, lda, x, P);
       k_symv_sum<<<gm, tb, 0, st>>>(m, nt, P, y);
     } else {
       k_rpy_mv<<<cdivk(nD, kMvB), 32 * kMvW, 0, st>>>(nD, qh, ql, xf, (float)a1, (float)a2, y);
@@ -502,9 +488,9 @@ int krylov_sqrt(int m, const double* A, int lda, bool df, const float4* qh, cons
   // context as a CUDA graph (its pointers and sizes are the context's) and
   // replayed; the legacy stream cannot be captured, so it runs them eagerly
   if (graphs && (graphs->m != m || graphs->kmax != kmax || graphs->scratch != scratch || graphs->A != A ||
-                 graphs->df != df || graphs->a1 != a1 || graphs->a2 != a2)) {
+                 graphs->a1 != a1 || graphs->a2 != a2)) {
     graphs->clear();
-    graphs->m = m, graphs->kmax = kmax, graphs->scratch = scratch, graphs->A = A, graphs->df = df;
+    graphs->m = m, graphs->kmax = kmax, graphs->scratch = scratch, graphs->A = A;
     graphs->a1 = a1, graphs->a2 = a2;
   }
   const bool use_graphs = graphs && st != nullptr;

@@ -54,11 +54,10 @@ __global__ void __launch_bounds__(256) k_rpy(int nD, const double* __restrict__ 
     }
     V3 rj = ld3(r + 3 * j);
     V3 sij{ri.x - rj.x, ri.y - rj.y, ri.z - rj.z};
-    double ssq = sij.x * sij.x + sij.y * sij.y + sij.z * sij.z;
-    double s = sqrt(ssq);
+    double s = sqrt(sij.x * sij.x + sij.y * sij.y + sij.z * sij.z);
     double radj = rad[j];
     double Db[3][3];
-    rpy_block(sij, ssq, s, radi, radj, a1, a2, Db);
+    rpy_block(sij, s, radi, radj, a1, a2, Db);
     for (int l = 0; l < 3; l++) {
       double* col = A + (size_t)(3 * j + l) * lda + 3 * i;
       for (int k = 0; k < 3; k++) col[k] = Db[k][l];

@@ -119,19 +119,11 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                : "memory");
 }
 
-// 32 consecutive FP32 columns of this warp's 32 TMEM lanes (one lane per thread).
 // L2 policy: streamed data, first to be evicted (sm_80+ cache hints)
 __device__ __forceinline__ uint64_t policy_evict_first() {
   uint64_t p;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
   return p;
-}
-__device__ __forceinline__ float4 ld_f4_hint(const float4* a, uint64_t pol) {
-  float4 v;
-  asm volatile("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "l"(a), "l"(pol));
-  return v;
 }
 __device__ __forceinline__ float2 ld_f2_hint(const float2* a, uint64_t pol) {
   float2 v;
