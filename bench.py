@@ -460,9 +460,9 @@ def run_ours(args):
 
 def mixed_schedule_bytes(m: int, kT: int = 128, triple_min: int = 40, pair_min: int = 24) -> float:
     """Algorithmic HBM bytes of one mixed factorisation of a 3N = m tensor: the
-    schedule of bdk::potrf_mixed (one launch per panel; groups of two triples of
-    panels a bulk pass while 40 tile rows remain, three pairs while 24 do, then
-    four single panels), 16 B (double-float read + write) per element of the
+    schedule of bdk::potrf_mixed (one launch per panel; groups of two accumulators
+    of three panels a bulk pass while 40 tile rows remain, three of two while 24 do,
+    then four of one), 16 B (double-float read + write) per element of the
     panel's column and of every tile an update job changes.  Equals the library's
     own count (bd_kernel_bytes)."""
     nt = -(-m // kT)

@@ -533,8 +533,8 @@ class Context:
         return it.value, ch.value
 
     def set_mixed_passes(self, passes: int) -> None:
-        """bd_set_mixed_passes: at most `passes` panels per trailing pass of the mixed
-        factorisation (3 fastest, 1 most accurate)."""
+        """bd_set_mixed_passes: at most `passes` panels per accumulator of the mixed
+        factorisation's trailing update (3 fastest, 1 most accurate)."""
         _check(self._L.bd_set_mixed_passes(self._h, int(passes)))
 
     def negative_pivots(self) -> int:
@@ -634,7 +634,7 @@ class Batch:
         return np.array(list(out))
 
     def set_mixed_passes(self, passes: int) -> None:
-        """bd_batch_set_mixed_passes: at most `passes` panels per trailing pass (1 = most accurate)."""
+        """bd_batch_set_mixed_passes: at most `passes` panels per accumulator (1 = most accurate)."""
         _check(self._L.bd_batch_set_mixed_passes(self._h, int(passes)))
 
     def launch_count(self) -> int:

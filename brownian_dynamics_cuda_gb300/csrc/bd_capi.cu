@@ -149,8 +149,10 @@ static int step_phases(bd_ctx* c, const double* d_rr, const double* d_p, double*
   bool rebuild = (c->step_count % c->freq_rp) == 0 || (krylov && c->a_holds_factor) || c->need_rebuild;
   // A whole step's first force pass needs the positions alone: it runs on a side
   // stream beside the tensor, its factor and the noise displacement, which leave
-  // most SMs idle at small sizes.  Not when phases are timed, nor in a batch,
-  // whose replicas already fill the GPU beside each other.
+  // most SMs idle at small sizes.  Not when phases are timed, nor in a batch: its
+  // replicas have no side streams.  Those of a mixed batch that rebuilds its
+  // tensors every step run beside each other on the batch's lanes; all others
+  // (FP64, frequency_RP > 1) run one after another, each in one row.
   const bool overlap = phases == (kPre | kChol | kPost) && !c->timing && !c->in_batch;
   const bdk::Side* side = overlap ? &c->side : nullptr;
   auto lost = [&]() {  // a fork or a join failed
@@ -1082,7 +1084,7 @@ extern "C" int bd_batch_create(int nrep, const bd_model* models, const bd_state*
       return rc;
     }
     c->in_batch = true;
-    side_free(c);  // replicas run beside each other on the batch's own side streams
+    side_free(c);  // (a step's or a force pass's parts run in one row: step_phases)
     b->ctx.push_back(c);
   }
   *out = b;

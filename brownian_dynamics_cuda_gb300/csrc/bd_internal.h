@@ -161,14 +161,14 @@ void rpy_assemble(int nD, const double* r_all, const double* rad, double a1, dou
 int potrf_fp64(int m, double* A, int lda, double* rd_acc, const double* p, double s2dt, int* d_negpiv,
                cudaStream_t st);
 size_t trmv_scratch_doubles(int m);
-// k_tc_chol.cu (mixed precision: FP64 storage, FP32-class arithmetic, tcgen05 trailing updates)
+// k_tc_chol.cu (mixed precision: double-float storage, FP32-class arithmetic, tcgen05)
 size_t mixed_panel_bytes(int m);
 int set_mixed_attributes();
 // kev (optional): 2 events per launch that carries a bulk trailing update
 // (the dominant kernel); *kev_pairs = how many were recorded, *kflop and
 // *kbytes accumulate the tensor work those launches issue and their
 // algorithmic HBM bytes.
-// max_pass: at most this many panels (1..3) per bulk trailing pass.
+// max_pass: at most this many panels (1..3) per accumulator of the trailing update.
 int potrf_mixed(int m, double* A, int lda, unsigned char* PS, int* negpiv, int* err, cudaStream_t st,
                 cudaEvent_t* kev = nullptr, int* kev_pairs = nullptr, double* kflop = nullptr,
                 double* kbytes = nullptr, int max_pass = 3, float scale = 1.f);
@@ -212,8 +212,8 @@ int krylov_sqrt(int m, const double* A, int lda, const float4* qh, const float4*
                 int* iters, double* change, struct KrylovGraphs* graphs = nullptr);
 int mixed_max_launches(int m);  // k_chol_step launches of one factorisation, at most
 // Many mixed factorisations (replicas) advanced together: launch i runs step
-// i of every factorisation's schedule (k_chol_step_multi), then one diagonal
-// scatter for all.  The plan holds the matrices' addresses.
+// i of every factorisation's schedule (k_chol_step_multi).  The plan holds the
+// matrices' addresses.
 struct MixedBatch;
 MixedBatch* mixed_batch_create(int nrep, const int* m, double* const* A, const int* lda, unsigned char* const* PS,
                                int* const* negpiv, int* const* err, const float* scale, int max_pass = 3);
@@ -249,7 +249,7 @@ struct bd_ctx {
   int freq_rp = 1;
   int use_graph = 0;
   float fscale = 1.f;    // mixed path: the panel slices hold fscale * L (mixed_scale)
-  int mixed_passes = 3;  // panels per bulk trailing pass of the mixed factorisation (bd_set_mixed_passes)
+  int mixed_passes = 3;  // panels per accumulator of the mixed factorisation's trailing update (bd_set_mixed_passes)
   // noise displacement: 0 = L p (the reference's), 1 = D^{1/2} p by Lanczos (bd_set_noise_mode)
   int noise_mode = 0;
   double krylov_tol = 1e-6;

@@ -119,7 +119,9 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
 // qh/ql with the radius in w, and x as float4); the FP32 RPY block of every pair
 // (rpy_block_f, the mixed tensor's own formula) applied to x_j; runs of 32 terms
 // in FP32, a run per warp, the runs added in order with Kahan compensation; lanes
-// summed in double-float in a fixed order.  Bound by FP32 issue.  n_D = 3,900: 55
+// summed in double-float (48 bits; the terms have 24) in a fixed order.  Error of the
+// displacement against FP64 products, 2-norm, 12 to 100 nucleosomes, tolerance 1e-10:
+// 1.29e-7 .. 1.65e-7, with FP64 lane sums the same to 0.5 %.  Bound by FP32 issue.  n_D = 3,900: 55
 // us with two beads and all runs a warp, eight warps a CTA (244 CTAs: three or
 // four warps a scheduler), FP64 lane sums and a test for the own bead in every
 // pair; 43 in this split, 36 with the far form of all four beads first.

@@ -287,8 +287,12 @@ __global__ void __launch_bounds__(TM * TN / (MR * NR)) k_syrk_update(double* A, 
 // ------------------------------------------------------------ L p
 constexpr int kRdRows = 256;
 // Columns a CTA sums: short runs at small sizes, where 512 left a few CTAs of one
-// serial chain each (3N = 912: 8 CTAs, 80 us; 32 columns: 11), long ones where
-// the rows alone fill the GPU and the partial sums would cost a second pass.
+// serial chain each, long ones at large ones, whose partial sums (m^2 / chunk
+// values, written and read again) take memory: 34 MB at 3N = 46,200 with 512, 133 with
+// 128.  32, 128, 512 columns, mixed / FP64, us: 3N = 972 16/21, 22/39, 39/123; 1,944 21/41,
+// 23/39, 58/123; 3,888 31/76, 33/99, 74/127; 8,100 91/240, 64/248, 100/442; past the
+// line, 8,262 93/246, 65/247, 102/363 and 10,368 127/364, 102/360, 111/477: there 128 would
+// still be the faster, at 4 times the memory.
 constexpr int kRdChunkMax = 512;
 int rd_chunk(int m) { return m <= 2048 ? 32 : m <= 8192 ? 128 : kRdChunkMax; }
 

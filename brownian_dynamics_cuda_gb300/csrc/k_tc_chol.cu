@@ -137,7 +137,9 @@ __device__ __forceinline__ float2 df_sub(float2 a, float v) {
 // where the repeated work also filled the GPU: 28.7 -> 19.0.
 // The explicit inverse is as accurate as the substitution here (condition
 // numbers of L_kk below 10): error of L p against FP64, 2-norm over 13 fibers
-// of 3N 912 .. 11,700: 2.6e-7 .. 5.4e-7 before, 2.5e-7 .. 5.1e-7 now.
+// of 3N 912 .. 11,700: 2.6e-7 .. 5.4e-7 before, 2.5e-7 .. 5.1e-7 now; 46,200: 5.3e-7, 5.1e-7.
+// (A fiber pressed to a tenth of its size, condition numbers in the hundreds: up
+// to a third above the substitution's 3e-6.)
 constexpr int kLd = 132;  // row stride (floats) of the diagonal block in shared memory: conflict-free 16-byte rows
 constexpr int kChainS = kTileBytes;                  // shared-memory offset of the FP32 diagonal block
 constexpr int kChainW = 130 * 1024;                  // ... and of the inverse's slices
@@ -935,19 +937,20 @@ __device__ __forceinline__ bool panel_body(unsigned char* smraw, const PanelArgs
 // the A operand stays in shared memory).  Warp-specialised, pipelined:
 //   warp 0 (one lane)  bulk-async copies: the two A slices when I changes,
 //                      the two B slices per tile in two K-halves (two
-//                      32 KB stages), and an L2 prefetch of the FP64 tile;
+//                      32 KB stages), and an L2 prefetch of the double-float
+//                      tile (BD_REST_PREFETCH);
 //   warp 1 (one lane)  three FP16 products per K-half into one of four TMEM
 //                      accumulators (128 columns each), tcgen05.commit to
 //                      release stages, the accumulator and the A operand;
 //   warps 2-9          epilogue: tcgen05.ld of the accumulator (warp w reads
 //                      TMEM lanes 32 (w % 4) .. + 31, half of the columns),
-//                      release it, then the FP64 read-modify-write.
+//                      release it, then the double-float read-modify-write.
 // So the next tile's copies and MMAs run under the current tile's epilogue.
 // Every wait is bounded; a timeout records an error code and raises a
 // shared abort flag that ends every role's loop; copies still in flight
 // are waited for (bounded) and TMEM is freed before the CTA exits.
 #ifndef BD_REST_PREFETCH
-#define BD_REST_PREFETCH 0  // L2 prefetch of the FP64 tile ahead of the epilogue (measured slower)
+#define BD_REST_PREFETCH 0  // L2 prefetch of the double-float tile ahead of the epilogue (measured slower)
 #endif
 #ifndef BD_EPI_EVICT_FIRST
 #define BD_EPI_EVICT_FIRST 1  // L2 evict-first hint on the epilogue's tile loads and stores
@@ -1099,7 +1102,7 @@ __device__ __forceinline__ bool rest_body(unsigned char* smraw, float2* A, int l
           curI = I;
           nA++;
         }
-        if (BD_REST_PREFETCH) {  // the FP64 tile's columns into L2 ahead of the epilogue
+        if (BD_REST_PREFETCH) {  // the tile's columns into L2 ahead of the epilogue
           const int rows = min(kT, lda - I * kT);
           const int jend = min(J * kT + kT, m);
           for (int gj = J * kT; gj < jend; gj++)
@@ -1554,7 +1557,9 @@ namespace bdk {
 // three panels: 4.8 ms at 11,700; four of two: 11.0 and 4.7; the bulk of a group
 // spread over the next group's launches: 131 at 46,200.)
 constexpr int kGroup[4] = {0, 4, 3, 2};  // accumulators by fold
-constexpr int kGroupMin = 4;             // tile rows right of a group (fewer accumulators at the end)
+// tile rows right of a group (fewer accumulators at the end).  2, 4, 8, 12: 3N = 1,944
+// 0.532, 0.535, 0.537, 0.545 ms; at 5,184 and above within 1 %
+constexpr int kGroupMin = 4;
 static_assert(kBufs > kGroup[1] && kBufs > 2 * kGroup[2] && kBufs > 3 * kGroup[3], "a group's panels and the next");
 // the slice buffers, then two buffers for the inverse of a diagonal factor
 // (W_k in buffer k & 1: read by the launch that writes W_k+1), then its factors,
@@ -1624,11 +1629,19 @@ static int rest_group(int tiles, int gmax) {
 //     column k + i + 1 and on diagonal block k + i + 2;
 //   launch k + g: panel k + g beside the group on the tiles right of column k + g.
 // Returns the number of kernel launches.
+// Lines of the panels an accumulator sums (fold), in tile rows right of its first
+// panels.  A group costs launches that hold one chain and its column updates; it
+// saves read-modify-writes of the rest, so it needs rows to save.  Measured:
+//   two from 48, 32, 24, 16, 8 rows: 3N = 5,184 1.57, 1.54, 1.53, 1.52, 1.52 ms, 3,888 1.10,
+//   1.10, 1.09, 1.09, 1.09 - flat below 32, where one panel an accumulator is also the
+//   more accurate;
+//   three from 96, 64, 40, 24 rows: 3N = 8,100 2.80, 2.81, 2.68, 2.66, 12,960 6.15, 5.74,
+//   5.60, 5.57, 5,184 1.53, 1.53, 1.53, 1.50 - flat from 40 down, likewise.
 #ifndef BD_PAIR_MIN
-#define BD_PAIR_MIN 24  // pair while at least this many tile rows remain right of column k+2 (k: last factored)
+#define BD_PAIR_MIN 24  // two panels an accumulator while this many tile rows remain right of column k + 2
 #endif
 #ifndef BD_TRIPLE_MIN
-#define BD_TRIPLE_MIN 40  // three panels per bulk pass while this many tile rows remain right of column k+3
+#define BD_TRIPLE_MIN 40  // three panels an accumulator while this many tile rows remain right of column k + 3
 #endif
 namespace {
 struct Job {
@@ -1638,10 +1651,10 @@ struct Job {
 
 // The launches of one factorisation: issued on st, or (plan != nullptr)
 // only recorded with their grid sizes.
-// max_pass (1..3): most panels one bulk pass carries (K = 128 max_pass).
-// Fewer panels per pass mean fewer FP32 tensor-memory accumulation steps per
-// stored update and more read-modify-write passes: 3 is the fastest, 1 the
-// most accurate.
+// max_pass (1..3): most panels an accumulator sums (K = 128 max_pass; a pass has
+// up to four of them).  Fewer mean fewer FP32 accumulation steps in tensor
+// memory per stored update and more subtractions from the double-float tile: 3
+// is the fastest, 1 the most accurate.
 static int potrf_mixed_impl(int m, double* A64, int lda, unsigned char* PS, int* negpiv, int* err, cudaStream_t st,
                             cudaEvent_t* kev, int* kev_pairs, double* kflop, double* kbytes,
                             std::vector<std::pair<StepArgs, int>>* plan, int max_pass, float scale) {
