@@ -34,9 +34,9 @@ sys.path.insert(0, ROOT)
 METRIC = "BD steps/s vs plain FP64 on 1 GB300 at <=1e-6 rel. error; replica-steps/s"
 # dram__bytes_read.sum + dram__bytes_write.sum / algorithmic bytes of one
 # k_chol_step launch under ncu (the eighth of a factorisation: panel 6 beside
-# the bulk update by panels 0-5, 3N = 11,700: 955.9 MB of DRAM traffic for
+# the bulk update by panels 0-5, 3N = 11,700: 954.2 MB of DRAM traffic for
 # 956.0 MB algorithmic)
-NCU_TRAFFIC_PER_ALG_BYTE = 955.9 / 956.0
+NCU_TRAFFIC_PER_ALG_BYTE = 954.2 / 956.0
 # largest 3N for which the GPU line's CPU baseline times complete oracle steps
 CPU_STEP_MAX_M = 20000
 

@@ -327,7 +327,7 @@ int bd_batch_launch_count(const bd_batch* b, int* out);
  * accumulator sums its panels' products in FP32 tensor memory before they are
  * added to the double-float tensor (up to four accumulators in one pass over
  * it), so fewer panels each give a more accurate factor at more work to add
- * them (measured at 3N = 11,700: 3 -> 4.5 ms, noise displacement 6.9e-7 from
+ * them (measured at 3N = 11,700: 3 -> 4.6 ms, noise displacement 6.9e-7 from
  * FP64; 2 -> 5.0 ms, 5.8e-7; 1 -> 5.7 ms, 5.0e-7).
  * The next step captures its graph again.  No counterpart in the reference
  * (its factorisation is FP64 cuSOLVER). */
