@@ -35,7 +35,8 @@ def _ctx(f, mixed, passes=3):
 
 
 # the bead in the first and in a middle tile, at the end, in a tile row's last columns
-GROWN = [("syn_4nuc_lh", "lh_rad", 12, -12.0), ("syn_4nuc_lh", "lh_rad", 3, -300.0),
+GROWN = [("syn_4nuc_lh", "rad", 2, -1.5), ("syn_4nuc_lh", "lh_rad", 9, -11.6),  # little growth, all rows fit
+         ("syn_4nuc_lh", "lh_rad", 12, -12.0), ("syn_4nuc_lh", "lh_rad", 3, -300.0),
          ("syn_4nuc_lh", "lh_rad", 40, -300.0), ("syn_4nuc_lh", "lh_rad", -1, -300.0),
          ("syn_4nuc_lh", "lh_rad", 40, -1e4), ("syn_4nuc_lh", "t_rad", 2, -300.0),
          ("syn_4nuc_lh", "t_rad", -1, -300.0), ("cfg0_12nuc", "t_rad", -1, -300.0),
